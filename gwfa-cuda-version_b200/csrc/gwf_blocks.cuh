@@ -1,0 +1,878 @@
+// gwf_blocks.cuh — the distance kernel of the batch forms: block wavefronts with exact pruning.
+//
+// Same scores as the sorted wavefront of gwf_kernels.cuh, another data structure. The diagonals of
+// a read live in blocks of 8 neighbouring diagonals of one vertex, one 128-byte line each, found
+// through a hash table of block ids and linked to their neighbours. A score step
+//   1. walks the list of live blocks: each diagonal's successor is max(k[d-1], k[d] + 1,
+//      k[d+1] + 1, arc-side candidate), dropped where the diagonal has passed the vertex end,
+//      extended and written to the row of the step's parity (gwf-ed.cu:902-1016);
+//   2. sends the vertex-end states over their arcs in waves (gwf-ed.cu:1106-1255): an arrival is
+//      a bit of the target diagonal's cell, a candidate a max into it, so that no arrival set, no
+//      sort, no merge and no interval list remain.
+//
+// Exact pruning. A lag-pruned run of the same loop first gives an upper bound U of the read's
+// distance (an alignment of U edits exists). Then a state at score s and query position i is
+// dropped when s + h(i + 1) >= U, where h counts edits that the rest of the query cannot avoid
+// (bw_seeds). Dropped states cannot lead to a distance below U, and the states of a shorter
+// alignment all survive, so the distance is the one of the unpruned run: U where that run finds
+// none below it. States per read, against the unpruned loop: configuration 3 39,200 -> 5,700,
+// configuration 4 962,000 -> 107,000, and 10,700 with windows from every base; the lag run needs
+// 600 and 2,300.
+//
+// What bounds it: instruction issue and fetch (ncu, 1 kbp reads: 0.49 issue slots active per cycle
+// at 32 warps per SM, a third of the stalls waiting for instructions), and the latency of one
+// read's chain of steps where a batch has few or unequal reads. Resident reads, graph replay,
+// kernel_ms against the sorted form: 100,000 x 1 kbp 26.1 -> 12.7 ms, 50,000 mixed 137 -> 27 ms,
+// 4,000 x 10 kbp on the dense graph 600 -> 33 ms, one 20 kbp read at 10% 374 -> 274 ms.
+#pragma once
+#include "gwf_kernels.cuh"
+
+namespace gwfb {
+
+constexpr int32_t BW_NONE = -(1 << 29);
+constexpr int32_t BW_ENDED = 1 << 29; // arc-side candidate that ends its diagonal
+constexpr int32_t BW_INF = 0x3fffffff;
+
+// One block, 128 bytes. rows[s & 1] holds the extended k of score step s.
+struct __align__(128) BwBlock {
+	uint32_t gb;       // first base of the vertex in the concatenated sequence
+	uint32_t arcs;     // its arcs (DevGraph::varcs)
+	uint32_t v;
+	int32_t db;        // diagonal of cell 0 (a multiple of 8)
+	int32_t vl;
+	int32_t left, right; // neighbouring blocks, -1 = none yet
+	uint8_t ended;     // diagonals past the vertex end
+	uint8_t has_c;     // some cell has an arc-side candidate
+	uint8_t inl[2];    // in the live list of even / odd steps
+	int32_t row[2][8];
+	int32_t c[8];      // arc-side candidate of the next step, k << 1 | arrived
+};
+static_assert(sizeof(BwBlock) == 128, "one line per block");
+
+// Words and bits of a 16-mer in the graph's filter (4 bits of one 64-bit word).
+__host__ __device__ inline uint32_t bloom_word(uint32_t x, uint32_t mask)
+{
+	x *= 0x9E3779B1u;
+	x ^= x >> 15;
+	x *= 0x2C1B3C6Du;
+	return (x ^ x >> 13) & mask;
+}
+__host__ __device__ inline uint64_t bloom_bits(uint32_t x)
+{
+	uint32_t y = (x ^ x >> 16) * 0x85EBCA6Bu;
+	y ^= y >> 13;
+	return 1ULL << (y & 63) | 1ULL << (y >> 6 & 63) | 1ULL << (y >> 12 & 63) | 1ULL << (y >> 18 & 63);
+}
+
+#ifndef GWF_KERNELS_DECL_ONLY
+constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few steps cost less than a bound
+constexpr int32_t kPruneLag = 12;    // lag of the run that gives an upper bound
+
+// The filter's build: every string of K = bloom_k bases that a walk of the graph spells, from
+// every position. One warp per vertex, one start per lane; walks branch through a stack (fewer than
+// K levels, as each vertex gives at least one base). A walk that dead-ends after K - 1 bases
+// enters all four extensions, so that a string of K - 1 bases may be looked up by extending it. A
+// start with more than kBloomLeaves walks sets *many, and the graph gets no filter.
+constexpr int32_t kBloomLeaves = 1024;
+__global__ void __launch_bounds__(256) k_bloom(const __grid_constant__ DevGraph g, unsigned long long *bloom,
+                                               int32_t *many)
+{
+	const int lane = threadIdx.x & 31;
+	const int32_t K = g.bloom_k;
+	const uint32_t mask = g.bloom_mask;
+	const uint32_t v0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+	if (v0 >= g.n_vtx) return;
+	const uint32_t l0 = __ldg(g.len + v0);
+	for (uint32_t o0 = lane; o0 < l0; o0 += 32) {
+		uint32_t st_x[17], st_a[17], st_e[17];
+		int32_t st_n[17];
+		int32_t depth = 0, n = 0, leaves = 0;
+		uint32_t v = v0, o = o0, x = 0;
+		for (int64_t guard = 0; guard < 64LL * kBloomLeaves; ++guard) {
+			const uint32_t vl = __ldg(g.len + v);
+			const uint64_t gb = __ldg(g.base + v);
+			for (; o < vl && n < K; ++o, ++n) {
+				const uint64_t p = gb + o;
+				x |= (uint32_t)(__ldg(g.pk + (p >> 5)) >> (2 * (p & 31)) & 3) << (2 * n);
+			}
+			bool up = false;
+			if (n == K) {
+				atomicOr(bloom + bloom_word(x, mask), (unsigned long long)bloom_bits(x));
+				up = true;
+			} else {
+				const uint32_t a = __ldg(g.arc_off + v), e = __ldg(g.arc_off + v + 1);
+				if (a == e) {
+					if (n == K - 1)
+						for (uint32_t y = 0; y < 4; ++y) {
+							const uint32_t z = x | y << (2 * K - 2);
+							atomicOr(bloom + bloom_word(z, mask), (unsigned long long)bloom_bits(z));
+						}
+					up = true;
+				} else
+					st_x[depth] = x, st_n[depth] = n, st_a[depth] = a, st_e[depth] = e, ++depth;
+			}
+			if (up && ++leaves > kBloomLeaves) break;
+			while (depth > 0 && st_a[depth - 1] == st_e[depth - 1]) --depth;
+			if (depth == 0) break;
+			const uint2 arc = __ldg(g.arc + st_a[depth - 1]++);
+			v = arc.x, o = arc.y, x = st_x[depth - 1], n = st_n[depth - 1];
+		}
+		if (leaves > kBloomLeaves || depth > 0) *many = 1;
+	}
+}
+
+// State of a warp's run, in the CTA's shared memory (one warp per CTA). The parts of the kernel
+// that are not run at every step are functions of their own that work on it: with everything
+// inlined the kernel had 87 KB of code, its 32 warps per SM stood in different parts of it, and
+// the instruction cache held half of their cycles.
+constexpr int kBwQueue = 31 + 16 * 8;
+struct BwShm {
+	uint2 queue[kBwQueue + 1]; // diagonals on their way to the extension: id << 4 | side << 3 | cell, k
+	BwBlock *blk;
+	uint2 *hash;               // (tag, id) per slot, id -1 = empty
+	uint32_t *slot;            // slot of each block
+	int32_t *nxt;              // live list of the next step
+	uint32_t *e, *f, *n;       // vertex-end states of a wave and of the next, entered states: id << 3 | cell
+	int32_t *nk;               // offsets of the entered states
+	uint16_t *h;               // edits that the last rem bases cannot avoid
+	const uint64_t *qpk;
+	const uint8_t *qraw;
+	const uint32_t *gpk;
+	const uint8_t *graw;
+	const uint4 *arcx;
+	const uint32_t *varcs, *arc_off;
+	const uint64_t *bloom;
+	uint32_t bloom_mask;
+	int32_t K;
+	uint32_t hmask;
+	int32_t nb;                // blocks in the pool
+	int32_t ql, packed, quirk;
+	int32_t n_blk, n_nxt;      // blocks in use, length of nxt
+	int32_t ovf;               // a buffer is full
+};
+__device__ __forceinline__ BwShm &bw_sh()
+{
+	extern __shared__ __align__(16) unsigned char bw_smem[];
+	return *(BwShm *)bw_smem;
+}
+
+__device__ __forceinline__ bool bloom_has(const BwShm &sh, uint32_t x)
+{
+	const uint64_t b = bloom_bits(x);
+	return (__ldg(sh.bloom + bloom_word(x, sh.bloom_mask)) & b) == b;
+}
+
+// Does the graph (as its filter says) spell the K-base string y with one edit? code = kind << 8 |
+// a << 2 | t. Kind 0: another base (xor t) at a; 1: the base t inserted before a (K + 1 bases: the
+// first K and the last K); 2: the base at a taken out and t appended.
+static __device__ __noinline__ bool bw_edit(uint32_t y, int code)
+{
+	const BwShm &sh = bw_sh();
+	const int K = sh.K, kind = code >> 8, a2 = code >> 1 & 126;
+	const uint32_t t = code & 3, lo = y & ((1u << a2) - 1), hi = y >> a2, kmask = ~0u >> (32 - 2 * K);
+	uint32_t z = y ^ t << a2;
+	if (kind == 1) z = ((hi << 2 | t) << a2 | lo) & kmask;
+	if (kind == 2) z = hi >> 2 << a2 | lo | t << (2 * K - 2);
+	bool ok = bloom_has(sh, z);
+	if (ok && kind == 1) ok = bloom_has(sh, (uint32_t)(((uint64_t)(hi << 2 | t) << a2 | lo) >> 2));
+	return ok;
+}
+
+// Edits that the last rem bases of the query cannot avoid, rem = 0 .. ql, into h[rem]; returns
+// h[ql]. A window of K bases costs 0, 1 or 2 edits when the graph spells a string within 0, 1 or
+// more edits of it; windows that do not overlap add up, so h[rem] = max(h[rem - 1], h[rem - K] +
+// cost of the window that starts rem bases before the end). Windows start every `stride` bases.
+// Lanes test 32 windows for exact presence. An absent one is looked up with one edit by the whole
+// warp (3 K substitutions, 4 (K - 1) insertions, 4 K deletions with any appended base); an edit
+// that is found is then tried on the other absent windows of the 32 that hold its position. A
+// window with a byte other than A/C/G/T costs 1 (the graph has none). With stride 1 every other
+// absent window counts 1 without the one-edit lookups: half of them, for a bound 0.5% lower.
+static __device__ __noinline__ int32_t bw_seeds(int32_t stride)
+{
+	const BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31;
+	const int32_t K = sh.K, ql = sh.ql, n_edit = 11 * K - 4;
+	uint16_t *const h = sh.h;
+#pragma unroll 1
+	for (int32_t j = lane; j <= ql; j += 32) h[j] = 0;
+	__syncwarp();
+#pragma unroll 1
+	for (int32_t base = K; base <= ql; base += 32 * stride) {
+		const int32_t rem = base + lane * stride, p = ql - rem;
+		uint32_t x = 0, nb = 0; // the window and the base after it
+		int32_t cost = 0;
+		if (rem <= ql) {
+			uint32_t lo, hi;
+			window32<false>((const uint32_t *)sh.qpk, p, lo, hi);
+			x = lo & ~0u >> (32 - 2 * K);
+			nb = (K == 16 ? hi : lo >> (2 * K)) & 3;
+			bool odd = false;
+			if (!sh.packed)
+#pragma unroll 1
+				for (int t = 0; t < K; ++t) {
+					const uint8_t ch = sh.qraw[p + t];
+					odd |= !(ch == 'A' || ch == 'C' || ch == 'G' || ch == 'T');
+				}
+			cost = odd ? 1 : bloom_has(sh, x) ? 0 : stride == 1 && (rem & 1) ? 1 : 2;
+		}
+		uint32_t todo = __ballot_sync(FULL, cost == 2);
+#pragma unroll 1
+		while (todo) {
+			const int src = __ffs(todo) - 1;
+			todo &= todo - 1;
+			uint32_t y = __shfl_sync(FULL, x, src), hit = 0;
+			const int32_t sp = __shfl_sync(FULL, p, src);
+			int code = 0;
+#pragma unroll 1
+			for (int t0 = 0; t0 < n_edit && !hit; t0 += 32) {
+				const int t = t0 + lane, u = t - 3 * K, w = u - 4 * (K - 1);
+				code = t < 3 * K ? (t / 3) << 2 | (t % 3 + 1) : w < 0 ? 1 << 8 | (u + 4) : 2 << 8 | w;
+				hit = __ballot_sync(FULL, t < n_edit && bw_edit(y, code));
+			}
+			if (!hit) continue;
+			// the same edit in this lane's window
+			const int c = __shfl_sync(FULL, code, __ffs(hit) - 1), kind = c >> 8;
+			const int a = sp + (c >> 2 & 63) - p;
+			const bool same = (todo >> lane & 1) && a >= (kind == 1) && a < K;
+			if (lane == src || (same && bw_edit(x, kind << 8 | a << 2 | (kind == 2 ? (int)nb : c & 3)))) cost = 1;
+			todo &= __ballot_sync(FULL, cost == 2);
+		}
+		if (rem <= ql) h[rem] = (uint16_t)cost;
+	}
+	__syncwarp();
+	// the maximum over disjoint windows, K entries at a time: lane l's entry takes its window after
+	// h[rem - K] of the pass before
+	int32_t prev = 0; // lane l < K: h[b - K + l]
+	int32_t last = 0; // h[b - 1]
+#pragma unroll 1
+	for (int32_t b = K; b <= ql; b += K) {
+		const int32_t rem = b + lane;
+		const bool on = lane < K && rem <= ql;
+		int32_t v = on ? prev + (int32_t)h[rem] : 0;
+		v = max(v, last);
+#pragma unroll
+		for (int o = 1; o < 16; o <<= 1) {
+			const int32_t u = __shfl_up_sync(FULL, v, o);
+			if (lane >= o) v = max(v, u);
+		}
+		if (on) h[rem] = (uint16_t)min(v, 65535);
+		prev = v;
+		last = __shfl_sync(FULL, v, K - 1);
+	}
+	__syncwarp();
+	return (int32_t)h[ql];
+}
+
+// gwf_extend1 (see ext) with the vertex's first base gb at hand. The whole warp calls it; on: this
+// lane extends. Every compare covers 32 bases and may run past either end (padding words).
+static __device__ __noinline__ int32_t bw_ext_raw(uint32_t gb, int32_t d, int32_t k, int32_t m)
+{
+	const BwShm &sh = bw_sh();
+#pragma unroll 1
+	for (int guard = 0; k < m && guard < (1 << 28); ++guard) {
+		const uint64_t x = window8<true>(sh.graw, (int64_t)gb + k + 1) ^ window8<false>(sh.qraw, (int64_t)d + k + 1);
+		if (x == 0) {
+			k += 8;
+			continue;
+		}
+		k += __ffsll((long long)x) - 1 >> 3;
+		break;
+	}
+	return k;
+}
+__device__ __forceinline__ int32_t bw_ext(const BwShm &sh, uint32_t gb, int32_t d, int32_t k, int32_t vl, bool on)
+{
+	const int32_t m = min(sh.ql - d, vl) - 1;
+	bool more = on && k < m && !(k < 0 && m < 31 && sh.quirk);
+	if (sh.packed) {
+		const uint32_t *const gp = sh.gpk, *const qp = (const uint32_t *)sh.qpk;
+#pragma unroll 1
+		while (__any_sync(FULL, more)) {
+			if (more) {
+				const uint32_t gx = gb + k + 1, qx = d + k + 1;
+				const uint32_t *const gw = gp + (gx >> 4), *const qw = qp + (qx >> 4);
+				const uint32_t g0 = __ldg(gw), g1 = __ldg(gw + 1), g2 = __ldg(gw + 2), q0 = qw[0], q1 = qw[1], q2 = qw[2];
+				const uint32_t gs = 2 * gx, qs = 2 * qx;
+				const uint32_t lo = __funnelshift_r(g0, g1, gs & 30) ^ __funnelshift_r(q0, q1, qs & 30);
+				const uint32_t hi = __funnelshift_r(g1, g2, gs & 30) ^ __funnelshift_r(q1, q2, qs & 30);
+				const int32_t a = __clz(__brev(lo)) >> 1, b = __clz(__brev(hi)) >> 1; // 16 where all are equal
+				const int32_t n = a < 16 ? a : 16 + b;
+				k += n;
+				more = n == 32 && k < m;
+			}
+		}
+	} else if (more)
+		k = bw_ext_raw(gb, d, k, m);
+	return min(k, m); // lanes that are on
+}
+
+// Hash table of the blocks: linear probing over slots of (tag, id).
+__device__ __forceinline__ uint32_t bw_tag(uint32_t v, int32_t bi)
+{
+	uint32_t x = v * 0x9E3779B1u + (uint32_t)bi * 0x85EBCA6Bu;
+	x ^= x >> 15;
+	return x * 0x2C1B3C6Du;
+}
+
+// Block bi (diagonals 8 bi .. 8 bi + 7) of vertex v, made where it is missing (the whole warp calls
+// it; on: this lane asks). Of the lanes that want one empty slot the first makes its block. Sets
+// ovf when the pool is full. gb, vl: the vertex's first base and length.
+static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, uint32_t gb, int32_t vl)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31;
+	BwBlock *const blk = sh.blk;
+	uint2 *const hash = sh.hash;
+	const uint32_t hmask = sh.hmask;
+	int32_t id = on ? -1 : 0;
+	bool made = false;
+	uint32_t tag = bw_tag(v, bi), sl = (tag ^ tag >> 16) & hmask;
+	int32_t n_blk = sh.n_blk;
+#pragma unroll 1
+	for (uint32_t guard = 0; guard <= hmask + 64; ++guard) {
+		bool want = false;
+		if (id < 0) {
+			const uint2 e = hash[sl];
+			want = (int32_t)e.y < 0;
+			if (!want) {
+				if (e.x == tag && blk[e.y].v == v && blk[e.y].db == 8 * bi) id = (int32_t)e.y;
+				else sl = sl + 1 & hmask;
+			}
+		}
+		if (__any_sync(FULL, want)) {
+			const uint32_t same = __match_any_sync(FULL, want ? (int32_t)sl : -1 - lane);
+			const bool won = want && (same & lanemask_lt()) == 0;
+			const uint32_t m = __ballot_sync(FULL, won);
+			if (n_blk + __popc(m) > sh.nb) {
+				sh.ovf = 1;
+				break;
+			}
+			if (won) {
+				id = n_blk + __popc(m & lanemask_lt());
+				hash[sl] = make_uint2(tag, (uint32_t)id);
+				int4 *q = (int4 *)(blk + id);
+				q[1] = make_int4(vl, -1, -1, 0);
+				const int4 none = make_int4(BW_NONE, BW_NONE, BW_NONE, BW_NONE);
+				const int4 nonec = make_int4(2 * BW_NONE, 2 * BW_NONE, 2 * BW_NONE, 2 * BW_NONE);
+				q[2] = none, q[3] = none, q[4] = none, q[5] = none, q[6] = nonec, q[7] = nonec;
+				q[0] = make_int4((int)gb, (int)__ldg(sh.varcs + v), (int)v, 8 * bi);
+				sh.slot[id] = sl;
+				made = true;
+			}
+			n_blk += __popc(m);
+			__syncwarp();
+		}
+		if (!__any_sync(FULL, id < 0)) break;
+	}
+	sh.n_blk = n_blk;
+	if (__any_sync(FULL, made)) {
+		// links to the neighbours that exist
+#pragma unroll 1
+		for (int side = -1; made && side <= 1; side += 2) {
+			tag = bw_tag(v, bi + side), sl = (tag ^ tag >> 16) & hmask;
+#pragma unroll 1
+			for (uint32_t guard = 0; guard <= hmask; ++guard) {
+				const uint2 e = hash[sl];
+				if ((int32_t)e.y < 0) break;
+				BwBlock *const B = blk + e.y;
+				if (e.x == tag && B->v == v && B->db == 8 * (bi + side)) {
+					*(side < 0 ? &blk[id].left : &blk[id].right) = (int32_t)e.y;
+					*(side < 0 ? &B->right : &B->left) = id;
+					break;
+				}
+				sl = sl + 1 & hmask;
+			}
+		}
+	}
+	__syncwarp();
+	return max(id, 0);
+}
+
+// Puts block id into the next live list, once (several lanes may name one block). np: the parity of
+// the next step.
+static __device__ __noinline__ void bw_push(bool on, int32_t id, int np)
+{
+	BwShm &sh = bw_sh();
+	const uint32_t same = __match_any_sync(FULL, on ? id : -1 - (int)(threadIdx.x & 31));
+	uint8_t *const f = &sh.blk[id].inl[np];
+	const bool app = on && (same & lanemask_lt()) == 0 && !*f;
+	if (app) *f = 1;
+	const uint32_t m = __ballot_sync(FULL, app);
+	const int32_t n = sh.n_nxt;
+	if (app) sh.nxt[n + __popc(m & lanemask_lt())] = id;
+	__syncwarp();
+	sh.n_nxt = n + __popc(m);
+	__syncwarp();
+}
+
+// Arc-side candidate k for diagonal d of vertex v at the next step (lanes that meet on one diagonal
+// bring the same k).
+static __device__ __noinline__ void bw_cand(bool on, uint32_t v, int32_t d, uint32_t gb, int32_t vl, int32_t k, int np)
+{
+	BwShm &sh = bw_sh();
+	const int32_t id = bw_get(on, v, d >> 3, gb, vl);
+	if (sh.ovf) return;
+	if (on) {
+		int32_t *const c = sh.blk[id].c + (d & 7);
+		const int32_t c0 = *c;
+		if (c0 >> 1 < k) *c = k << 1 | (c0 & 1);
+		sh.blk[id].has_c = 1;
+	}
+	bw_push(on, id, np);
+}
+
+// A live edge diagonal (act: block id, cell l) gives the neighbouring block a candidate at the next
+// step: lists the neighbour, made where it is missing.
+static __device__ __noinline__ void bw_side(bool act, int32_t id, int32_t l, int np)
+{
+	BwShm &sh = bw_sh();
+	__syncwarp();
+	const BwBlock *const B = sh.blk + id;
+	const int32_t t = l == 0 ? B->left : B->right;
+	const bool miss = act && t < 0;
+	int32_t u = t;
+	if (__any_sync(FULL, miss)) {
+		const int32_t w = bw_get(miss, B->v, (B->db >> 3) + (l == 0 ? -1 : 1), B->gb, B->vl);
+		if (sh.ovf) return;
+		if (miss) u = w;
+	}
+	bw_push(act, act ? u : 0, np);
+}
+
+// Successors of the live blocks base .. of the list cur (n_cur entries), two lanes per block and
+// four diagonals per lane, until the queue (n_q entries) holds 32 diagonals that may live or the
+// list ends. Blocks that stay go to the next list. kmin: the least offset of a candidate. Returns
+// (base, n_q).
+static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t base, int32_t n_cur, int32_t n_q, int par,
+                                            int32_t kmin)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31, np = par ^ 1, hf = lane & 1;
+	int32_t n_nxt = sh.n_nxt;
+#pragma unroll 1
+	while (n_q < 32 && base < n_cur) {
+		const bool in = base + (lane >> 1) < n_cur;
+		const int32_t bid = cur[in ? base + (lane >> 1) : base];
+		BwBlock *const B = sh.blk + bid;
+		const int4 h1 = *((const int4 *)B + 1);
+		const int32_t nid = hf ? h1.z : h1.y; // the neighbour at this lane's side
+		const uint32_t fl = (uint32_t)h1.w;   // ended, has_c, inl[0], inl[1]
+		const int4 kk = *((const int4 *)B->row[np] + hf);
+		int32_t ek = BW_NONE;
+		if (nid >= 0) ek = sh.blk[nid].row[np][hf ? 0 : 7];
+		const int32_t ok = __shfl_xor_sync(FULL, hf ? kk.x : kk.w, 1);
+		const int32_t lf = hf ? ok : ek, rt = hf ? ek : ok;
+		int32_t kq[4] = {max(lf, max(kk.x, kk.y) + 1), max(kk.x, max(kk.y, kk.z) + 1),
+		                 max(kk.y, max(kk.z, kk.w) + 1), max(kk.z, max(kk.w, rt) + 1)};
+		if (__any_sync(FULL, (fl & 0xff00) != 0)) {
+			int4 *const cp = (int4 *)B->c + hf;
+			const int4 c = *cp;
+			kq[0] = max(kq[0], c.x >> 1), kq[1] = max(kq[1], c.y >> 1);
+			kq[2] = max(kq[2], c.z >> 1), kq[3] = max(kq[3], c.w >> 1);
+			if (in)
+				*cp = make_int4(2 * BW_NONE | (c.x & 1), 2 * BW_NONE | (c.y & 1), 2 * BW_NONE | (c.z & 1),
+				                2 * BW_NONE | (c.w & 1));
+		}
+		uint32_t en = 0, up = 0;
+#pragma unroll
+		for (int q = 0; q < 4; ++q) {
+			en |= (uint32_t)(kq[q] >= h1.x) << q;
+			up |= (uint32_t)(kq[q] >= kmin) << q;
+		}
+		up &= in ? ~(en | fl >> (4 * hf)) & 15u : 0u;
+		// the block stays listed while it has, or just lost, live diagonals (a block that leaves has
+		// both rows empty)
+		const bool stays = up != 0 || (in && max(max(kk.x, kk.y), max(kk.z, kk.w)) > BW_NONE);
+		const uint32_t w = en << (4 * hf) | (stays ? 0x100u : 0u);
+		const uint32_t w2 = w | __shfl_xor_sync(FULL, w, 1);
+		const uint32_t inb = 0x10000u << (8 * np);
+		const bool first = hf == 0 && in, app = first && (w2 & 0x100) && !(fl & inb);
+		if (in) *((int4 *)B->row[par] + hf) = make_int4(BW_NONE, BW_NONE, BW_NONE, BW_NONE);
+		if (first) *((uint32_t *)B + 7) = (fl & ~(0xff00u | 0xff0000u << (8 * par))) | (w2 & 0xff) | (app ? inb : 0);
+		const uint32_t mp = __ballot_sync(FULL, app);
+		if (app) sh.nxt[n_nxt + __popc(mp & lanemask_lt())] = bid;
+		n_nxt += __popc(mp);
+		// side: an edge diagonal whose neighbour has no live diagonal beside it
+		const uint32_t tag = (uint32_t)bid << 4 | (uint32_t)hf << 2, sq = ek > BW_NONE ? 0u : hf ? 8u : 1u;
+#pragma unroll
+		for (int q = 0; q < 4; ++q) {
+			const bool on = up >> q & 1;
+			const uint32_t m = __ballot_sync(FULL, on);
+			if (on)
+				sh.queue[n_q + __popc(m & lanemask_lt())] = make_uint2(tag | q | ((sq >> q & 1) << 3), (uint32_t)kq[q]);
+			n_q += __popc(m);
+		}
+		base += 16;
+		__syncwarp();
+	}
+	sh.n_nxt = n_nxt;
+	__syncwarp();
+	return make_int2(base, n_q);
+}
+
+// Vertex-end states of step s (n_e entries of e) over their arcs, in waves, until no state is
+// entered with a free match (gwf-ed.cu:1106-1255). Four lanes per state, one arc each. Returns
+// this lane's furthest query position, INT32_MAX in every lane when the query's end was reached.
+static __device__ __noinline__ int32_t bw_waves(int32_t s, int32_t T, int32_t n_e)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31, np = ~s & 1;
+	BwBlock *const blk = sh.blk;
+	const int32_t ql = sh.ql, ne = sh.nb;
+	int32_t far = INT32_MIN;
+	bool found = false;
+#pragma unroll 1
+	for (int32_t wave = 0; n_e > 0 && !sh.ovf; ++wave) {
+		int32_t n_n = 0;
+#pragma unroll 1
+		for (int32_t base = 0; base < n_e; base += 8) {
+			const bool act = base + (lane >> 2) < n_e;
+			const uint32_t e = sh.e[act ? base + (lane >> 2) : 0];
+			const int32_t id = (int32_t)(e >> 3), cl = (int32_t)(e & 7);
+			const int4 b0 = *(const int4 *)(blk + id); // gb, arcs, v, db
+			const int32_t vl = blk[id].vl, i = b0.w + cl + vl - 1;
+			const uint32_t aoff = (uint32_t)b0.y & kVArcsMask;
+			uint32_t deg = (uint32_t)b0.y >> kVArcsBits, n_ext = 0;
+			if (deg == kVArcsMany) deg = __ldg(sh.arc_off + b0.z + 1) - aoff;
+			if (!act) deg = 0;
+			const uint32_t qc = (uint32_t)(sh.qpk[(i + 1) >> 5] >> (2 * ((i + 1) & 31))) & 3;
+			// least scores of a path through the deletion into an arc's target and the mismatch
+			const int32_t ha = s + 1 + (int32_t)sh.h[ql - 1 - i], hb = s + 1 + (int32_t)sh.h[ql - 2 - i];
+			const uint32_t max_deg = __reduce_max_sync(FULL, deg);
+#pragma unroll 1
+			for (uint32_t t0 = lane & 3; t0 < max_deg + (lane & 3); t0 += 4) {
+				const bool has = t0 < deg;
+				uint4 a = make_uint4(0, 0, 0, 0);
+				if (has) a = __ldg(sh.arcx + aoff + t0);
+				const uint32_t w = a.x;
+				const int32_t ol = (int32_t)(a.y & 0x3fffffff), dd = i + 1 - ol;
+				bool eq = has && (sh.packed ? a.y >> 30 == qc : __ldg(sh.graw + a.z + ol) == sh.qraw[i + 1]);
+				n_ext += __popc(__ballot_sync(FULL, eq) >> (lane & 28) & 15);
+				// arrival key 0 is never new (gwf-ed.cu:1022-1026); a state that the bound drops leaves
+				// no mark: later arrivals are dropped too
+				const bool on = has && !(w == 0 && i == -1) && (eq ? hb - 1 : hb) < T;
+				if (!__any_sync(FULL, on)) continue;
+				const int32_t id2 = bw_get(on, w, dd >> 3, a.z, (int32_t)a.w);
+				if (sh.ovf) break;
+				int32_t *const cp = blk[id2].c + (dd & 7);
+				const int32_t cw = *cp;
+				bool neu = on && !(cw & 1);
+				const uint32_t same = __match_any_sync(FULL, neu ? (id2 << 3 | (dd & 7)) : -1 - lane);
+				neu = neu && (same & lanemask_lt()) == 0;
+				const bool enter = neu && eq, two = neu && !eq;
+				if (neu) *cp = (two ? max(cw >> 1, ol) : cw >> 1) << 1 | 1;
+				const uint32_t mn = __ballot_sync(FULL, enter);
+				const int32_t pn = n_n + __popc(mn & lanemask_lt());
+				if (enter && pn < ne) sh.n[pn] = (uint32_t)id2 << 3 | (dd & 7), sh.nk[pn] = ol;
+				n_n += __popc(mn);
+				__syncwarp();
+				if (__any_sync(FULL, two)) {
+					if (two) blk[id2].has_c = 1;
+					bw_push(two, id2, np);
+					bw_cand(two && ha < T, w, dd - 1, a.z, (int32_t)a.w, ol, np);
+					if (sh.ovf) break;
+				}
+			}
+			// entered states that reached the vertex end: the diagonal has ended (gwf-ed.cu:1177-1183),
+			// and the insertion at the vertex end stays where an arc did not match
+			// (gwf-ed.cu:1225-1226). For the states of step 1 the successor rule does both.
+			if (wave > 0 && !sh.ovf) {
+				const bool one = act && (lane & 3) == 0;
+				if (one) blk[id].c[cl] = BW_ENDED << 1 | 1, blk[id].has_c = 1;
+				__syncwarp();
+				bw_push(one, id, np);
+				bw_cand(one && (n_ext != deg || deg == 0), (uint32_t)b0.z, i - vl + 2, (uint32_t)b0.x, vl, vl - 1, np);
+			}
+			if (sh.ovf) break;
+		}
+		if (n_n > ne || wave > ql + 2) sh.ovf = 1;
+		__syncwarp();
+		if (sh.ovf) break;
+		// extension of the entered states (gwf-ed.cu:1132-1160): one that stays inside its vertex
+		// joins the step's row, whose successors are its three candidates
+		int32_t n_f = 0;
+#pragma unroll 1
+		for (int32_t base = 0; base < n_n; base += 32) {
+			const bool act = base + lane < n_n;
+			const int32_t j = act ? base + lane : 0;
+			const uint32_t e = sh.n[j];
+			const int32_t id = (int32_t)(e >> 3), cl = (int32_t)(e & 7);
+			BwBlock *const B = blk + id;
+			const int32_t vl = B->vl, d = B->db + cl;
+			const int32_t k = bw_ext(sh, B->gb, d, sh.nk[j], vl, act);
+			const int32_t i = act ? d + k : INT32_MIN;
+			far = max(far, i);
+			const bool qend = i == ql - 1, in = act && !qend && k + 1 < vl, toF = act && !qend && !in;
+			found |= qend;
+			if (in && B->row[np ^ 1][cl] < k) B->row[np ^ 1][cl] = k;
+			const uint32_t mf = __ballot_sync(FULL, toF);
+			if (toF) sh.f[n_f + __popc(mf & lanemask_lt())] = (uint32_t)id << 3 | cl;
+			n_f += __popc(mf); // n_f <= n_n <= ne
+			if (__any_sync(FULL, in)) {
+				bw_push(in, id, np);
+				const bool eb = in && (cl == 0 || cl == 7);
+				if (__any_sync(FULL, eb)) bw_side(eb, id, cl, np);
+			}
+		}
+		if (__any_sync(FULL, found)) return INT32_MAX;
+		uint32_t *const t = sh.e;
+		__syncwarp();
+		sh.e = sh.f;
+		__syncwarp();
+		sh.f = t;
+		n_e = n_f;
+		__syncwarp();
+	}
+	return far;
+}
+
+// Aligns read r with one warp in the arena wsb laid out by p.bw; the hash table is empty (-1) on
+// entry and on return. All control flow is warp-uniform.
+__device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, uint8_t *wsb)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31;
+	const DevGraph &g = p.g;
+	const int32_t ql = p.r.ql[r], v0 = p.r.v0[r];
+	if (ql <= 0 || v0 < 0 || (uint32_t)v0 >= g.n_vtx) {
+		if (lane == 0) p.dist[r] = -1, p.status[r] = ST_BAD_INPUT;
+		return;
+	}
+	BwBlock *const blk = (BwBlock *)wsb;
+	__syncwarp();
+	sh.qpk = p.r.pk + p.r.pk_off[r], sh.qraw = p.r.raw + p.r.raw_off[r];
+	sh.ql = ql, sh.packed = g.pure && p.r.pure[r], sh.quirk = !(p.flags & 1);
+	__syncwarp();
+	const int32_t kmin1 = sh.quirk ? 0 : -1; // least offset of a candidate after the first step
+	const int32_t ne = p.bw.nb, max_steps = (ql < 64 ? 64 : ql) * 4 + 1024;
+
+	int32_t dist = -1, st = ST_OK, steps = 0;
+	int32_t T = BW_INF;    // states with s + h >= T are dropped
+	bool attained = false; // an alignment of T edits exists
+	bool lag = false;      // the run that looks for such a T
+	int32_t h0 = 0;
+	if (g.bloom && ql >= kPruneMinQl) {
+		h0 = bw_seeds(g.bloom_k);
+		// nearly all windows at their largest cost: the read is unlike the graph, and no bound helps
+		lag = (float)h0 < 1.7f * (float)(ql / g.bloom_k);
+	}
+	for (;;) { // runs of the score loop
+		uint32_t off_cur = p.bw.list0;
+		sh.n_blk = 0, sh.ovf = 0;
+		__syncwarp();
+		bw_get(lane == 0, (uint32_t)v0, 0, (uint32_t)__ldg(g.base + v0), (int32_t)__ldg(g.len + v0));
+		// the start state (v0, 0), k = -1, as an arc-side candidate (gwf-ed.cu:1303-1308)
+		if (lane == 0) blk[0].c[0] = -2, blk[0].has_c = 1, blk[0].inl[0] = 1, *(int32_t *)(wsb + off_cur) = 0;
+		__syncwarp();
+		int32_t n_cur = 1, imin = INT32_MIN, s = 0;
+		int32_t sc = -1; // the run's score
+#pragma unroll 1
+		for (;; ++s) {
+			const int32_t *const cur = (const int32_t *)(wsb + off_cur);
+			bool found = false, any = false;
+			int32_t n_e = 0, far = INT32_MIN;
+			if (s >= max_steps) {
+				sh.ovf = 1;
+				break;
+			}
+			// ---- 1. successors and extension of the live blocks
+			if (n_cur <= 4) {
+				// Up to four blocks: one lane per diagonal, and step after step in registers until one
+				// reaches its vertex's end or the query's, none lives, or a live edge diagonal has its
+				// neighbour outside the four blocks (unlisted blocks have no live diagonals).
+				const int gr = lane >> 3, l = lane & 7;
+				const bool has = gr < n_cur;
+				const int32_t id = cur[has ? gr : 0];
+				BwBlock *const B = blk + id;
+				const int4 b0 = *(const int4 *)B, h1 = *((const int4 *)B + 1); // gb, arcs, v, db; vl, left, right, flags
+				int32_t k = has ? B->row[~s & 1][l] : BW_NONE;
+				const uint32_t fl = (uint32_t)h1.w; // ended, has_c, inl[0], inl[1]
+				const bool edge = (0x81 >> l & 1) != 0;
+				const int32_t nid = l == 0 ? h1.y : h1.z, vl = h1.x, d = b0.w + l;
+				int src = -1; // edge lanes: the lane of the diagonal across
+#pragma unroll
+				for (int j = 0; j < 4; ++j)
+					if (__shfl_sync(FULL, id, 8 * j) == nid && j < n_cur && edge) src = 8 * j + 7 - l;
+				const bool out = edge && src < 0, nu = l == 0 && out, nd = l == 7 && out;
+				const int su = l == 0 ? max(src, 0) : lane - 1, sd = l == 7 ? max(src, 0) : lane + 1;
+				bool dead = !has || (fl >> l & 1); // absent, or past the vertex end
+				int32_t c = BW_NONE;               // the first step's arc-side candidates
+				if (__any_sync(FULL, has && (fl & 0xff00))) {
+					const int32_t cw = B->c[l];
+					if (has) c = cw >> 1, B->c[l] = 2 * BW_NONE | (cw & 1);
+				}
+				int32_t lo = s == 0 ? -1 : kmin1;
+				bool live, qend, vend;
+#pragma unroll 1
+				for (;;) {
+					const int32_t up = __shfl_sync(FULL, k, su), dn = __shfl_sync(FULL, k, sd);
+					k = max(max(nu ? BW_NONE : up, max(k, nd ? BW_NONE : dn) + 1), c);
+					dead |= k >= vl; // at the first step only: later ones follow no vertex end
+					live = !dead && k >= lo;
+					const int32_t hv = sh.h[live ? ql - 1 - d - k : 0]; // any value below BW_INF while T is BW_INF
+					live = live && s + hv < T && d + k >= imin;
+					k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
+					if (!live) k = BW_NONE;
+					far = live ? d + k : INT32_MIN;
+					qend = far == ql - 1, vend = live && k == vl - 1 && !qend;
+					const bool stop = qend || vend || (live && out) || s + 1 >= max_steps;
+					if (__any_sync(FULL, stop) || !__any_sync(FULL, live)) break;
+					if (lag) imin = __reduce_max_sync(FULL, far) - kPruneLag;
+					++s, lo = kmin1, c = BW_NONE;
+				}
+				found = qend, any = live;
+				const int par = s & 1, np = par ^ 1;
+				// back to the blocks: both rows, the ended diagonals, the next list
+				const uint32_t em = (__ballot_sync(FULL, has && dead) >> (8 * gr)) & 0xff;
+				const uint32_t ml = __ballot_sync(FULL, live);
+				if (has) B->row[par][l] = k, B->row[np][l] = BW_NONE;
+				const bool first = l == 0 && has, app = first && (ml >> (8 * gr) & 0xff) != 0;
+				if (first) *((uint32_t *)B + 7) = em | (app ? 0x10000u << (8 * np) : 0);
+				const uint32_t mp = __ballot_sync(FULL, app);
+				off_cur = par ? p.bw.list1 : p.bw.list0; // the list at hand is in registers
+				int32_t *const nxt = (int32_t *)(wsb + (par ? p.bw.list0 : p.bw.list1));
+				if (app) nxt[__popc(mp & lanemask_lt())] = id;
+				sh.nxt = nxt, sh.n_nxt = __popc(mp);
+				const uint32_t me = __ballot_sync(FULL, vend);
+				if (vend) sh.e[__popc(me & lanemask_lt())] = (uint32_t)id << 3 | l;
+				n_e = __popc(me);
+				__syncwarp();
+				// a live edge diagonal gives the neighbouring block a candidate at the next step
+				const bool act = live && edge && (src < 0 || (ml >> (src & 24) & 0xff) == 0);
+				if (__any_sync(FULL, act)) bw_side(act, id, l, np);
+			} else {
+				// More blocks: two lanes per block and four diagonals per lane; the diagonals that may
+				// live go through the warp's queue, so that the extension runs on full warps (of a dense
+				// graph's diagonals in live blocks one in four lives).
+				const int par = s & 1;
+				int2 at = make_int2(0, 0); // next block, queued diagonals
+				sh.nxt = (int32_t *)(wsb + (par ? p.bw.list0 : p.bw.list1)), sh.n_nxt = 0;
+				__syncwarp();
+#pragma unroll 1
+				do {
+					if (at.y < 32 && at.x < n_cur) at = bw_fill(cur, at.x, n_cur, at.y, par, s == 0 ? -1 : kmin1);
+					const int32_t take = min(at.y, 32); // from the queue's end
+					at.y -= take;
+					const bool alive = lane < take;
+					const uint2 e = sh.queue[at.y + (alive ? lane : 0)];
+					const int32_t id = alive ? (int32_t)(e.x >> 4) : 0, l = (int32_t)(e.x & 7);
+					int32_t k = (int32_t)e.y;
+					const int4 b0 = *(const int4 *)(blk + id);
+					const int32_t vl = blk[id].vl, d = b0.w + l;
+					const int32_t hv = sh.h[alive ? ql - 1 - d - k : 0];
+					const bool live = alive && s + hv < T && d + k >= imin;
+					k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
+					if (live) blk[id].row[par][l] = k;
+					const int32_t i = live ? d + k : INT32_MIN;
+					far = max(far, i);
+					const bool qend = i == ql - 1, vend = live && k == vl - 1 && !qend;
+					found |= qend;
+					any |= live;
+					const uint32_t me = __ballot_sync(FULL, vend);
+					if (me) {
+						const int32_t pos = n_e + __popc(me & lanemask_lt());
+						if (vend && pos < ne) sh.e[pos] = (uint32_t)id << 3 | l;
+						n_e += __popc(me);
+					}
+					// a neighbour whose diagonal beside it was live stays listed by itself
+					const bool act = live && (e.x & 8);
+					if (__any_sync(FULL, act)) {
+						bw_side(act, id, l, par ^ 1);
+						if (sh.ovf) break;
+					}
+				} while (at.x < n_cur || at.y > 0);
+				__syncwarp();
+			}
+			if (__any_sync(FULL, found)) {
+				sc = s;
+				break;
+			}
+			if (!__any_sync(FULL, any)) break; // no state is left
+			// ---- 2. vertex-end states over arcs
+			if (n_e > ne) sh.ovf = 1;
+			__syncwarp();
+			if (sh.ovf) break;
+			if (n_e > 0) {
+				far = max(far, bw_waves(s, T, n_e));
+				if (__any_sync(FULL, far == INT32_MAX)) {
+					sc = s;
+					break;
+				}
+				if (sh.ovf) break;
+			}
+			n_cur = sh.n_nxt;
+			off_cur = s & 1 ? p.bw.list0 : p.bw.list1;
+			if (lag) imin = __reduce_max_sync(FULL, far) - kPruneLag;
+		}
+		// the hash table back to empty
+		__syncwarp();
+		const int32_t n_blk = sh.n_blk;
+		const bool ovf = sh.ovf != 0;
+#pragma unroll 1
+		for (int32_t j = lane; j < n_blk; j += 32) sh.hash[sh.slot[j]].y = 0xffffffffu;
+		__syncwarp();
+		if (lag) { // its score, where it found one, is the bound
+			lag = false;
+			if (sc >= 0) {
+				attained = true, T = sc;
+				// The exact run makes about beta / 4 slack^2 iterations of step 1 more than one per
+				// score (slack = T - h; beta 1.2 measured on the sparse benchmark graph, 4 to 14 on the
+				// dense one); windows from every base cost the time of ~0.2 per base and make the
+				// slack 2.2 times smaller.
+				const float slack = (float)(T - h0);
+				if ((p.dens_milli >= 20 ? 8.0f : 1.2f) * slack * slack > (float)ql) bw_seeds(1);
+			}
+			continue;
+		}
+		if (ovf && sc < 0) {
+			st = ST_CAPACITY, steps = s + 1;
+			break;
+		}
+		dist = sc >= 0 ? sc : attained ? T : -1;
+		steps = dist >= 0 ? dist + 1 : s;
+		break;
+	}
+	if (lane == 0) {
+		p.dist[r] = st == ST_OK ? dist : -1;
+		p.status[r] = st;
+		if (st == ST_CAPACITY && p.retry_list) {
+			const int32_t q = atomicAdd(p.retry_n, 1);
+			p.retry_list[q] = r;
+		}
+		if (p.steps_out) p.steps_out[r] = steps;
+	}
+}
+
+// Persistent form: each one-warp CTA owns one arena (p.bw, sized for the longest read of the
+// launch) and pulls reads from the cost-ordered queue.
+__global__ void __launch_bounds__(32, 32) k_align_blocks(const __grid_constant__ KParams p)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x;
+	uint8_t *const wsb = p.ws + (int64_t)blockIdx.x * p.bw.total;
+	if (lane == 0) {
+		sh.blk = (BwBlock *)wsb, sh.hash = (uint2 *)(wsb + p.bw.hash), sh.slot = (uint32_t *)(wsb + p.bw.slot);
+		sh.e = (uint32_t *)(wsb + p.bw.e), sh.f = (uint32_t *)(wsb + p.bw.f), sh.n = (uint32_t *)(wsb + p.bw.n);
+		sh.nk = (int32_t *)(wsb + p.bw.nk), sh.h = (uint16_t *)(wsb + p.bw.h);
+		sh.gpk = (const uint32_t *)p.g.pk, sh.graw = p.g.raw, sh.arcx = p.g.arcx, sh.varcs = p.g.varcs;
+		sh.arc_off = p.g.arc_off, sh.bloom = p.g.bloom, sh.bloom_mask = p.g.bloom_mask, sh.K = p.g.bloom_k;
+		sh.hmask = (uint32_t)p.bw.hs - 1, sh.nb = p.bw.nb;
+	}
+	{
+		int4 *const h4 = (int4 *)(wsb + p.bw.hash);
+#pragma unroll 1
+		for (int32_t j = lane; j < p.bw.hs / 2; j += 32) h4[j] = make_int4(-1, -1, -1, -1);
+	}
+	__syncwarp();
+#pragma unroll 1
+	for (int32_t guard = 0; guard < p.n_order + 1; ++guard) {
+		int32_t qi = 0;
+		if (lane == 0) qi = atomicAdd(p.head, 1);
+		qi = __shfl_sync(FULL, qi, 0);
+		if (qi >= p.n_order) break;
+		align_read_blocks(p, p.order[qi], wsb);
+	}
+}
+#endif
+
+} // namespace gwfb

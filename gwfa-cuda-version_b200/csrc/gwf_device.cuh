@@ -33,6 +33,8 @@ constexpr int32_t ST_OK = 0;
 constexpr int32_t ST_BAD_INPUT = -2;
 constexpr int32_t ST_CAPACITY = -4;
 
+constexpr uint32_t kVArcsBits = 28, kVArcsMask = (1u << kVArcsBits) - 1, kVArcsMany = 15;
+
 struct DevGraph {
 	const uint32_t *len;     // [n_vtx]
 	const uint64_t *base;    // [n_vtx] first base of the vertex in the concatenated sequence
@@ -42,6 +44,13 @@ struct DevGraph {
 	const uint2 *arc;        // (target, overlap)
 	const uint32_t *arc_key; // vertex part of the arrival key per arc (entry id), or null when
 	                         // every vertex's in-arcs share one overlap (the key is the target)
+	const uint4 *arcx;       // per arc: target, overlap | code of the base entered << 30, first base of
+	                         // the target in the concatenation, its length (graphs of < 2^30 bases)
+	const uint32_t *varcs;   // per vertex: first arc | arcs << kVArcsBits (kVArcsMany = look up arc_off)
+	const uint64_t *bloom;   // filter of the strings of bloom_k bases that walks spell, or null
+	uint32_t bloom_mask;     // words - 1
+	int32_t bloom_k;         // 14 to 16
+	uint64_t total_len;      // bases of all vertices
 	uint32_t n_vtx;
 	int32_t pure;            // 1 when every graph byte is A/C/G/T
 };

@@ -5,6 +5,38 @@
 
 namespace gwfb {
 
+// Block form (gwf_blocks.cuh): byte offsets of a warp's arena, which starts with the blocks.
+struct BwLay {
+	uint32_t hash, slot, list0, list1, e, f, n, nk, h;
+	int32_t nb, hs; // blocks, hash slots (power of two)
+	int64_t total;
+};
+
+// Arena for reads of up to ql bases at retry class level (0, 1) on a graph of dens_milli vertices
+// per 1000 bases. Pruned runs of 10 kbp reads at 5% on the dense benchmark graph make ~1,000
+// blocks (34,000 unpruned), 20 kbp reads at 10% ~33,000, 1 kbp reads on the sparse graph ~50.
+__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli)
+{
+	const int64_t q = ql < 64 ? 64 : ql;
+	int64_t nb = 128 + q / 2 + (int64_t)dens_milli * q * q / 400000 + (int64_t)dens_milli * q * 8 / 1000;
+	if (level > 0) nb *= 8;
+	if (nb > (1 << 22)) nb = 1 << 22;
+	BwLay o;
+	o.nb = (int32_t)nb, o.hs = pow2ceil_i(2 * o.nb);
+	int64_t at = 128 * nb;
+	o.hash = (uint32_t)at, at += 8LL * o.hs;
+	o.slot = (uint32_t)at, at = al16(at + 4 * nb);
+	o.list0 = (uint32_t)at, at = al16(at + 4 * nb);
+	o.list1 = (uint32_t)at, at = al16(at + 4 * nb);
+	o.e = (uint32_t)at, at = al16(at + 4 * nb);
+	o.f = (uint32_t)at, at = al16(at + 4 * nb);
+	o.n = (uint32_t)at, at = al16(at + 4 * nb);
+	o.nk = (uint32_t)at, at = al16(at + 4 * nb);
+	o.h = (uint32_t)at, at = al16(at + 2 * (q + 2)); // at most 2^22 * 200 bytes: offsets fit 32 bits
+	o.total = (at + 127) & ~127LL;
+	return o;
+}
+
 struct KParams {
 	DevGraph g;
 	DevReads r;
@@ -32,6 +64,7 @@ struct KParams {
 	int32_t *path_v;        // path vertices from v0
 	int32_t *path_arc;      // arc index into path_v[j] (-1 for j = 0)
 	int32_t max_nv;
+	BwLay bw;               // block form: layout of a warp's arena
 };
 
 // ---- serving: one resident kernel, warps pull single reads from a device queue

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "../../include/gwfa.h"
+#include "gwf_blocks.cuh"
 #include "gwf_cigar.cuh"
 #include "gwf_group.cuh"
 #include "gwf_kernels.cuh"
@@ -133,6 +134,12 @@ DevGraph GraphDev::view() const
 	v.arc_off = (const uint32_t *)arc_off.p;
 	v.arc = (const uint2 *)arc.p;
 	v.arc_key = (const uint32_t *)arc_key.p;
+	v.arcx = (const uint4 *)arcx.p;
+	v.varcs = (const uint32_t *)varcs.p;
+	v.bloom = (const uint64_t *)bloom.p;
+	v.bloom_mask = bloom_mask;
+	v.bloom_k = bloom_k;
+	v.total_len = total_len;
 	v.n_vtx = n_vtx;
 	v.pure = pure;
 	return v;
@@ -144,7 +151,7 @@ GraphDev::~GraphDev()
 	cudaGetDevice(&cur);
 	if (device >= 0) cudaSetDevice(device);
 	len.release(), base.release(), pk.release(), raw.release(), arc_off.release(), arc.release();
-	arc_key.release();
+	arc_key.release(), arcx.release(), varcs.release(), bloom.release();
 	if (cur >= 0) cudaSetDevice(cur);
 }
 
@@ -156,6 +163,43 @@ GraphDev *gwf_find_graph(const gwf_graph_t *g)
 }
 
 static uint8_t code2(uint8_t c) { return (uint8_t)((c >> 1) & 3); } // A0 C1 T2 G3
+
+// Filter of the strings of K bases that the graph's walks spell (exact pruning, gwf_blocks.cuh):
+// one 64-bit word per base, as a power of two, so about one string per word (5 Mbp: 64 MiB). K is
+// the smallest of 14 to 16 at which few of a window's ~11 K one-edit neighbours are present by
+// chance (4^14 = 2^28 against 2^18 bases and ~160 neighbours: 15%). A graph with other bytes than
+// A/C/G/T, of more than 2^26 bases, without room for it, or with too many walks from one base gets
+// none.
+static int build_bloom(GraphDev *G)
+{
+	if (!G->pure || G->total_len > (1ULL << 26)) return 0;
+	uint32_t words = 1024;
+	while (words < G->total_len) words <<= 1;
+	if (words <= (1u << 20)) words <<= 1; // half a string per word where that stays small
+	DBuf many;
+	if (G->bloom.ensure(8 * (size_t)words) || many.ensure(4)) {
+		G->bloom.release(), many.release();
+		return 0;
+	}
+	G->bloom_mask = words - 1;
+	G->bloom_k = G->total_len <= (1u << 18) ? 14 : G->total_len <= (1u << 20) ? 15 : 16;
+	int32_t h_many = 0;
+	cudaError_t e = cudaMemset(G->bloom.p, 0, 8 * (size_t)words);
+	if (e == cudaSuccess) e = cudaMemset(many.p, 0, 4);
+	if (e == cudaSuccess) {
+		DevGraph v = G->view();
+		k_bloom<<<(G->n_vtx + 7) / 8, 256>>>(v, (unsigned long long *)G->bloom.p, (int32_t *)many.p);
+		e = cudaGetLastError();
+	}
+	if (e == cudaSuccess) e = cudaMemcpy(&h_many, many.p, 4, cudaMemcpyDeviceToHost);
+	many.release();
+	if (e != cudaSuccess) {
+		gwf_set_errorf("building the graph's filter failed: %s", cudaGetErrorString(e));
+		return GWF_E_CUDA;
+	}
+	if (h_many) G->bloom.release();
+	return 0;
+}
 
 static int upload_graph(const gwf_graph_t *g, GraphDev *G)
 {
@@ -234,7 +278,20 @@ static int upload_graph(const gwf_graph_t *g, GraphDev *G)
 		if ((rc = G->arc_key.ensure(sizeof(uint32_t) * key.size()))) return rc;
 		CK(cudaMemcpy(G->arc_key.p, key.data(), sizeof(uint32_t) * key.size(), cudaMemcpyHostToDevice));
 	}
-	return 0;
+	// arc records of the block form (one load per arc): graphs of < 2^30 bases and < 2^28 arcs
+	if (tot < (1ULL << 30) && g->n_arc < kVArcsMask) {
+		std::vector<uint4> ax(arc.size());
+		std::vector<uint32_t> va(std::max<size_t>(nv, 1));
+		for (uint32_t e = 0; e < g->n_arc; ++e) {
+			const uint32_t w = arc[e].x, o = arc[e].y, code = code2((uint8_t)g->seq[w][o]);
+			ax[e] = make_uint4(w, o | code << 30, (uint32_t)base[w], len[w]);
+		}
+		for (uint32_t v = 0; v < nv; ++v) va[v] = off[v] | std::min(off[v + 1] - off[v], kVArcsMany) << kVArcsBits;
+		if ((rc = G->arcx.ensure(16 * ax.size())) || (rc = G->varcs.ensure(4 * va.size()))) return rc;
+		CK(cudaMemcpy(G->arcx.p, ax.data(), 16 * ax.size(), cudaMemcpyHostToDevice));
+		CK(cudaMemcpy(G->varcs.p, va.data(), 4 * va.size(), cudaMemcpyHostToDevice));
+	}
+	return build_bloom(G);
 }
 
 extern "C" void gwf_ed_index(gwf_graph_t *g)
@@ -339,6 +396,9 @@ Engine *gwf_engine(int dev)
 	int occ = 0;
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_persistent<false>, 256, 0);
 	E->persistent_ctas_per_sm = occ > 0 ? occ : 1;
+	occ = 0;
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_blocks, 32, sizeof(BwShm));
+	E->blocks_warps_per_sm = occ > 0 ? occ : 1;
 	occ = 0;
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_classes, 256, 0);
 	E->classes_ctas_per_sm = occ > 0 ? occ : 1;
@@ -566,6 +626,42 @@ static int enqueue_persistent(Engine &E, KParams p, const PersistPlan &pl, const
 	return 0;
 }
 
+// ---- block form (gwf_blocks.cuh): the persistent queue on block wavefronts. It takes every read
+// that ends at the query's end (no target vertex) on a graph whose in-arcs share one overlap per
+// vertex; lag pruning as an option, targets and mixed overlaps stay with the sorted form.
+static bool blocks_ok(const KParams &p) { return p.r.v1 < 0 && p.max_lag == 0 && p.g.arc_key == nullptr && p.g.arcx != nullptr; }
+
+static int plan_blocks(Engine &E, KParams *p, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
+                       PersistPlan *pl)
+{
+	p->bw = bw_layout(ql_cap, level, p->dens_milli);
+	int64_t warps = std::min<int64_t>((int64_t)E.sm_count * warps_per_sm, n_order);
+	const int64_t budget = std::max<int64_t>(E.mem_budget, (int64_t)E.ws.cap);
+	warps = std::min(warps, budget / p->bw.total);
+	if (warps < 1) {
+		gwf_set_errorf("arena of %lld bytes per warp does not fit the device", (long long)p->bw.total);
+		return GWF_E_NOMEM;
+	}
+	int rc;
+	if ((rc = E.ws.ensure((size_t)(warps * p->bw.total)))) return rc;
+	if ((rc = E.head.ensure(16))) return rc;
+	pl->ctas = (int)warps;
+	pl->slot = p->bw.total;
+	return 0;
+}
+
+static int enqueue_blocks(Engine &E, KParams p, const PersistPlan &pl, const int32_t *d_order, int32_t n_order)
+{
+	CK(cudaMemsetAsync(E.head.p, 0, 4, E.stream));
+	p.order = d_order;
+	p.n_order = n_order;
+	p.head = (int32_t *)E.head.p;
+	p.ws = (uint8_t *)E.ws.p;
+	k_align_blocks<<<pl.ctas, 32, sizeof(BwShm), E.stream>>>(p);
+	CK(cudaGetLastError());
+	return 0;
+}
+
 // Persistent launch over the reads listed in d_order (device), arenas sized for ql_cap.
 static int launch_persistent(Engine &E, KParams p, const int32_t *d_order, int32_t n_order,
                              int32_t ql_cap, int32_t level, int ctas_per_sm, int *launches)
@@ -789,12 +885,14 @@ static int enqueue_classes(Engine &E, KParams p, const ClassLaunch &cl)
 // Level-0 sequence of the persistent form as one CUDA graph: pack, clear the overflow count,
 // persistent kernel, copy the overflow count to the host. Captured once per batch contents and
 // launch shape, replayed on every run.
-static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_per_sm, bool classes)
+static int launch_level0_graph(Engine &E, Batch &B, KParams &p, int ctas_per_sm, bool classes, bool blocks)
 {
 	PersistPlan pl;
 	ClassLaunch cl;
 	int rc;
-	if (classes) {
+	if (blocks) {
+		if ((rc = plan_blocks(E, &p, B.n, B.max_ql, 0, ctas_per_sm, &pl))) return rc;
+	} else if (classes) {
 		if ((rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl))) return rc;
 		pl.ctas = cl.ctas, pl.slot = cl.cp.cta_bytes;
 	} else if ((rc = plan_persistent(E, B.n, B.max_ql, 0, ctas_per_sm, p.dens_milli, &pl)))
@@ -803,13 +901,14 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 	                         (uint64_t)(uint32_t)p.flags | (uint64_t)(uint32_t)p.max_lag << 32,
 	                         (uint64_t)(uintptr_t)E.retry_n.p,
 	                         (uint64_t)(uintptr_t)E.h_small.p, (uint64_t)(uintptr_t)E.retry_list.p,
-	                         classes ? B.cls_key ^ B.cls_gen << 40 : ~0ULL};
+	                         blocks ? ~1ULL : classes ? B.cls_key ^ B.cls_gen << 40 : ~0ULL};
 	if (!B.gexec || memcmp(key, B.gkey, sizeof key) != 0) {
 		if (B.gexec) cudaGraphExecDestroy(B.gexec), B.gexec = nullptr;
 		CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
 		int erc = enqueue_pack(E, B);
 		if (!erc && cudaMemsetAsync(E.retry_n.p, 0, 4, E.stream) != cudaSuccess) erc = GWF_E_CUDA;
-		if (!erc) erc = classes ? enqueue_classes(E, p, cl)
+		if (!erc) erc = blocks ? enqueue_blocks(E, p, pl, (const int32_t *)B.order_ql.p, B.n)
+		                : classes ? enqueue_classes(E, p, cl)
 		                        : enqueue_persistent(E, p, pl, (const int32_t *)B.order_ql.p, B.n, B.max_ql, 0);
 		if (!erc && cudaMemcpyAsync(E.h_small.p, E.retry_n.p, 4, cudaMemcpyDeviceToHost, E.stream) != cudaSuccess)
 			erc = GWF_E_CUDA;
@@ -863,16 +962,20 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		if (gwf_tune_lookup(E.device, B.dom_bucket, &f, &c)) mode = f, ctas_per_sm = c;
 	}
 	bool classes = false;
-	if (mode != GWF_MODE_PLAIN) {
+	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p) &&
+	                    *std::max_element(nw_b, nw_b + GWF_TUNE_NBUCKETS) <= 1;
+	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;
 		classes = B.cls_n > 1 || B.cls_nw[0] > 1;
 	}
-	if (ctas_per_sm <= 0) ctas_per_sm = classes ? E.classes_ctas_per_sm : E.persistent_ctas_per_sm;
+	const int warps_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm * kWarpsPerCta, E.blocks_warps_per_sm) : E.blocks_warps_per_sm;
+	if (ctas_per_sm <= 0)
+		ctas_per_sm = classes ? E.classes_ctas_per_sm : E.persistent_ctas_per_sm;
 	bool count_copied = false;
 	CK(cudaEventRecord(E.ev0, E.stream));
 	if (use_graph && mode != GWF_MODE_PLAIN) {
-		if ((rc = launch_level0_graph(E, B, p, ctas_per_sm, classes))) return rc;
+		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks))) return rc;
 		launches += 2;
 		count_copied = true;
 	} else {
@@ -880,7 +983,12 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		++launches;
 		CK(cudaMemsetAsync(E.retry_n.p, 0, 4, E.stream));
 		if (mode == GWF_MODE_PLAIN) rc = launch_plain(E, p, B, &launches);
-		else if (classes) {
+		else if (blocks) {
+			PersistPlan pl;
+			if (!(rc = plan_blocks(E, &p, B.n, B.max_ql, 0, warps_per_sm, &pl)) &&
+			    !(rc = enqueue_blocks(E, p, pl, (const int32_t *)B.order_ql.p, B.n)))
+				++launches;
+		} else if (classes) {
 			ClassLaunch cl;
 			if (!(rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl)) && !(rc = enqueue_classes(E, p, cl)))
 				++launches;
@@ -888,8 +996,9 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 			rc = launch_persistent(E, p, (const int32_t *)B.order_ql.p, B.n, B.max_ql, 0, ctas_per_sm, &launches);
 		if (rc) return rc;
 	}
-	// re-run arena overflows at larger size classes
-	for (int level = 1; level <= kMaxLevel; ++level) {
+	// re-run arena overflows at larger size classes (the block form's first in a larger arena of its
+	// own, then as the sorted form's)
+	for (int level = blocks ? 0 : 1; level <= kMaxLevel; ++level) {
 		int32_t nr = 0;
 		if (!count_copied) CK(cudaMemcpyAsync(E.h_small.p, E.retry_n.p, 4, cudaMemcpyDeviceToHost, E.stream));
 		count_copied = false;
@@ -907,6 +1016,14 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		CK(cudaMemcpyAsync(E.order.p, ids.data(), 4 * (size_t)nr, cudaMemcpyHostToDevice, E.stream));
 		CK(cudaMemsetAsync(E.retry_n.p, 0, 4, E.stream));
 		KParams q = p;
+		if (level == 0) {
+			PersistPlan pl;
+			if ((rc = plan_blocks(E, &q, nr, cap, 1, warps_per_sm, &pl)) ||
+			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr)))
+				return rc;
+			++launches;
+			continue;
+		}
 		if (level == kMaxLevel) q.retry_list = nullptr; // last class: keep GWF_E_CAPACITY
 		if ((rc = launch_persistent(E, q, (const int32_t *)E.order.p, nr, cap, level,
 		                            std::min(ctas_per_sm, E.persistent_ctas_per_sm), &launches)))

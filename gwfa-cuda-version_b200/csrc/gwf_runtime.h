@@ -29,6 +29,10 @@ struct GraphDev { // device-resident copy of one gwf_graph_t
 	uint64_t total_len = 0;
 	DBuf len, base, pk, raw, arc_off, arc;
 	DBuf arc_key; // entry id per arc, only when some vertex's in-arcs carry different overlaps
+	DBuf arcx, varcs; // arc records and arc ranges of the block form (empty on graphs it does not take)
+	DBuf bloom;   // filter of the walks' strings of bloom_k bases (bloom_mask + 1 words), or empty
+	uint32_t bloom_mask = 0;
+	int32_t bloom_k = 16;
 	gwfb::DevGraph view() const;
 	~GraphDev();
 };
@@ -38,6 +42,7 @@ struct Engine { // per-device launch state: stream, events, warp arenas
 	int sm_count = 0;
 	int persistent_ctas_per_sm = 1;
 	int classes_ctas_per_sm = 1;
+	int blocks_warps_per_sm = 1;
 	int64_t mem_budget = 0; // device bytes the arenas may take
 	cudaStream_t stream = nullptr;
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
