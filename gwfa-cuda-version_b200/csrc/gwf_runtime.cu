@@ -12,7 +12,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <iterator>
 #include <numeric>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 
@@ -108,11 +110,12 @@ int gwf_select_device(int want, int *dev_out)
 		gwf_set_error("device ordinal out of range");
 		return GWF_E_BAD_INPUT;
 	}
-	cudaDeviceProp prop;
-	CK(cudaGetDeviceProperties(&prop, dev));
-	if (prop.major != 10) {
-		gwf_set_errorf("device %d is sm_%d%d; this library is built for sm_100a (B200) only", dev,
-		               prop.major, prop.minor);
+	// one attribute, not cudaGetDeviceProperties: that call takes ~2.5 ms, and every entry point comes here
+	int major = 0, minor = 0;
+	CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
+	if (major != 10) {
+		CK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev));
+		gwf_set_errorf("device %d is sm_%d%d; this library is built for sm_100a (B200) only", dev, major, minor);
 		return GWF_E_CUDA;
 	}
 	CK(cudaSetDevice(dev));
@@ -357,7 +360,7 @@ extern "C" void gwf_cleanup(gwf_graph_t *g)
 Engine::~Engine()
 {
 	cudaSetDevice(device);
-	for (DBuf *b : {&pk_off, &order, &head, &retry_list, &retry_n, &ws, &slot_off, &w_out})
+	for (DBuf *b : {&order, &head, &retry_list, &ws, &slot_off})
 		b->release();
 	for (HBuf *b : {&h_small, &h_stage}) b->release();
 	for (cudaEvent_t e : stage_ev)
@@ -380,8 +383,9 @@ Engine *gwf_engine(int dev)
 	cudaSetDevice(dev);
 	if (cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking) != cudaSuccess ||
 	    cudaEventCreate(&E->ev0) != cudaSuccess || cudaEventCreate(&E->ev1) != cudaSuccess ||
-	    cudaEventCreateWithFlags(&E->stage_ev[0], cudaEventDisableTiming) != cudaSuccess ||
-	    cudaEventCreateWithFlags(&E->stage_ev[1], cudaEventDisableTiming) != cudaSuccess) {
+	    !std::all_of(std::begin(E->stage_ev), std::end(E->stage_ev), [](cudaEvent_t &e) {
+		    return cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+	    })) {
 		cudaGetLastError();
 		gwf_set_error("stream/event creation failed");
 		delete E;
@@ -409,43 +413,69 @@ Engine *gwf_engine(int dev)
 // ------------------------------------------------------------------ batches
 void Batch::release()
 {
-	for (DBuf *b : {&raw, &raw_off, &ql, &v0, &pk, &pk_off, &pure, &dist, &status, &steps, &order_ql, &order_cls})
+	for (DBuf *b : {&in, &raw, &pk, &pure, &res, &steps, &order_cls})
 		b->release();
 	cls_key = ~0ULL, cls_gen = ~0ULL;
 	h_meta.release();
 	if (gexec) cudaGraphExecDestroy(gexec), gexec = nullptr;
 }
 
-// Copies n reads (host, concatenated) into the batch's device buffers; computes host-side
-// layout (packed offsets, cost order).
-// Host-to-device copy on the engine's stream. A page-locked source goes to the DMA engine as
-// it is; a pageable one of more than 1 MiB passes through two pinned 8 MiB chunks in turn, so
-// that filling one chunk overlaps the transfer of the other.
 static const int kWarpsPerCtaPack = 8; // warps per CTA of the per-read helper kernels
+
+// Host-to-device copy on the engine's stream. A page-locked source goes to the DMA engine as it is.
+// A pageable one of more than 4 MiB passes through pinned 4 MiB chunks, two per thread, so that the
+// copies into the chunks overlap the transfers and each other: one thread fills ~10 GB/s, the link
+// takes ~50 (100 MB: 10 ms with one thread, 3 with four).
+static const size_t kStageChunk = (size_t)4 << 20;
+
+static cudaError_t stage_chunks(Engine &E, char *dst, const char *src, size_t n, int t, int threads)
+{
+	cudaError_t e = cudaSetDevice(E.device);
+	int i = 0;
+	for (size_t off = (size_t)t * kStageChunk; e == cudaSuccess && off < n; off += (size_t)threads * kStageChunk, ++i) {
+		const int b = 2 * t + (i & 1);
+		const size_t len = std::min(kStageChunk, n - off);
+		char *stage = (char *)E.h_stage.p + (size_t)b * kStageChunk;
+		e = cudaEventSynchronize(E.stage_ev[b]); // the transfer that last read this chunk, if any
+		if (e != cudaSuccess) break;
+		memcpy(stage, src + off, len);
+		e = cudaMemcpyAsync(dst + off, stage, len, cudaMemcpyHostToDevice, E.stream);
+		if (e == cudaSuccess) e = cudaEventRecord(E.stage_ev[b], E.stream);
+	}
+	return e;
+}
 
 static int upload(Engine &E, void *dst, const void *src, size_t n)
 {
 	cudaPointerAttributes at;
 	const bool pinned = cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeHost;
 	cudaGetLastError();
-	if (pinned || n <= ((size_t)1 << 20)) {
+	if (pinned || n <= kStageChunk) {
 		CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, E.stream));
 		return 0;
 	}
-	const size_t chunk = (size_t)8 << 20;
 	int rc;
-	if ((rc = E.h_stage.ensure(2 * chunk))) return rc;
-	for (size_t off = 0, i = 0; off < n; off += chunk, ++i) {
-		const size_t b = i & 1, len = std::min(chunk, n - off);
-		CK(cudaEventSynchronize(E.stage_ev[b])); // the DMA that last read this chunk, if any
-		char *stage = (char *)E.h_stage.p + b * chunk;
-		memcpy(stage, (const char *)src + off, len);
-		CK(cudaMemcpyAsync((char *)dst + off, stage, len, cudaMemcpyHostToDevice, E.stream));
-		CK(cudaEventRecord(E.stage_ev[b], E.stream));
+	if ((rc = E.h_stage.ensure(2 * kStageThreads * kStageChunk))) return rc;
+	const int threads = (int)std::min<size_t>(kStageThreads, (n + kStageChunk - 1) / kStageChunk);
+	cudaError_t err[kStageThreads] = {};
+	std::thread th[kStageThreads];
+	for (int t = 1; t < threads; ++t) {
+		try {
+			th[t] = std::thread([&, t] { err[t] = stage_chunks(E, (char *)dst, (const char *)src, n, t, threads); });
+		} catch (...) { // no thread to be had: its chunks from here
+			err[t] = stage_chunks(E, (char *)dst, (const char *)src, n, t, threads);
+		}
 	}
+	err[0] = stage_chunks(E, (char *)dst, (const char *)src, n, 0, threads);
+	for (int t = 1; t < threads; ++t)
+		if (th[t].joinable()) th[t].join();
+	for (int t = 0; t < threads; ++t) CK(err[t]);
 	return 0;
 }
 
+// Copies n reads (host, concatenated) into the batch's device buffers; computes the host-side
+// layout (packed offsets, cost order). Everything but the bases of a large batch goes up in one
+// copy from pinned memory.
 int gwf_batch_load(Engine &E, Batch &B, int32_t n_in, const char *seqs, const int64_t *offs,
                    const int32_t *ql_in, const int32_t *v0, int32_t v1, bool both)
 {
@@ -453,7 +483,7 @@ int gwf_batch_load(Engine &E, Batch &B, int32_t n_in, const char *seqs, const in
 	// i, made on the device, with the same v0
 	const int32_t n = both ? 2 * n_in : n_in;
 	if (both && n_in > INT32_MAX / 2) return GWF_E_BAD_INPUT;
-	B.n = n, B.n_in = n_in, B.both = both, B.v1 = v1;
+	B.n = n, B.n_in = n_in, B.both = both, B.v1 = v1, B.fetched = false;
 	++B.generation;
 	B.h_ql.assign(ql_in, ql_in + n_in);
 	if (both) B.h_ql.insert(B.h_ql.end(), ql_in, ql_in + n_in);
@@ -468,14 +498,23 @@ int gwf_batch_load(Engine &E, Batch &B, int32_t n_in, const char *seqs, const in
 		}
 	}
 	const int64_t span = hi - lo, rc_base = span + 16; // the reverse complements after the reads
-	// pinned metadata: raw offsets and packed offsets (int64), queue order (int32)
+	// pinned input block: raw offsets, packed offsets (int64), lengths, start vertices, queue order
+	// (int32), and the bases of a small batch
+	const size_t nraw = (size_t)(both ? 2 * rc_base : rc_base), o_raw = (28 * (size_t)n + 15) & ~(size_t)15;
+	const bool small = span <= (int64_t)1 << 18;
 	int rc;
-	if ((rc = B.h_meta.ensure(20 * (size_t)n + 64))) return rc;
-	int64_t *h_raw_off = (int64_t *)B.h_meta.p, *h_pk_off = h_raw_off + n;
-	int32_t *h_order = (int32_t *)(h_pk_off + n);
+	if ((rc = B.h_meta.ensure(o_raw + (small ? (size_t)span + 16 : 0) + 64))) return rc;
+	char *const hm = (char *)B.h_meta.p;
+	int64_t *h_raw_off = (int64_t *)hm, *h_pk_off = h_raw_off + n;
+	int32_t *h_ql = (int32_t *)(h_pk_off + n), *h_v0 = h_ql + n, *h_order = h_v0 + n;
 	for (int32_t i = 0; i < n_in; ++i) h_raw_off[i] = offs[i] - lo;
 	if (both)
 		for (int32_t i = 0; i < n_in; ++i) h_raw_off[n_in + i] = rc_base + offs[i] - lo;
+	memcpy(h_ql, ql, 4 * (size_t)n);
+	memcpy(h_v0, v0, 4 * (size_t)n_in);
+	if (both) memcpy(h_v0 + n_in, v0, 4 * (size_t)n_in);
+	if (small && span > 0) memcpy(hm + o_raw, seqs + lo, (size_t)span);
+	if (small) memset(hm + o_raw + span, 0, 16);
 	int64_t words = 0;
 	for (int32_t i = 0; i < n; ++i) h_pk_off[i] = words, words += (ql[i] + 31) / 32 + 2;
 	B.pk_words = words;
@@ -495,32 +534,28 @@ int gwf_batch_load(Engine &E, Batch &B, int32_t n_in, const char *seqs, const in
 		for (int32_t b = 0; b < nb; ++b) cnt[(size_t)b + 1] += cnt[(size_t)b];
 		for (int32_t i = 0; i < n; ++i) h_order[cnt[(size_t)(nb - 1 - (ql[i] >> 6))]++] = i;
 	}
-	const size_t nraw = (size_t)(both ? 2 * rc_base : rc_base);
-	if ((rc = B.raw.ensure(nraw)) || (rc = B.raw_off.ensure(8 * (size_t)n + 8)) ||
-	    (rc = B.ql.ensure(4 * (size_t)n + 4)) || (rc = B.v0.ensure(4 * (size_t)n + 4)) ||
-	    (rc = B.pk.ensure(8 * (size_t)words + 8)) || (rc = B.pk_off.ensure(8 * (size_t)n + 8)) ||
-	    (rc = B.pure.ensure((size_t)n + 8)) || (rc = B.dist.ensure(4 * (size_t)n + 4)) ||
-	    (rc = B.status.ensure(4 * (size_t)n + 4)) || (rc = B.steps.ensure(4 * (size_t)n + 4)) ||
-	    (rc = B.order_ql.ensure(4 * (size_t)n + 4)))
+	if ((rc = B.in.ensure(o_raw + (small ? nraw : 0) + 64)) || (rc = B.pk.ensure(8 * (size_t)words + 8)) ||
+	    (rc = B.pure.ensure((size_t)n + 8)) || (rc = B.res.ensure(8 * (size_t)n + 16)) ||
+	    (rc = B.steps.ensure(4 * (size_t)n + 4)) || (!small && (rc = B.raw.ensure(nraw))))
 		return rc;
+	char *const dm = (char *)B.in.p;
+	B.d_raw_off = (int64_t *)dm, B.d_pk_off = B.d_raw_off + n;
+	B.d_ql = (int32_t *)(B.d_pk_off + n), B.d_v0 = B.d_ql + n, B.d_order = B.d_v0 + n;
+	B.d_raw = small ? (uint8_t *)dm + o_raw : (uint8_t *)B.raw.p;
+	B.d_dist = (int32_t *)B.res.p, B.d_status = B.d_dist + n, B.d_count = B.d_status + n;
 	cudaStream_t s = E.stream;
 	if (n > 0) {
-		if ((rc = upload(E, B.raw.p, seqs + lo, (size_t)span))) return rc;
-		CK(cudaMemsetAsync((char *)B.raw.p + span, 0, 16, s));
-		CK(cudaMemcpyAsync(B.raw_off.p, h_raw_off, 8 * (size_t)n, cudaMemcpyHostToDevice, s));
-		if ((rc = upload(E, B.ql.p, ql_in, 4 * (size_t)n_in)) || (rc = upload(E, B.v0.p, v0, 4 * (size_t)n_in)))
-			return rc;
+		if (!small) {
+			if ((rc = upload(E, B.d_raw, seqs + lo, (size_t)span))) return rc;
+			CK(cudaMemsetAsync(B.d_raw + span, 0, 16, s));
+		}
+		CK(cudaMemcpyAsync(dm, hm, small ? o_raw + (size_t)span + 16 : 28 * (size_t)n, cudaMemcpyHostToDevice, s));
 		if (both) {
-			CK(cudaMemcpyAsync((int32_t *)B.ql.p + n_in, B.ql.p, 4 * (size_t)n_in, cudaMemcpyDeviceToDevice, s));
-			CK(cudaMemcpyAsync((int32_t *)B.v0.p + n_in, B.v0.p, 4 * (size_t)n_in, cudaMemcpyDeviceToDevice, s));
-			CK(cudaMemsetAsync((char *)B.raw.p + rc_base + span, 0, 16, s));
+			CK(cudaMemsetAsync(B.d_raw + rc_base + span, 0, 16, s));
 			const int ctas = (n_in + kWarpsPerCtaPack - 1) / kWarpsPerCtaPack;
-			k_revcomp_reads<<<ctas, 32 * kWarpsPerCtaPack, 0, s>>>((uint8_t *)B.raw.p, (const int64_t *)B.raw_off.p,
-			                                                      (const int32_t *)B.ql.p, n_in);
+			k_revcomp_reads<<<ctas, 32 * kWarpsPerCtaPack, 0, s>>>(B.d_raw, B.d_raw_off, B.d_ql, n_in);
 			CK(cudaGetLastError());
 		}
-		CK(cudaMemcpyAsync(B.pk_off.p, h_pk_off, 8 * (size_t)n, cudaMemcpyHostToDevice, s));
-		CK(cudaMemcpyAsync(B.order_ql.p, h_order, 4 * (size_t)n, cudaMemcpyHostToDevice, s));
 	}
 	return 0;
 }
@@ -547,11 +582,11 @@ static DevReads reads_view(const Batch &B)
 {
 	DevReads r;
 	r.pk = (const uint64_t *)B.pk.p;
-	r.pk_off = (const int64_t *)B.pk_off.p;
-	r.raw = (const uint8_t *)B.raw.p;
-	r.raw_off = (const int64_t *)B.raw_off.p;
-	r.ql = (const int32_t *)B.ql.p;
-	r.v0 = (const int32_t *)B.v0.p;
+	r.pk_off = B.d_pk_off;
+	r.raw = B.d_raw;
+	r.raw_off = B.d_raw_off;
+	r.ql = B.d_ql;
+	r.v0 = B.d_v0;
 	r.pure = (const uint8_t *)B.pure.p;
 	r.v1 = B.v1;
 	r.n = B.n;
@@ -566,10 +601,10 @@ static KParams base_params(Engine &E, const GraphDev &G, Batch &B, int32_t flags
 	p.r = reads_view(B);
 	p.dens_milli = G.dens_milli;
 	p.flags = flags;
-	p.dist = (int32_t *)B.dist.p;
-	p.status = (int32_t *)B.status.p;
+	p.dist = B.d_dist;
+	p.status = B.d_status;
 	p.retry_list = (int32_t *)E.retry_list.p;
-	p.retry_n = (int32_t *)E.retry_n.p;
+	p.retry_n = B.d_count;
 	p.steps_out = (int32_t *)B.steps.p;
 	p.w_out = nullptr;
 	return p;
@@ -720,8 +755,7 @@ static int enqueue_pack(Engine &E, Batch &B)
 {
 	const int ctas = (B.n + kWarpsPerCta - 1) / kWarpsPerCta;
 	k_pack_reads<<<ctas, 32 * kWarpsPerCta, 0, E.stream>>>(
-	    (const uint8_t *)B.raw.p, (const int64_t *)B.raw_off.p, (const int32_t *)B.ql.p,
-	    (const int64_t *)B.pk_off.p, (uint64_t *)B.pk.p, (uint8_t *)B.pure.p, B.n);
+	    B.d_raw, B.d_raw_off, B.d_ql, B.d_pk_off, (uint64_t *)B.pk.p, (uint8_t *)B.pure.p, B.n);
 	CK(cudaGetLastError());
 	return 0;
 }
@@ -899,18 +933,18 @@ static int launch_level0_graph(Engine &E, Batch &B, KParams &p, int ctas_per_sm,
 		return rc;
 	const uint64_t key[9] = {B.generation, (uint64_t)(uintptr_t)E.ws.p, (uint64_t)pl.slot, (uint64_t)pl.ctas,
 	                         (uint64_t)(uint32_t)p.flags | (uint64_t)(uint32_t)p.max_lag << 32,
-	                         (uint64_t)(uintptr_t)E.retry_n.p,
+	                         (uint64_t)(uintptr_t)B.res.p,
 	                         (uint64_t)(uintptr_t)E.h_small.p, (uint64_t)(uintptr_t)E.retry_list.p,
 	                         blocks ? ~1ULL : classes ? B.cls_key ^ B.cls_gen << 40 : ~0ULL};
 	if (!B.gexec || memcmp(key, B.gkey, sizeof key) != 0) {
 		if (B.gexec) cudaGraphExecDestroy(B.gexec), B.gexec = nullptr;
 		CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
 		int erc = enqueue_pack(E, B);
-		if (!erc && cudaMemsetAsync(E.retry_n.p, 0, 4, E.stream) != cudaSuccess) erc = GWF_E_CUDA;
-		if (!erc) erc = blocks ? enqueue_blocks(E, p, pl, (const int32_t *)B.order_ql.p, B.n)
+		if (!erc && cudaMemsetAsync(B.d_count, 0, 4, E.stream) != cudaSuccess) erc = GWF_E_CUDA;
+		if (!erc) erc = blocks ? enqueue_blocks(E, p, pl, B.d_order, B.n)
 		                : classes ? enqueue_classes(E, p, cl)
-		                        : enqueue_persistent(E, p, pl, (const int32_t *)B.order_ql.p, B.n, B.max_ql, 0);
-		if (!erc && cudaMemcpyAsync(E.h_small.p, E.retry_n.p, 4, cudaMemcpyDeviceToHost, E.stream) != cudaSuccess)
+		                        : enqueue_persistent(E, p, pl, B.d_order, B.n, B.max_ql, 0);
+		if (!erc && cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream) != cudaSuccess)
 			erc = GWF_E_CUDA;
 		cudaGraph_t graph = nullptr;
 		const cudaError_t ce = cudaStreamEndCapture(E.stream, &graph);
@@ -936,16 +970,16 @@ static int launch_level0_graph(Engine &E, Batch &B, KParams &p, int ctas_per_sm,
 
 int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t flags,
                    int ctas_per_sm, float *ms, int *launches_out, int use_graph, int32_t max_lag,
-                   int32_t warps_per_read)
+                   int32_t warps_per_read, bool fetch)
 {
 	int launches = 0, rc;
+	B.fetched = false;
 	if (B.n == 0) {
 		if (ms) *ms = 0;
 		if (launches_out) *launches_out = 0;
 		return 0;
 	}
-	if ((rc = E.retry_list.ensure(4 * (size_t)B.n + 4)) || (rc = E.retry_n.ensure(16)) ||
-	    (rc = E.h_small.ensure(4 * (size_t)B.n + 64)))
+	if ((rc = E.retry_list.ensure(4 * (size_t)B.n + 4)) || (rc = E.h_small.ensure(4 * (size_t)B.n + 64)))
 		return rc;
 	KParams p = base_params(E, G, B, flags);
 	p.max_lag = max_lag > 0 ? max_lag : 0;
@@ -973,7 +1007,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	if (ctas_per_sm <= 0)
 		ctas_per_sm = classes ? E.classes_ctas_per_sm : E.persistent_ctas_per_sm;
 	bool count_copied = false;
-	CK(cudaEventRecord(E.ev0, E.stream));
+	if (ms) CK(cudaEventRecord(E.ev0, E.stream));
 	if (use_graph && mode != GWF_MODE_PLAIN) {
 		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks))) return rc;
 		launches += 2;
@@ -981,30 +1015,37 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	} else {
 		if ((rc = enqueue_pack(E, B))) return rc;
 		++launches;
-		CK(cudaMemsetAsync(E.retry_n.p, 0, 4, E.stream));
+		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		if (mode == GWF_MODE_PLAIN) rc = launch_plain(E, p, B, &launches);
 		else if (blocks) {
 			PersistPlan pl;
 			if (!(rc = plan_blocks(E, &p, B.n, B.max_ql, 0, warps_per_sm, &pl)) &&
-			    !(rc = enqueue_blocks(E, p, pl, (const int32_t *)B.order_ql.p, B.n)))
+			    !(rc = enqueue_blocks(E, p, pl, B.d_order, B.n)))
 				++launches;
 		} else if (classes) {
 			ClassLaunch cl;
 			if (!(rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl)) && !(rc = enqueue_classes(E, p, cl)))
 				++launches;
 		} else
-			rc = launch_persistent(E, p, (const int32_t *)B.order_ql.p, B.n, B.max_ql, 0, ctas_per_sm, &launches);
+			rc = launch_persistent(E, p, B.d_order, B.n, B.max_ql, 0, ctas_per_sm, &launches);
 		if (rc) return rc;
 	}
 	// re-run arena overflows at larger size classes (the block form's first in a larger arena of its
 	// own, then as the sorted form's)
 	for (int level = blocks ? 0 : 1; level <= kMaxLevel; ++level) {
 		int32_t nr = 0;
-		if (!count_copied) CK(cudaMemcpyAsync(E.h_small.p, E.retry_n.p, 4, cudaMemcpyDeviceToHost, E.stream));
+		if (fetch) { // results and the overflow count in one copy, through the pinned input block
+			if ((rc = B.h_meta.ensure(8 * (size_t)B.n + 64))) return rc;
+			CK(cudaMemcpyAsync(B.h_meta.p, B.res.p, 8 * (size_t)B.n + 4, cudaMemcpyDeviceToHost, E.stream));
+		} else if (!count_copied)
+			CK(cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream));
 		count_copied = false;
 		CK(cudaStreamSynchronize(E.stream));
-		nr = *(int32_t *)E.h_small.p;
-		if (nr == 0) break;
+		nr = fetch ? ((const int32_t *)B.h_meta.p)[2 * (size_t)B.n] : *(int32_t *)E.h_small.p;
+		if (nr == 0) {
+			B.fetched = fetch;
+			break;
+		}
 		std::vector<int32_t> ids((size_t)nr);
 		CK(cudaMemcpyAsync(E.h_small.p, E.retry_list.p, 4 * (size_t)nr, cudaMemcpyDeviceToHost, E.stream));
 		CK(cudaStreamSynchronize(E.stream));
@@ -1014,7 +1055,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		std::sort(ids.begin(), ids.end(), [&](int32_t x, int32_t y) { return B.h_ql[(size_t)x] > B.h_ql[(size_t)y]; });
 		if ((rc = E.order.ensure(4 * (size_t)nr))) return rc;
 		CK(cudaMemcpyAsync(E.order.p, ids.data(), 4 * (size_t)nr, cudaMemcpyHostToDevice, E.stream));
-		CK(cudaMemsetAsync(E.retry_n.p, 0, 4, E.stream));
+		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		KParams q = p;
 		if (level == 0) {
 			PersistPlan pl;
@@ -1029,9 +1070,12 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		                            std::min(ctas_per_sm, E.persistent_ctas_per_sm), &launches)))
 			return rc;
 	}
-	CK(cudaEventRecord(E.ev1, E.stream));
-	CK(cudaEventSynchronize(E.ev1));
-	if (ms) CK(cudaEventElapsedTime(ms, E.ev0, E.ev1));
+	if (ms) {
+		CK(cudaEventRecord(E.ev1, E.stream));
+		CK(cudaEventSynchronize(E.ev1));
+		CK(cudaEventElapsedTime(ms, E.ev0, E.ev1));
+	} else if (!B.fetched)
+		CK(cudaStreamSynchronize(E.stream));
 	if (launches_out) *launches_out = launches;
 	return 0;
 }
@@ -1043,9 +1087,10 @@ int gwf_batch_fetch(Engine &E, Batch &B, int32_t *dist, int32_t *status, int32_t
 	int rc;
 	if ((rc = B.h_meta.ensure(8 * (size_t)B.n + 64))) return rc;
 	int32_t *hd = (int32_t *)B.h_meta.p, *hs = hd + B.n;
-	if (dist || B.both) CK(cudaMemcpyAsync(hd, B.dist.p, 4 * (size_t)B.n, cudaMemcpyDeviceToHost, E.stream));
-	if (status || B.both) CK(cudaMemcpyAsync(hs, B.status.p, 4 * (size_t)B.n, cudaMemcpyDeviceToHost, E.stream));
-	CK(cudaStreamSynchronize(E.stream));
+	if (!B.fetched) {
+		CK(cudaMemcpyAsync(hd, B.res.p, 8 * (size_t)B.n, cudaMemcpyDeviceToHost, E.stream));
+		CK(cudaStreamSynchronize(E.stream));
+	}
 	if (B.both) {
 		combine_strands(B.n_in, hd, hs, dist, status, strand);
 		return 0;
@@ -1151,7 +1196,7 @@ extern "C" int gwf_ed_batch_concat(const gwf_graph_t *g, int32_t n, const char *
 	const int32_t cps = opt ? opt->ctas_per_sm : 0;
 	const int32_t lag = (flags & GWF_F_MAX_LAG) ? (int32_t)std::min<uint32_t>(max_lag, INT32_MAX) : 0;
 	if ((rc = gwf_batch_exec(*E, *G, *B, mode, flags, cps, nullptr, nullptr, opt ? opt->use_graph : 0, lag,
-	                         opt ? opt->warps_per_read : 0)))
+	                         opt ? opt->warps_per_read : 0, true)))
 		return rc;
 	std::vector<int32_t> st;
 	if (!status) st.resize((size_t)n), status = st.data();
@@ -1294,8 +1339,8 @@ static int launch_cigar(Engine &E, const GraphDev &G, Batch &B, TraceBufs &T, co
 	p.g = G.view();
 	p.r = reads_view(B);
 	p.max_nv = max_nv, p.max_ops = max_ops;
-	p.dist = (const int32_t *)B.dist.p;
-	p.status = (const int32_t *)B.status.p;
+	p.dist = B.d_dist;
+	p.status = B.d_status;
 	p.end_off = (const int32_t *)T.end_off.p;
 	p.path_n = (const int32_t *)T.path_n.p;
 	p.path_v = (const int32_t *)T.path_v.p;
@@ -1374,8 +1419,7 @@ extern "C" int gwf_ed_batch_align(const gwf_graph_t *g, int32_t n, const char *s
 	if ((rc = T->end_off.ensure(4 * (size_t)n)) || (rc = T->path_n.ensure(4 * (size_t)n)) ||
 	    (rc = T->path_v.ensure(4 * cells)) || (rc = T->path_arc.ensure(4 * cells)) ||
 	    (max_ops > 0 && ((rc = T->cigar_n.ensure(4 * (size_t)n)) || (rc = T->cigar.ensure(4 * ops)))) ||
-	    (rc = E->retry_list.ensure(4 * (size_t)n + 4)) || (rc = E->retry_n.ensure(16)) ||
-	    (rc = E->h_small.ensure(4 * (size_t)n + 64)))
+	    (rc = E->retry_list.ensure(4 * (size_t)n + 4)) || (rc = E->h_small.ensure(4 * (size_t)n + 64)))
 		return rc;
 	KParams p = base_params(*E, *G, *B, flags);
 	p.end_off = (int32_t *)T->end_off.p;
@@ -1388,11 +1432,11 @@ extern "C" int gwf_ed_batch_align(const gwf_graph_t *g, int32_t n, const char *s
 	std::vector<int32_t> ids((size_t)n);
 	std::iota(ids.begin(), ids.end(), 0);
 	for (int level = 0; level <= kMaxLevel && !ids.empty(); ++level) {
-		CK(cudaMemsetAsync(E->retry_n.p, 0, 4, E->stream));
+		CK(cudaMemsetAsync(B->d_count, 0, 4, E->stream));
 		KParams q = p;
 		if (level == kMaxLevel) q.retry_list = nullptr; // last class: keep GWF_E_CAPACITY
 		if ((rc = launch_trace(*E, q, *B, ids, level, &launches))) return rc;
-		CK(cudaMemcpyAsync(E->h_small.p, E->retry_n.p, 4, cudaMemcpyDeviceToHost, E->stream));
+		CK(cudaMemcpyAsync(E->h_small.p, B->d_count, 4, cudaMemcpyDeviceToHost, E->stream));
 		CK(cudaStreamSynchronize(E->stream));
 		const int32_t nr = level == kMaxLevel ? 0 : *(int32_t *)E->h_small.p;
 		ids.resize((size_t)nr);

@@ -37,6 +37,8 @@ struct GraphDev { // device-resident copy of one gwf_graph_t
 	~GraphDev();
 };
 
+constexpr int kStageThreads = 4; // threads that fill the chunks of a large pageable upload
+
 struct Engine { // per-device launch state: stream, events, warp arenas
 	int device = 0;
 	int sm_count = 0;
@@ -46,10 +48,10 @@ struct Engine { // per-device launch state: stream, events, warp arenas
 	int64_t mem_budget = 0; // device bytes the arenas may take
 	cudaStream_t stream = nullptr;
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-	DBuf pk_off, order, head, retry_list, retry_n, ws, slot_off, w_out;
+	DBuf order, head, retry_list, ws, slot_off;
 	HBuf h_small;
-	HBuf h_stage;                              // two pinned chunks for pageable uploads
-	cudaEvent_t stage_ev[2] = {nullptr, nullptr};
+	HBuf h_stage;                              // pinned chunks for pageable uploads, two per thread
+	cudaEvent_t stage_ev[2 * kStageThreads] = {};
 	~Engine();
 };
 
@@ -63,8 +65,16 @@ struct Batch { // reads resident on the device
 	cudaGraphExec_t gexec = nullptr;  // captured level-0 sequence of the persistent form
 	uint64_t gkey[9] = {};
 	std::vector<int32_t> h_ql;
-	HBuf h_meta; // pinned: raw offsets, packed offsets, queue order; results on the way back
-	DBuf raw, raw_off, ql, v0, pk, pk_off, pure, dist, status, steps, order_ql;
+	HBuf h_meta; // pinned input block; results on the way back
+	DBuf in;     // raw offsets, packed offsets, lengths, start vertices, queue order, bases of a small batch
+	DBuf raw;    // bases of a large batch
+	DBuf res;    // distances, statuses, overflow count
+	DBuf pk, pure, steps;
+	int64_t *d_raw_off = nullptr, *d_pk_off = nullptr;
+	int32_t *d_ql = nullptr, *d_v0 = nullptr, *d_order = nullptr;
+	uint8_t *d_raw = nullptr;
+	int32_t *d_dist = nullptr, *d_status = nullptr, *d_count = nullptr;
+	bool fetched = false; // h_meta holds the last run's results
 	// read classes of the persistent form (reads aligned by groups of warps), cached per layout
 	DBuf order_cls;
 	uint64_t cls_key = ~0ULL, cls_gen = ~0ULL; // layout key and the batch generation it was made for
@@ -79,7 +89,7 @@ int gwf_batch_load(Engine &E, Batch &B, int32_t n, const char *seqs, const int64
                    const int32_t *ql, const int32_t *v0, int32_t v1, bool both = false);
 int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t flags,
                    int ctas_per_sm, float *ms, int *launches_out, int use_graph = 0, int32_t max_lag = 0,
-                   int32_t warps_per_read = 0);
+                   int32_t warps_per_read = 0, bool fetch = false);
 int gwf_batch_fetch(Engine &E, Batch &B, int32_t *dist, int32_t *status, int32_t *strand = nullptr);
 namespace gwfb {
 struct KParams;
