@@ -121,15 +121,14 @@ __global__ void __launch_bounds__(256) k_bloom(const __grid_constant__ DevGraph 
 	}
 }
 
-// State of a warp's run, in the CTA's shared memory (one warp per CTA). The parts of the kernel
-// that are not run at every step are functions of their own that work on it: with everything
-// inlined the kernel had 87 KB of code, its 32 warps per SM stood in different parts of it, and
-// the instruction cache held half of their cycles.
+// State of a read's run, in the CTA's shared memory (a CTA aligns one read at a time, with one warp
+// or, MW, with several). The parts of the kernel that are not run at every step are functions of
+// their own that work on it: with everything inlined the kernel had 87 KB of code, its 32 warps per
+// SM stood in different parts of it, and the instruction cache held half of their cycles.
 constexpr int kBwQueue = 31 + 16 * 8;
 struct BwShm {
-	uint2 queue[kBwQueue + 1]; // diagonals on their way to the extension: id << 4 | side << 3 | cell, k
 	BwBlock *blk;
-	uint2 *hash;               // (tag, id) per slot, id -1 = empty
+	uint2 *hash;               // (tag, id) per slot, all ones = empty
 	uint32_t *slot;            // slot of each block
 	int32_t *nxt;              // live list of the next step
 	uint32_t *e, *f, *n;       // vertex-end states of a wave and of the next, entered states: id << 3 | cell
@@ -147,13 +146,52 @@ struct BwShm {
 	uint32_t hmask;
 	int32_t nb;                // blocks in the pool
 	int32_t ql, packed, quirk;
-	int32_t n_blk, n_nxt;      // blocks in use, length of nxt
+	int32_t n_blk;             // blocks in use
 	int32_t ovf;               // a buffer is full
+	// of a step (bw_step_begin)
+	int32_t s, imin;           // score; query position behind which the lag run drops states
+	int32_t n_nxt, n_e;        // lengths of nxt and e
+	int32_t next;              // next entry of the live list to be taken
+	int32_t any, found, far;   // a state lives, one reached the query's end, furthest query position
+	int32_t n_n[2], n_f[2];    // of a wave, by its parity
+	int32_t claim;             // MW: queue position of the group's read
 };
 __device__ __forceinline__ BwShm &bw_sh()
 {
 	extern __shared__ __align__(16) unsigned char bw_smem[];
 	return *(BwShm *)bw_smem;
+}
+// Diagonals on their way to the extension: id << 4 | side << 3 | cell, k; one queue per warp
+__device__ __forceinline__ uint2 *bw_queue()
+{
+	return (uint2 *)(&bw_sh() + 1) + (threadIdx.x >> 5) * (kBwQueue + 1);
+}
+constexpr size_t bw_shm_bytes(int warps) { return sizeof(BwShm) + (size_t)warps * (kBwQueue + 1) * sizeof(uint2); }
+static_assert(sizeof(BwShm) % 16 == 0, "the queues follow");
+
+template <bool MW>
+__device__ __forceinline__ void bw_bar()
+{
+	if constexpr (MW) __syncthreads();
+	else __syncwarp();
+}
+// n entries appended behind the counter c (a warp's; the lanes of mask m, in lane order): this
+// lane's place
+template <bool MW>
+__device__ __forceinline__ int32_t bw_append(int32_t *c, uint32_t m)
+{
+	int32_t at;
+	if constexpr (MW) {
+		at = 0;
+		if ((threadIdx.x & 31) == 0 && m) at = atomicAdd(c, __popc(m));
+		at = __shfl_sync(FULL, at, 0);
+	} else {
+		at = *c;
+		__syncwarp();
+		*c = at + __popc(m);
+		__syncwarp();
+	}
+	return at + __popc(m & lanemask_lt());
 }
 
 __device__ __forceinline__ bool bloom_has(const BwShm &sh, uint32_t x)
@@ -187,17 +225,19 @@ static __device__ __noinline__ bool bw_edit(uint32_t y, int code)
 // that is found is then tried on the other absent windows of the 32 that hold its position. A
 // window with a byte other than A/C/G/T costs 1 (the graph has none). With stride 1 every other
 // absent window counts 1 without the one-edit lookups: half of them, for a bound 0.5% lower.
+template <bool MW>
 static __device__ __noinline__ int32_t bw_seeds(int32_t stride)
 {
 	const BwShm &sh = bw_sh();
 	const int lane = threadIdx.x & 31;
 	const int32_t K = sh.K, ql = sh.ql, n_edit = 11 * K - 4;
 	uint16_t *const h = sh.h;
+	const int32_t wid = MW ? threadIdx.x >> 5 : 0, nw = MW ? blockDim.x >> 5 : 1;
 #pragma unroll 1
-	for (int32_t j = lane; j <= ql; j += 32) h[j] = 0;
-	__syncwarp();
+	for (int32_t j = 32 * wid + lane; j <= ql; j += 32 * nw) h[j] = 0;
+	bw_bar<MW>();
 #pragma unroll 1
-	for (int32_t base = K; base <= ql; base += 32 * stride) {
+	for (int32_t base = K + 32 * stride * wid; base <= ql; base += 32 * stride * nw) {
 		const int32_t rem = base + lane * stride, p = ql - rem;
 		uint32_t x = 0, nb = 0; // the window and the base after it
 		int32_t cost = 0;
@@ -239,13 +279,13 @@ static __device__ __noinline__ int32_t bw_seeds(int32_t stride)
 		}
 		if (rem <= ql) h[rem] = (uint16_t)cost;
 	}
-	__syncwarp();
+	bw_bar<MW>();
 	// the maximum over disjoint windows, K entries at a time: lane l's entry takes its window after
 	// h[rem - K] of the pass before
 	int32_t prev = 0; // lane l < K: h[b - K + l]
 	int32_t last = 0; // h[b - 1]
 #pragma unroll 1
-	for (int32_t b = K; b <= ql; b += K) {
+	for (int32_t b = K; b <= ql && wid == 0; b += K) {
 		const int32_t rem = b + lane;
 		const bool on = lane < K && rem <= ql;
 		int32_t v = on ? prev + (int32_t)h[rem] : 0;
@@ -259,7 +299,7 @@ static __device__ __noinline__ int32_t bw_seeds(int32_t stride)
 		prev = v;
 		last = __shfl_sync(FULL, v, K - 1);
 	}
-	__syncwarp();
+	bw_bar<MW>();
 	return (int32_t)h[ql];
 }
 
@@ -314,9 +354,20 @@ __device__ __forceinline__ uint32_t bw_tag(uint32_t v, int32_t bi)
 	return x * 0x2C1B3C6Du;
 }
 
+__device__ __forceinline__ uint2 bw_slot_load(const uint2 *p)
+{
+	unsigned long long v;
+	asm volatile("ld.relaxed.cta.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+	return make_uint2((uint32_t)v, (uint32_t)(v >> 32));
+}
+constexpr uint32_t BW_BUSY = 0xfffffffeu; // MW: a slot whose block is being made
+
 // Block bi (diagonals 8 bi .. 8 bi + 7) of vertex v, made where it is missing (the whole warp calls
-// it; on: this lane asks). Of the lanes that want one empty slot the first makes its block. Sets
-// ovf when the pool is full. gb, vl: the vertex's first base and length.
+// it; on: this lane asks). Of a warp's lanes that want one empty slot the first makes its block; MW:
+// it claims the slot by compare-and-swap, and lanes of other warps that want the same tag look again
+// until it is published (the maker never waits in between; the tries are bounded). Sets ovf when the
+// pool is full. gb, vl: the vertex's first base and length.
+template <bool MW>
 static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, uint32_t gb, int32_t vl)
 {
 	BwShm &sh = bw_sh();
@@ -327,29 +378,49 @@ static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, u
 	int32_t id = on ? -1 : 0;
 	bool made = false;
 	uint32_t tag = bw_tag(v, bi), sl = (tag ^ tag >> 16) & hmask;
-	int32_t n_blk = sh.n_blk;
+	int32_t n_blk = MW ? 0 : sh.n_blk;
 #pragma unroll 1
-	for (uint32_t guard = 0; guard <= hmask + 64; ++guard) {
+	for (uint32_t guard = 0; guard <= hmask + (1u << 16); ++guard) {
 		bool want = false;
 		if (id < 0) {
-			const uint2 e = hash[sl];
-			want = (int32_t)e.y < 0;
+			const uint2 e = MW ? bw_slot_load(hash + sl) : hash[sl];
+			want = e.y == 0xffffffffu;
 			if (!want) {
-				if (e.x == tag && blk[e.y].v == v && blk[e.y].db == 8 * bi) id = (int32_t)e.y;
-				else sl = sl + 1 & hmask;
+				const bool busy = MW && e.y == BW_BUSY;
+				if (!busy && e.x == tag && blk[e.y].v == v && blk[e.y].db == 8 * bi) id = (int32_t)e.y;
+				else if (!busy || e.x != tag) sl = sl + 1 & hmask;
 			}
 		}
 		if (__any_sync(FULL, want)) {
 			const uint32_t same = __match_any_sync(FULL, want ? (int32_t)sl : -1 - lane);
-			const bool won = want && (same & lanemask_lt()) == 0;
-			const uint32_t m = __ballot_sync(FULL, won);
-			if (n_blk + __popc(m) > sh.nb) {
-				sh.ovf = 1;
-				break;
+			bool won = want && (same & lanemask_lt()) == 0;
+			int32_t at = 0;
+			if constexpr (MW) {
+				if (won)
+					won = atomicCAS((unsigned long long *)(hash + sl), ~0ULL,
+					                (unsigned long long)BW_BUSY << 32 | tag) == ~0ULL;
+				if (won) at = atomicAdd(&sh.n_blk, 1);
+				if (won && at >= sh.nb) { // full: the claimed slot goes back
+					atomicExch((unsigned long long *)(hash + sl), ~0ULL);
+					won = false;
+					sh.ovf = 1;
+				}
+				if (__any_sync(FULL, sh.ovf != 0)) {
+					if (won) sh.slot[at] = sl, atomicExch((unsigned long long *)(hash + sl), (unsigned long long)at << 32 | tag);
+					sh.ovf = 1;
+					break;
+				}
+			} else {
+				const uint32_t m = __ballot_sync(FULL, won);
+				if (n_blk + __popc(m) > sh.nb) {
+					sh.ovf = 1;
+					break;
+				}
+				at = n_blk + __popc(m & lanemask_lt());
+				n_blk += __popc(m);
 			}
 			if (won) {
-				id = n_blk + __popc(m & lanemask_lt());
-				hash[sl] = make_uint2(tag, (uint32_t)id);
+				id = at;
 				int4 *q = (int4 *)(blk + id);
 				q[1] = make_int4(vl, -1, -1, 0);
 				const int4 none = make_int4(BW_NONE, BW_NONE, BW_NONE, BW_NONE);
@@ -358,27 +429,36 @@ static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, u
 				q[0] = make_int4((int)gb, (int)__ldg(sh.varcs + v), (int)v, 8 * bi);
 				sh.slot[id] = sl;
 				made = true;
+				if constexpr (MW) {
+					__threadfence_block(); // the block before its id
+					atomicExch((unsigned long long *)(hash + sl), (unsigned long long)(uint32_t)id << 32 | tag);
+				} else
+					hash[sl] = make_uint2(tag, (uint32_t)id);
 			}
-			n_blk += __popc(m);
 			__syncwarp();
 		}
 		if (!__any_sync(FULL, id < 0)) break;
+		if (MW && guard == hmask + (1u << 16)) sh.ovf = 1; // not reached: a maker publishes at once
 	}
-	sh.n_blk = n_blk;
+	if constexpr (!MW) sh.n_blk = n_blk;
 	if (__any_sync(FULL, made)) {
-		// links to the neighbours that exist
+		// links to the neighbours that exist (MW: of two neighbours made at once, the one that is
+		// published last finds the other)
+		if constexpr (MW) __threadfence_block();
 #pragma unroll 1
 		for (int side = -1; made && side <= 1; side += 2) {
 			tag = bw_tag(v, bi + side), sl = (tag ^ tag >> 16) & hmask;
 #pragma unroll 1
 			for (uint32_t guard = 0; guard <= hmask; ++guard) {
-				const uint2 e = hash[sl];
-				if ((int32_t)e.y < 0) break;
-				BwBlock *const B = blk + e.y;
-				if (e.x == tag && B->v == v && B->db == 8 * (bi + side)) {
-					*(side < 0 ? &blk[id].left : &blk[id].right) = (int32_t)e.y;
-					*(side < 0 ? &B->right : &B->left) = id;
-					break;
+				const uint2 e = MW ? bw_slot_load(hash + sl) : hash[sl];
+				if (e.y == 0xffffffffu) break;
+				if (!(MW && e.y == BW_BUSY)) {
+					BwBlock *const B = blk + e.y;
+					if (e.x == tag && B->v == v && B->db == 8 * (bi + side)) {
+						*(side < 0 ? &blk[id].left : &blk[id].right) = (int32_t)e.y;
+						*(side < 0 ? &B->right : &B->left) = id;
+						break;
+					}
 				}
 				sl = sl + 1 & hmask;
 			}
@@ -390,39 +470,61 @@ static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, u
 
 // Puts block id into the next live list, once (several lanes may name one block). np: the parity of
 // the next step.
+template <bool MW>
 static __device__ __noinline__ void bw_push(bool on, int32_t id, int np)
 {
 	BwShm &sh = bw_sh();
 	const uint32_t same = __match_any_sync(FULL, on ? id : -1 - (int)(threadIdx.x & 31));
+	bool app = on && (same & lanemask_lt()) == 0;
 	uint8_t *const f = &sh.blk[id].inl[np];
-	const bool app = on && (same & lanemask_lt()) == 0 && !*f;
-	if (app) *f = 1;
+	app = app && !*f;
+	if constexpr (MW) {
+		const uint32_t bit = 0x10000u << (8 * np);
+		if (app) app = !(atomicOr((uint32_t *)(sh.blk + id) + 7, bit) & bit);
+	} else if (app)
+		*f = 1;
 	const uint32_t m = __ballot_sync(FULL, app);
-	const int32_t n = sh.n_nxt;
-	if (app) sh.nxt[n + __popc(m & lanemask_lt())] = id;
-	__syncwarp();
-	sh.n_nxt = n + __popc(m);
+	if (m) {
+		const int32_t at = bw_append<MW>(&sh.n_nxt, m);
+		if (app) sh.nxt[at] = id;
+	}
 	__syncwarp();
 }
 
-// Arc-side candidate k for diagonal d of vertex v at the next step (lanes that meet on one diagonal
-// bring the same k).
+// Arc-side candidate k for cell c (k << 1 | arrived); MW: other warps may change it
+template <bool MW>
+__device__ __forceinline__ void bw_raise(int32_t *c, int32_t k)
+{
+	int32_t c0 = MW ? *(volatile int32_t *)c : *c;
+	if constexpr (MW) {
+#pragma unroll 1
+		while (c0 >> 1 < k) { // each retry means that another lane raised it
+			const int32_t was = atomicCAS(c, c0, k << 1 | (c0 & 1));
+			if (was == c0) break;
+			c0 = was;
+		}
+	} else if (c0 >> 1 < k)
+		*c = k << 1 | (c0 & 1);
+}
+
+// Arc-side candidate k for diagonal d of vertex v at the next step (lanes of a warp that meet on one
+// diagonal bring the same k).
+template <bool MW>
 static __device__ __noinline__ void bw_cand(bool on, uint32_t v, int32_t d, uint32_t gb, int32_t vl, int32_t k, int np)
 {
 	BwShm &sh = bw_sh();
-	const int32_t id = bw_get(on, v, d >> 3, gb, vl);
+	const int32_t id = bw_get<MW>(on, v, d >> 3, gb, vl);
 	if (sh.ovf) return;
 	if (on) {
-		int32_t *const c = sh.blk[id].c + (d & 7);
-		const int32_t c0 = *c;
-		if (c0 >> 1 < k) *c = k << 1 | (c0 & 1);
+		bw_raise<MW>(sh.blk[id].c + (d & 7), k);
 		sh.blk[id].has_c = 1;
 	}
-	bw_push(on, id, np);
+	bw_push<MW>(on, id, np);
 }
 
 // A live edge diagonal (act: block id, cell l) gives the neighbouring block a candidate at the next
 // step: lists the neighbour, made where it is missing.
+template <bool MW>
 static __device__ __noinline__ void bw_side(bool act, int32_t id, int32_t l, int np)
 {
 	BwShm &sh = bw_sh();
@@ -432,25 +534,36 @@ static __device__ __noinline__ void bw_side(bool act, int32_t id, int32_t l, int
 	const bool miss = act && t < 0;
 	int32_t u = t;
 	if (__any_sync(FULL, miss)) {
-		const int32_t w = bw_get(miss, B->v, (B->db >> 3) + (l == 0 ? -1 : 1), B->gb, B->vl);
-		if (sh.ovf) return;
+		const int32_t w = bw_get<MW>(miss, B->v, (B->db >> 3) + (l == 0 ? -1 : 1), B->gb, B->vl);
+		if (__any_sync(FULL, sh.ovf != 0)) return;
 		if (miss) u = w;
 	}
-	bw_push(act, act ? u : 0, np);
+	bw_push<MW>(act, act ? u : 0, np);
 }
 
-// Successors of the live blocks base .. of the list cur (n_cur entries), two lanes per block and
-// four diagonals per lane, until the queue (n_q entries) holds 32 diagonals that may live or the
-// list ends. Blocks that stay go to the next list. kmin: the least offset of a candidate. Returns
-// (base, n_q).
-static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t base, int32_t n_cur, int32_t n_q, int par,
-                                            int32_t kmin)
+// Successors of the live blocks of the list cur (n_cur entries), two lanes per block and four
+// diagonals per lane, until the warp's queue (n_q entries) holds 32 diagonals that may live or the
+// list is empty. Blocks that stay go to the next list. kmin: the least offset of a candidate.
+// Returns (1 = the list may hold more, n_q).
+template <bool MW>
+static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t n_cur, int32_t n_q, int par, int32_t kmin)
 {
 	BwShm &sh = bw_sh();
+	uint2 *const queue = bw_queue();
 	const int lane = threadIdx.x & 31, np = par ^ 1, hf = lane & 1;
-	int32_t n_nxt = sh.n_nxt;
 #pragma unroll 1
-	while (n_q < 32 && base < n_cur) {
+	while (n_q < 32) {
+		int32_t base;
+		if constexpr (MW) {
+			base = 0;
+			if (lane == 0) base = atomicAdd(&sh.next, 16);
+			base = __shfl_sync(FULL, base, 0);
+		} else {
+			base = sh.next;
+			__syncwarp();
+			sh.next = base + 16;
+		}
+		if (base >= n_cur) return make_int2(0, n_q);
 		const bool in = base + (lane >> 1) < n_cur;
 		const int32_t bid = cur[in ? base + (lane >> 1) : base];
 		BwBlock *const B = sh.blk + bid;
@@ -467,6 +580,7 @@ static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t base, in
 		if (__any_sync(FULL, (fl & 0xff00) != 0)) {
 			int4 *const cp = (int4 *)B->c + hf;
 			const int4 c = *cp;
+			__syncwarp();
 			kq[0] = max(kq[0], c.x >> 1), kq[1] = max(kq[1], c.y >> 1);
 			kq[2] = max(kq[2], c.z >> 1), kq[3] = max(kq[3], c.w >> 1);
 			if (in)
@@ -486,48 +600,196 @@ static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t base, in
 		const uint32_t w = en << (4 * hf) | (stays ? 0x100u : 0u);
 		const uint32_t w2 = w | __shfl_xor_sync(FULL, w, 1);
 		const uint32_t inb = 0x10000u << (8 * np);
-		const bool first = hf == 0 && in, app = first && (w2 & 0x100) && !(fl & inb);
+		const bool first = hf == 0 && in;
+		bool app = first && (w2 & 0x100) && !(fl & inb);
 		if (in) *((int4 *)B->row[par] + hf) = make_int4(BW_NONE, BW_NONE, BW_NONE, BW_NONE);
-		if (first) *((uint32_t *)B + 7) = (fl & ~(0xff00u | 0xff0000u << (8 * par))) | (w2 & 0xff) | (app ? inb : 0);
+		if constexpr (MW) { // other warps may list the block meanwhile: bytes, and a bit by atomicOr
+			if (first) B->ended = (uint8_t)(fl | w2), B->has_c = 0, B->inl[par] = 0;
+			if (app) app = !(atomicOr((uint32_t *)B + 7, inb) & inb);
+		} else if (first)
+			*((uint32_t *)B + 7) = (fl & ~(0xff00u | 0xff0000u << (8 * par))) | (w2 & 0xff) | (app ? inb : 0);
 		const uint32_t mp = __ballot_sync(FULL, app);
-		if (app) sh.nxt[n_nxt + __popc(mp & lanemask_lt())] = bid;
-		n_nxt += __popc(mp);
+		const int32_t at = bw_append<MW>(&sh.n_nxt, mp);
+		if (app) sh.nxt[at] = bid;
 		// side: an edge diagonal whose neighbour has no live diagonal beside it
 		const uint32_t tag = (uint32_t)bid << 4 | (uint32_t)hf << 2, sq = ek > BW_NONE ? 0u : hf ? 8u : 1u;
 #pragma unroll
 		for (int q = 0; q < 4; ++q) {
 			const bool on = up >> q & 1;
 			const uint32_t m = __ballot_sync(FULL, on);
-			if (on)
-				sh.queue[n_q + __popc(m & lanemask_lt())] = make_uint2(tag | q | ((sq >> q & 1) << 3), (uint32_t)kq[q]);
+			if (on) queue[n_q + __popc(m & lanemask_lt())] = make_uint2(tag | q | ((sq >> q & 1) << 3), (uint32_t)kq[q]);
 			n_q += __popc(m);
 		}
-		base += 16;
 		__syncwarp();
 	}
-	sh.n_nxt = n_nxt;
-	__syncwarp();
-	return make_int2(base, n_q);
+	return make_int2(1, n_q);
 }
 
-// Vertex-end states of step s (n_e entries of e) over their arcs, in waves, until no state is
-// entered with a free match (gwf-ed.cu:1106-1255). Four lanes per state, one arc each. Returns
-// this lane's furthest query position, INT32_MAX in every lane when the query's end was reached.
-static __device__ __noinline__ int32_t bw_waves(int32_t s, int32_t T, int32_t n_e)
+// Step 1 for up to four blocks, by one warp: one lane per diagonal, and step after step in registers
+// until one reaches its vertex's end or the query's, none lives, or a live edge diagonal has its
+// neighbour outside the four blocks (unlisted blocks have no live diagonals).
+template <bool MW>
+__device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int32_t *list0, int32_t *list1, int32_t T,
+                                              bool lag, int32_t max_steps)
 {
 	BwShm &sh = bw_sh();
-	const int lane = threadIdx.x & 31, np = ~s & 1;
-	BwBlock *const blk = sh.blk;
-	const int32_t ql = sh.ql, ne = sh.nb;
+	const int lane = threadIdx.x & 31, gr = lane >> 3, l = lane & 7;
+	const int32_t ql = sh.ql, kmin1 = sh.quirk ? 0 : -1;
+	int32_t s = sh.s, imin = sh.imin;
+	const bool has = gr < n_cur;
+	const int32_t id = cur[has ? gr : 0];
+	BwBlock *const B = sh.blk + id;
+	const int4 b0 = *(const int4 *)B, h1 = *((const int4 *)B + 1); // gb, arcs, v, db; vl, left, right, flags
+	int32_t k = has ? B->row[~s & 1][l] : BW_NONE;
+	const uint32_t fl = (uint32_t)h1.w; // ended, has_c, inl[0], inl[1]
+	const bool edge = (0x81 >> l & 1) != 0;
+	const int32_t nid = l == 0 ? h1.y : h1.z, vl = h1.x, d = b0.w + l;
+	int src = -1; // edge lanes: the lane of the diagonal across
+#pragma unroll
+	for (int j = 0; j < 4; ++j)
+		if (__shfl_sync(FULL, id, 8 * j) == nid && j < n_cur && edge) src = 8 * j + 7 - l;
+	const bool out = edge && src < 0, nu = l == 0 && out, nd = l == 7 && out;
+	const int su = l == 0 ? max(src, 0) : lane - 1, sd = l == 7 ? max(src, 0) : lane + 1;
+	bool dead = !has || (fl >> l & 1); // absent, or past the vertex end
+	int32_t c = BW_NONE;               // the first step's arc-side candidates
+	if (__any_sync(FULL, has && (fl & 0xff00))) {
+		const int32_t cw = B->c[l];
+		__syncwarp();
+		if (has) c = cw >> 1, B->c[l] = 2 * BW_NONE | (cw & 1);
+	}
+	int32_t lo = s == 0 ? -1 : kmin1, i;
+	bool live, qend, vend;
+#pragma unroll 1
+	for (;;) {
+		const int32_t up = __shfl_sync(FULL, k, su), dn = __shfl_sync(FULL, k, sd);
+		k = max(max(nu ? BW_NONE : up, max(k, nd ? BW_NONE : dn) + 1), c);
+		dead |= k >= vl; // at the first step only: later ones follow no vertex end
+		live = !dead && k >= lo;
+		const int32_t hv = sh.h[live ? ql - 1 - d - k : 0]; // any value below BW_INF while T is BW_INF
+		live = live && s + hv < T && d + k >= imin;
+		k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
+		if (!live) k = BW_NONE;
+		i = live ? d + k : INT32_MIN;
+		qend = i == ql - 1, vend = live && k == vl - 1 && !qend;
+		const bool stop = qend || vend || (live && out) || s + 1 >= max_steps;
+		if (__any_sync(FULL, stop) || !__any_sync(FULL, live)) break;
+		if (lag) imin = __reduce_max_sync(FULL, i) - kPruneLag;
+		++s, lo = kmin1, c = BW_NONE;
+	}
+	const int par = s & 1, np = par ^ 1;
+	// back to the blocks: both rows, the ended diagonals, the next list
+	const uint32_t em = (__ballot_sync(FULL, has && dead) >> (8 * gr)) & 0xff;
+	const uint32_t ml = __ballot_sync(FULL, live);
+	if (has) B->row[par][l] = k, B->row[np][l] = BW_NONE;
+	const bool first = l == 0 && has, app = first && (ml >> (8 * gr) & 0xff) != 0;
+	if (first) *((uint32_t *)B + 7) = em | (app ? 0x10000u << (8 * np) : 0);
+	const uint32_t mp = __ballot_sync(FULL, app);
+	int32_t *const nxt = par ? list0 : list1; // the list at hand is in registers
+	if (app) nxt[__popc(mp & lanemask_lt())] = id;
+	const uint32_t me = __ballot_sync(FULL, vend);
+	if (vend) sh.e[__popc(me & lanemask_lt())] = (uint32_t)id << 3 | l;
+	const int32_t far = __reduce_max_sync(FULL, i);
+	const bool any_q = __any_sync(FULL, qend);
+	__syncwarp();
+	sh.s = s, sh.imin = imin, sh.nxt = nxt, sh.n_nxt = __popc(mp), sh.n_e = __popc(me), sh.far = far;
+	sh.found = any_q, sh.any = ml != 0;
+	__syncwarp();
+	// a live edge diagonal gives the neighbouring block a candidate at the next step
+	const bool act = live && edge && (src < 0 || (ml >> (src & 24) & 0xff) == 0);
+	if (__any_sync(FULL, act)) bw_side<MW>(act, id, l, np);
+}
+
+// Step 1 for more blocks: bw_fill's diagonals through the warp's queue, so that the extension runs on
+// full warps (of a dense graph's diagonals in live blocks one in four lives).
+template <bool MW>
+__device__ __forceinline__ void bw_wide(const int32_t *cur, int32_t n_cur, int32_t T)
+{
+	BwShm &sh = bw_sh();
+	const uint2 *const queue = bw_queue();
+	const int lane = threadIdx.x & 31;
+	const int32_t ql = sh.ql, s = sh.s, imin = sh.imin, ne = sh.nb;
+	const int par = s & 1;
+	bool found = false, any = false;
 	int32_t far = INT32_MIN;
-	bool found = false;
+	int2 at = make_int2(1, 0); // more blocks, queued diagonals
 #pragma unroll 1
-	for (int32_t wave = 0; n_e > 0 && !sh.ovf; ++wave) {
-		int32_t n_n = 0;
+	do {
+		if (at.x && at.y < 32) at = bw_fill<MW>(cur, n_cur, at.y, par, s == 0 || !sh.quirk ? -1 : 0);
+		const int32_t take = min(at.y, 32); // from the queue's end
+		at.y -= take;
+		const bool alive = lane < take;
+		const uint2 e = queue[at.y + (alive ? lane : 0)];
+		const int32_t id = alive ? (int32_t)(e.x >> 4) : 0, l = (int32_t)(e.x & 7);
+		int32_t k = (int32_t)e.y;
+		BwBlock *const B = sh.blk + id;
+		const int4 b0 = *(const int4 *)B;
+		const int32_t vl = B->vl, d = b0.w + l;
+		const int32_t hv = sh.h[alive ? ql - 1 - d - k : 0];
+		const bool live = alive && s + hv < T && d + k >= imin;
+		k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
+		if (live) B->row[par][l] = k;
+		const int32_t i = live ? d + k : INT32_MIN;
+		far = max(far, i);
+		const bool qend = i == ql - 1, vend = live && k == vl - 1 && !qend;
+		found |= qend;
+		any |= live;
+		const uint32_t me = __ballot_sync(FULL, vend);
+		if (me) {
+			const int32_t pos = bw_append<MW>(&sh.n_e, me);
+			if (vend && pos < ne) sh.e[pos] = (uint32_t)id << 3 | l;
+		}
+		// a neighbour whose diagonal beside it was live stays listed by itself
+		const bool act = live && (e.x & 8);
+		if (__any_sync(FULL, act)) {
+			bw_side<MW>(act, id, l, par ^ 1);
+			if (__any_sync(FULL, sh.ovf != 0)) break;
+		}
+	} while (at.x || at.y > 0);
+	found = __any_sync(FULL, found), any = __any_sync(FULL, any);
+	far = __reduce_max_sync(FULL, far);
+	if (lane == 0) {
+		if (found) sh.found = 1;
+		if (any) sh.any = 1;
+		if constexpr (MW) atomicMax(&sh.far, far);
+		else sh.far = far;
+	}
+	__syncwarp();
+}
+
+// Inlined into the one-warp kernel (100,000 x 1 kbp: 14.3 -> 13.4 ms); out of line with several warps,
+// whose time is that of one read (20 kbp at 10%: 84.7 against 88.7 ms inlined)
+static __device__ __noinline__ void bw_narrow_mw(const int32_t *cur, int32_t n_cur, int32_t *list0, int32_t *list1,
+                                                 int32_t T, bool lag, int32_t max_steps)
+{
+	bw_narrow<true>(cur, n_cur, list0, list1, T, lag, max_steps);
+}
+static __device__ __noinline__ void bw_wide_mw(const int32_t *cur, int32_t n_cur, int32_t T)
+{
+	bw_wide<true>(cur, n_cur, T);
+}
+
+// Step 2: the vertex-end states of e over their arcs, in waves, until no state is entered with a
+// free match (gwf-ed.cu:1106-1255). Four lanes per state, one arc each. Begins and ends at a
+// barrier.
+template <bool MW>
+static __device__ __noinline__ void bw_waves(int32_t T)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31;
+	const int32_t wid = MW ? threadIdx.x >> 5 : 0, nw = MW ? blockDim.x >> 5 : 1;
+	const int32_t ql = sh.ql, ne = sh.nb, s = sh.s;
+	const int np = ~s & 1;
+	BwBlock *const blk = sh.blk;
+	int32_t far = INT32_MIN, n_e = sh.n_e;
+	bw_bar<MW>(); // every warp has read the flags of step 1 before one is set here
 #pragma unroll 1
-		for (int32_t base = 0; base < n_e; base += 8) {
+	for (int32_t wave = 0; n_e > 0; ++wave) {
+		const uint32_t *const E = wave & 1 ? sh.f : sh.e;
+		uint32_t *const F = wave & 1 ? sh.e : sh.f;
+#pragma unroll 1
+		for (int32_t base = 8 * wid; base < n_e; base += 8 * nw) {
 			const bool act = base + (lane >> 2) < n_e;
-			const uint32_t e = sh.e[act ? base + (lane >> 2) : 0];
+			const uint32_t e = E[act ? base + (lane >> 2) : 0];
 			const int32_t id = (int32_t)(e >> 3), cl = (int32_t)(e & 7);
 			const int4 b0 = *(const int4 *)(blk + id); // gb, arcs, v, db
 			const int32_t vl = blk[id].vl, i = b0.w + cl + vl - 1;
@@ -539,6 +801,7 @@ static __device__ __noinline__ int32_t bw_waves(int32_t s, int32_t T, int32_t n_
 			// least scores of a path through the deletion into an arc's target and the mismatch
 			const int32_t ha = s + 1 + (int32_t)sh.h[ql - 1 - i], hb = s + 1 + (int32_t)sh.h[ql - 2 - i];
 			const uint32_t max_deg = __reduce_max_sync(FULL, deg);
+			bool full = false;
 #pragma unroll 1
 			for (uint32_t t0 = lane & 3; t0 < max_deg + (lane & 3); t0 += 4) {
 				const bool has = t0 < deg;
@@ -546,53 +809,67 @@ static __device__ __noinline__ int32_t bw_waves(int32_t s, int32_t T, int32_t n_
 				if (has) a = __ldg(sh.arcx + aoff + t0);
 				const uint32_t w = a.x;
 				const int32_t ol = (int32_t)(a.y & 0x3fffffff), dd = i + 1 - ol;
-				bool eq = has && (sh.packed ? a.y >> 30 == qc : __ldg(sh.graw + a.z + ol) == sh.qraw[i + 1]);
+				const bool eq = has && (sh.packed ? a.y >> 30 == qc : __ldg(sh.graw + a.z + ol) == sh.qraw[i + 1]);
 				n_ext += __popc(__ballot_sync(FULL, eq) >> (lane & 28) & 15);
 				// arrival key 0 is never new (gwf-ed.cu:1022-1026); a state that the bound drops leaves
 				// no mark: later arrivals are dropped too
 				const bool on = has && !(w == 0 && i == -1) && (eq ? hb - 1 : hb) < T;
 				if (!__any_sync(FULL, on)) continue;
-				const int32_t id2 = bw_get(on, w, dd >> 3, a.z, (int32_t)a.w);
-				if (sh.ovf) break;
+				const int32_t id2 = bw_get<MW>(on, w, dd >> 3, a.z, (int32_t)a.w);
+				if ((full = __any_sync(FULL, sh.ovf != 0))) break;
 				int32_t *const cp = blk[id2].c + (dd & 7);
-				const int32_t cw = *cp;
-				bool neu = on && !(cw & 1);
-				const uint32_t same = __match_any_sync(FULL, neu ? (id2 << 3 | (dd & 7)) : -1 - lane);
-				neu = neu && (same & lanemask_lt()) == 0;
-				const bool enter = neu && eq, two = neu && !eq;
-				if (neu) *cp = (two ? max(cw >> 1, ol) : cw >> 1) << 1 | 1;
+				bool neu, enter, two;
+				if constexpr (MW) { // of several lanes one sets the cell's arrival bit
+					neu = on && !(atomicOr(cp, 1) & 1);
+					enter = neu && eq, two = neu && !eq;
+					if (two) atomicMax(cp, ol << 1 | 1);
+				} else {
+					const int32_t cw = *cp;
+					neu = on && !(cw & 1);
+					const uint32_t same = __match_any_sync(FULL, neu ? (id2 << 3 | (dd & 7)) : -1 - lane);
+					neu = neu && (same & lanemask_lt()) == 0;
+					enter = neu && eq, two = neu && !eq;
+					if (neu) *cp = (two ? max(cw >> 1, ol) : cw >> 1) << 1 | 1;
+				}
 				const uint32_t mn = __ballot_sync(FULL, enter);
-				const int32_t pn = n_n + __popc(mn & lanemask_lt());
-				if (enter && pn < ne) sh.n[pn] = (uint32_t)id2 << 3 | (dd & 7), sh.nk[pn] = ol;
-				n_n += __popc(mn);
+				if (mn) {
+					const int32_t pn = bw_append<MW>(&sh.n_n[wave & 1], mn);
+					if (enter && pn < ne) sh.n[pn] = (uint32_t)id2 << 3 | (dd & 7), sh.nk[pn] = ol;
+				}
 				__syncwarp();
 				if (__any_sync(FULL, two)) {
 					if (two) blk[id2].has_c = 1;
-					bw_push(two, id2, np);
-					bw_cand(two && ha < T, w, dd - 1, a.z, (int32_t)a.w, ol, np);
-					if (sh.ovf) break;
+					bw_push<MW>(two, id2, np);
+					bw_cand<MW>(two && ha < T, w, dd - 1, a.z, (int32_t)a.w, ol, np);
+					if ((full = __any_sync(FULL, sh.ovf != 0))) break;
 				}
 			}
 			// entered states that reached the vertex end: the diagonal has ended (gwf-ed.cu:1177-1183),
 			// and the insertion at the vertex end stays where an arc did not match
 			// (gwf-ed.cu:1225-1226). For the states of step 1 the successor rule does both.
-			if (wave > 0 && !sh.ovf) {
+			if (wave > 0 && !full) {
 				const bool one = act && (lane & 3) == 0;
-				if (one) blk[id].c[cl] = BW_ENDED << 1 | 1, blk[id].has_c = 1;
+				if (one) {
+					if constexpr (MW) atomicMax(blk[id].c + cl, BW_ENDED << 1 | 1);
+					else blk[id].c[cl] = BW_ENDED << 1 | 1;
+					blk[id].has_c = 1;
+				}
 				__syncwarp();
-				bw_push(one, id, np);
-				bw_cand(one && (n_ext != deg || deg == 0), (uint32_t)b0.z, i - vl + 2, (uint32_t)b0.x, vl, vl - 1, np);
+				bw_push<MW>(one, id, np);
+				bw_cand<MW>(one && (n_ext != deg || deg == 0), (uint32_t)b0.z, i - vl + 2, (uint32_t)b0.x, vl, vl - 1, np);
 			}
-			if (sh.ovf) break;
+			if (__any_sync(FULL, sh.ovf != 0)) break;
 		}
-		if (n_n > ne || wave > ql + 2) sh.ovf = 1;
-		__syncwarp();
-		if (sh.ovf) break;
+		bw_bar<MW>();
+		const int32_t n_n = sh.n_n[wave & 1];
+		if (threadIdx.x == 0) { // the other parity's counters: read before the barrier above
+			sh.n_n[~wave & 1] = 0, sh.n_f[~wave & 1] = 0;
+			if (n_n > ne || wave > ql + 2) sh.ovf = 1;
+		}
 		// extension of the entered states (gwf-ed.cu:1132-1160): one that stays inside its vertex
 		// joins the step's row, whose successors are its three candidates
-		int32_t n_f = 0;
 #pragma unroll 1
-		for (int32_t base = 0; base < n_n; base += 32) {
+		for (int32_t base = 32 * wid; base < n_n && n_n <= ne; base += 32 * nw) {
 			const bool act = base + lane < n_n;
 			const int32_t j = act ? base + lane : 0;
 			const uint32_t e = sh.n[j];
@@ -603,48 +880,54 @@ static __device__ __noinline__ int32_t bw_waves(int32_t s, int32_t T, int32_t n_
 			const int32_t i = act ? d + k : INT32_MIN;
 			far = max(far, i);
 			const bool qend = i == ql - 1, in = act && !qend && k + 1 < vl, toF = act && !qend && !in;
-			found |= qend;
+			if (qend) sh.found = 1;
 			if (in && B->row[np ^ 1][cl] < k) B->row[np ^ 1][cl] = k;
 			const uint32_t mf = __ballot_sync(FULL, toF);
-			if (toF) sh.f[n_f + __popc(mf & lanemask_lt())] = (uint32_t)id << 3 | cl;
-			n_f += __popc(mf); // n_f <= n_n <= ne
+			if (mf) {
+				const int32_t pf = bw_append<MW>(&sh.n_f[wave & 1], mf); // n_f <= n_n <= ne
+				if (toF) F[pf] = (uint32_t)id << 3 | cl;
+			}
 			if (__any_sync(FULL, in)) {
-				bw_push(in, id, np);
+				bw_push<MW>(in, id, np);
 				const bool eb = in && (cl == 0 || cl == 7);
-				if (__any_sync(FULL, eb)) bw_side(eb, id, cl, np);
+				if (__any_sync(FULL, eb)) bw_side<MW>(eb, id, cl, np);
 			}
 		}
-		if (__any_sync(FULL, found)) return INT32_MAX;
-		uint32_t *const t = sh.e;
-		__syncwarp();
-		sh.e = sh.f;
-		__syncwarp();
-		sh.f = t;
-		n_e = n_f;
-		__syncwarp();
+		bw_bar<MW>();
+		n_e = sh.n_f[wave & 1];
+		const bool stop = sh.found || sh.ovf;
+		bw_bar<MW>(); // every warp has read them before the next wave sets them
+		if (stop) break;
 	}
-	return far;
+	far = __reduce_max_sync(FULL, far);
+	if (lane == 0) {
+		if constexpr (MW) atomicMax(&sh.far, far);
+		else sh.far = max(sh.far, far);
+	}
+	bw_bar<MW>();
 }
 
-// Aligns read r with one warp in the arena wsb laid out by p.bw; the hash table is empty (-1) on
-// entry and on return. All control flow is warp-uniform.
+// Aligns read r with the CTA in the arena wsb laid out by p.bw; the hash table is empty on entry and
+// on return. All control flow is uniform over the CTA between barriers.
+template <bool MW>
 __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, uint8_t *wsb)
 {
 	BwShm &sh = bw_sh();
 	const int lane = threadIdx.x & 31;
+	const bool lead = threadIdx.x == 0, warp0 = !MW || threadIdx.x < 32;
 	const DevGraph &g = p.g;
 	const int32_t ql = p.r.ql[r], v0 = p.r.v0[r];
 	if (ql <= 0 || v0 < 0 || (uint32_t)v0 >= g.n_vtx) {
-		if (lane == 0) p.dist[r] = -1, p.status[r] = ST_BAD_INPUT;
+		if (lead) p.dist[r] = -1, p.status[r] = ST_BAD_INPUT;
 		return;
 	}
-	BwBlock *const blk = (BwBlock *)wsb;
-	__syncwarp();
-	sh.qpk = p.r.pk + p.r.pk_off[r], sh.qraw = p.r.raw + p.r.raw_off[r];
-	sh.ql = ql, sh.packed = g.pure && p.r.pure[r], sh.quirk = !(p.flags & 1);
-	__syncwarp();
-	const int32_t kmin1 = sh.quirk ? 0 : -1; // least offset of a candidate after the first step
-	const int32_t ne = p.bw.nb, max_steps = (ql < 64 ? 64 : ql) * 4 + 1024;
+	int32_t *const list0 = (int32_t *)(wsb + p.bw.list0), *const list1 = (int32_t *)(wsb + p.bw.list1);
+	if (lead) {
+		sh.qpk = p.r.pk + p.r.pk_off[r], sh.qraw = p.r.raw + p.r.raw_off[r];
+		sh.ql = ql, sh.packed = g.pure && p.r.pure[r], sh.quirk = !(p.flags & 1);
+	}
+	bw_bar<MW>();
+	const int32_t max_steps = (ql < 64 ? 64 : ql) * 4 + 1024;
 
 	int32_t dist = -1, st = ST_OK, steps = 0;
 	int32_t T = BW_INF;    // states with s + h >= T are dropped
@@ -652,165 +935,80 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 	bool lag = false;      // the run that looks for such a T
 	int32_t h0 = 0;
 	if (g.bloom && ql >= kPruneMinQl) {
-		h0 = bw_seeds(g.bloom_k);
+		h0 = bw_seeds<MW>(g.bloom_k);
 		// nearly all windows at their largest cost: the read is unlike the graph, and no bound helps
 		lag = (float)h0 < 1.7f * (float)(ql / g.bloom_k);
 	}
-	for (;;) { // runs of the score loop
-		uint32_t off_cur = p.bw.list0;
-		sh.n_blk = 0, sh.ovf = 0;
-		__syncwarp();
-		bw_get(lane == 0, (uint32_t)v0, 0, (uint32_t)__ldg(g.base + v0), (int32_t)__ldg(g.len + v0));
-		// the start state (v0, 0), k = -1, as an arc-side candidate (gwf-ed.cu:1303-1308)
-		if (lane == 0) blk[0].c[0] = -2, blk[0].has_c = 1, blk[0].inl[0] = 1, *(int32_t *)(wsb + off_cur) = 0;
-		__syncwarp();
-		int32_t n_cur = 1, imin = INT32_MIN, s = 0;
-		int32_t sc = -1; // the run's score
 #pragma unroll 1
-		for (;; ++s) {
-			const int32_t *const cur = (const int32_t *)(wsb + off_cur);
-			bool found = false, any = false;
-			int32_t n_e = 0, far = INT32_MIN;
+	for (;;) { // runs of the score loop
+		if (lead) sh.n_blk = 0, sh.ovf = 0, sh.s = 0, sh.imin = INT32_MIN;
+		__syncwarp();
+		if (warp0) {
+			bw_get<MW>(lane == 0, (uint32_t)v0, 0, (uint32_t)__ldg(g.base + v0), (int32_t)__ldg(g.len + v0));
+			// the start state (v0, 0), k = -1, as an arc-side candidate (gwf-ed.cu:1303-1308)
+			if (lane == 0) sh.blk[0].c[0] = -2, sh.blk[0].has_c = 1, sh.blk[0].inl[0] = 1, list0[0] = 0;
+		}
+		const int32_t *cur = list0;
+		int32_t n_cur = 1, s = 0;
+		int32_t sc = -1; // the run's score
+		bool ovf = false;
+#pragma unroll 1
+		for (;;) {
+			if (lead) {
+				sh.nxt = s & 1 ? list0 : list1;
+				sh.n_nxt = 0, sh.n_e = 0, sh.next = 0, sh.any = 0, sh.found = 0, sh.far = INT32_MIN;
+				sh.n_n[0] = 0, sh.n_f[0] = 0;
+			}
+			bw_bar<MW>();
 			if (s >= max_steps) {
-				sh.ovf = 1;
+				ovf = true;
 				break;
 			}
-			// ---- 1. successors and extension of the live blocks
-			if (n_cur <= 4) {
-				// Up to four blocks: one lane per diagonal, and step after step in registers until one
-				// reaches its vertex's end or the query's, none lives, or a live edge diagonal has its
-				// neighbour outside the four blocks (unlisted blocks have no live diagonals).
-				const int gr = lane >> 3, l = lane & 7;
-				const bool has = gr < n_cur;
-				const int32_t id = cur[has ? gr : 0];
-				BwBlock *const B = blk + id;
-				const int4 b0 = *(const int4 *)B, h1 = *((const int4 *)B + 1); // gb, arcs, v, db; vl, left, right, flags
-				int32_t k = has ? B->row[~s & 1][l] : BW_NONE;
-				const uint32_t fl = (uint32_t)h1.w; // ended, has_c, inl[0], inl[1]
-				const bool edge = (0x81 >> l & 1) != 0;
-				const int32_t nid = l == 0 ? h1.y : h1.z, vl = h1.x, d = b0.w + l;
-				int src = -1; // edge lanes: the lane of the diagonal across
-#pragma unroll
-				for (int j = 0; j < 4; ++j)
-					if (__shfl_sync(FULL, id, 8 * j) == nid && j < n_cur && edge) src = 8 * j + 7 - l;
-				const bool out = edge && src < 0, nu = l == 0 && out, nd = l == 7 && out;
-				const int su = l == 0 ? max(src, 0) : lane - 1, sd = l == 7 ? max(src, 0) : lane + 1;
-				bool dead = !has || (fl >> l & 1); // absent, or past the vertex end
-				int32_t c = BW_NONE;               // the first step's arc-side candidates
-				if (__any_sync(FULL, has && (fl & 0xff00))) {
-					const int32_t cw = B->c[l];
-					if (has) c = cw >> 1, B->c[l] = 2 * BW_NONE | (cw & 1);
-				}
-				int32_t lo = s == 0 ? -1 : kmin1;
-				bool live, qend, vend;
-#pragma unroll 1
-				for (;;) {
-					const int32_t up = __shfl_sync(FULL, k, su), dn = __shfl_sync(FULL, k, sd);
-					k = max(max(nu ? BW_NONE : up, max(k, nd ? BW_NONE : dn) + 1), c);
-					dead |= k >= vl; // at the first step only: later ones follow no vertex end
-					live = !dead && k >= lo;
-					const int32_t hv = sh.h[live ? ql - 1 - d - k : 0]; // any value below BW_INF while T is BW_INF
-					live = live && s + hv < T && d + k >= imin;
-					k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
-					if (!live) k = BW_NONE;
-					far = live ? d + k : INT32_MIN;
-					qend = far == ql - 1, vend = live && k == vl - 1 && !qend;
-					const bool stop = qend || vend || (live && out) || s + 1 >= max_steps;
-					if (__any_sync(FULL, stop) || !__any_sync(FULL, live)) break;
-					if (lag) imin = __reduce_max_sync(FULL, far) - kPruneLag;
-					++s, lo = kmin1, c = BW_NONE;
-				}
-				found = qend, any = live;
-				const int par = s & 1, np = par ^ 1;
-				// back to the blocks: both rows, the ended diagonals, the next list
-				const uint32_t em = (__ballot_sync(FULL, has && dead) >> (8 * gr)) & 0xff;
-				const uint32_t ml = __ballot_sync(FULL, live);
-				if (has) B->row[par][l] = k, B->row[np][l] = BW_NONE;
-				const bool first = l == 0 && has, app = first && (ml >> (8 * gr) & 0xff) != 0;
-				if (first) *((uint32_t *)B + 7) = em | (app ? 0x10000u << (8 * np) : 0);
-				const uint32_t mp = __ballot_sync(FULL, app);
-				off_cur = par ? p.bw.list1 : p.bw.list0; // the list at hand is in registers
-				int32_t *const nxt = (int32_t *)(wsb + (par ? p.bw.list0 : p.bw.list1));
-				if (app) nxt[__popc(mp & lanemask_lt())] = id;
-				sh.nxt = nxt, sh.n_nxt = __popc(mp);
-				const uint32_t me = __ballot_sync(FULL, vend);
-				if (vend) sh.e[__popc(me & lanemask_lt())] = (uint32_t)id << 3 | l;
-				n_e = __popc(me);
-				__syncwarp();
-				// a live edge diagonal gives the neighbouring block a candidate at the next step
-				const bool act = live && edge && (src < 0 || (ml >> (src & 24) & 0xff) == 0);
-				if (__any_sync(FULL, act)) bw_side(act, id, l, np);
-			} else {
-				// More blocks: two lanes per block and four diagonals per lane; the diagonals that may
-				// live go through the warp's queue, so that the extension runs on full warps (of a dense
-				// graph's diagonals in live blocks one in four lives).
-				const int par = s & 1;
-				int2 at = make_int2(0, 0); // next block, queued diagonals
-				sh.nxt = (int32_t *)(wsb + (par ? p.bw.list0 : p.bw.list1)), sh.n_nxt = 0;
-				__syncwarp();
-#pragma unroll 1
-				do {
-					if (at.y < 32 && at.x < n_cur) at = bw_fill(cur, at.x, n_cur, at.y, par, s == 0 ? -1 : kmin1);
-					const int32_t take = min(at.y, 32); // from the queue's end
-					at.y -= take;
-					const bool alive = lane < take;
-					const uint2 e = sh.queue[at.y + (alive ? lane : 0)];
-					const int32_t id = alive ? (int32_t)(e.x >> 4) : 0, l = (int32_t)(e.x & 7);
-					int32_t k = (int32_t)e.y;
-					const int4 b0 = *(const int4 *)(blk + id);
-					const int32_t vl = blk[id].vl, d = b0.w + l;
-					const int32_t hv = sh.h[alive ? ql - 1 - d - k : 0];
-					const bool live = alive && s + hv < T && d + k >= imin;
-					k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
-					if (live) blk[id].row[par][l] = k;
-					const int32_t i = live ? d + k : INT32_MIN;
-					far = max(far, i);
-					const bool qend = i == ql - 1, vend = live && k == vl - 1 && !qend;
-					found |= qend;
-					any |= live;
-					const uint32_t me = __ballot_sync(FULL, vend);
-					if (me) {
-						const int32_t pos = n_e + __popc(me & lanemask_lt());
-						if (vend && pos < ne) sh.e[pos] = (uint32_t)id << 3 | l;
-						n_e += __popc(me);
-					}
-					// a neighbour whose diagonal beside it was live stays listed by itself
-					const bool act = live && (e.x & 8);
-					if (__any_sync(FULL, act)) {
-						bw_side(act, id, l, par ^ 1);
-						if (sh.ovf) break;
-					}
-				} while (at.x < n_cur || at.y > 0);
-				__syncwarp();
-			}
-			if (__any_sync(FULL, found)) {
+			// ---- 1. successors and extension of the live blocks (may go on to a later step)
+			if constexpr (MW) {
+				if (n_cur > 4) bw_wide_mw(cur, n_cur, T);
+				else if (warp0) bw_narrow_mw(cur, n_cur, list0, list1, T, lag, max_steps);
+			} else if (n_cur > 4)
+				bw_wide<MW>(cur, n_cur, T);
+			else
+				bw_narrow<MW>(cur, n_cur, list0, list1, T, lag, max_steps);
+			bw_bar<MW>();
+			s = sh.s;
+			if (sh.found) {
 				sc = s;
 				break;
 			}
-			if (!__any_sync(FULL, any)) break; // no state is left
+			if (!sh.any) break; // no state is left
 			// ---- 2. vertex-end states over arcs
-			if (n_e > ne) sh.ovf = 1;
-			__syncwarp();
-			if (sh.ovf) break;
-			if (n_e > 0) {
-				far = max(far, bw_waves(s, T, n_e));
-				if (__any_sync(FULL, far == INT32_MAX)) {
+			ovf = sh.ovf || sh.n_e > sh.nb;
+			if (ovf) break;
+			if (sh.n_e > 0) {
+				bw_waves<MW>(T);
+				if (sh.found) {
 					sc = s;
 					break;
 				}
-				if (sh.ovf) break;
+				ovf = sh.ovf != 0;
+				if (ovf) break;
 			}
 			n_cur = sh.n_nxt;
-			off_cur = s & 1 ? p.bw.list0 : p.bw.list1;
-			if (lag) imin = __reduce_max_sync(FULL, far) - kPruneLag;
+			cur = s & 1 ? list0 : list1;
+			++s;
+			const int32_t far = sh.far;
+			bw_bar<MW>();
+			if (lead) {
+				sh.s = s;
+				if (lag) sh.imin = far - kPruneLag;
+			}
+			__syncwarp();
 		}
 		// the hash table back to empty
-		__syncwarp();
-		const int32_t n_blk = sh.n_blk;
-		const bool ovf = sh.ovf != 0;
+		bw_bar<MW>();
+		const int32_t n_blk = min(sh.n_blk, sh.nb);
 #pragma unroll 1
-		for (int32_t j = lane; j < n_blk; j += 32) sh.hash[sh.slot[j]].y = 0xffffffffu;
-		__syncwarp();
+		for (int32_t j = threadIdx.x; j < n_blk; j += MW ? blockDim.x : 32)
+			sh.hash[sh.slot[j]] = make_uint2(0xffffffffu, 0xffffffffu);
+		bw_bar<MW>();
 		if (lag) { // its score, where it found one, is the bound
 			lag = false;
 			if (sc >= 0) {
@@ -820,7 +1018,7 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 				// dense one); windows from every base cost the time of ~0.2 per base and make the
 				// slack 2.2 times smaller.
 				const float slack = (float)(T - h0);
-				if ((p.dens_milli >= 20 ? 8.0f : 1.2f) * slack * slack > (float)ql) bw_seeds(1);
+				if ((p.dens_milli >= 20 ? 8.0f : 1.2f) * slack * slack > (float)ql) bw_seeds<MW>(1);
 			}
 			continue;
 		}
@@ -832,7 +1030,7 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 		steps = dist >= 0 ? dist + 1 : s;
 		break;
 	}
-	if (lane == 0) {
+	if (lead) {
 		p.dist[r] = st == ST_OK ? dist : -1;
 		p.status[r] = st;
 		if (st == ST_CAPACITY && p.retry_list) {
@@ -843,34 +1041,55 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 	}
 }
 
+// Points the CTA's shared state at its arena and empties the hash table.
+__device__ __forceinline__ void bw_init(const DevGraph &g, const BwLay &bw, uint8_t *wsb)
+{
+	BwShm &sh = bw_sh();
+	if (threadIdx.x == 0) {
+		sh.blk = (BwBlock *)wsb, sh.hash = (uint2 *)(wsb + bw.hash), sh.slot = (uint32_t *)(wsb + bw.slot);
+		sh.e = (uint32_t *)(wsb + bw.e), sh.f = (uint32_t *)(wsb + bw.f), sh.n = (uint32_t *)(wsb + bw.n);
+		sh.nk = (int32_t *)(wsb + bw.nk), sh.h = (uint16_t *)(wsb + bw.h);
+		sh.gpk = (const uint32_t *)g.pk, sh.graw = g.raw, sh.arcx = g.arcx, sh.varcs = g.varcs;
+		sh.arc_off = g.arc_off, sh.bloom = g.bloom, sh.bloom_mask = g.bloom_mask, sh.K = g.bloom_k;
+		sh.hmask = (uint32_t)bw.hs - 1, sh.nb = bw.nb;
+	}
+	int4 *const h4 = (int4 *)(wsb + bw.hash);
+#pragma unroll 1
+	for (int32_t j = threadIdx.x; j < bw.hs / 2; j += blockDim.x) h4[j] = make_int4(-1, -1, -1, -1);
+	__syncthreads();
+}
+
 // Persistent form: each one-warp CTA owns one arena (p.bw, sized for the longest read of the
 // launch) and pulls reads from the cost-ordered queue.
 __global__ void __launch_bounds__(32, 32) k_align_blocks(const __grid_constant__ KParams p)
 {
-	BwShm &sh = bw_sh();
-	const int lane = threadIdx.x;
 	uint8_t *const wsb = p.ws + (int64_t)blockIdx.x * p.bw.total;
-	if (lane == 0) {
-		sh.blk = (BwBlock *)wsb, sh.hash = (uint2 *)(wsb + p.bw.hash), sh.slot = (uint32_t *)(wsb + p.bw.slot);
-		sh.e = (uint32_t *)(wsb + p.bw.e), sh.f = (uint32_t *)(wsb + p.bw.f), sh.n = (uint32_t *)(wsb + p.bw.n);
-		sh.nk = (int32_t *)(wsb + p.bw.nk), sh.h = (uint16_t *)(wsb + p.bw.h);
-		sh.gpk = (const uint32_t *)p.g.pk, sh.graw = p.g.raw, sh.arcx = p.g.arcx, sh.varcs = p.g.varcs;
-		sh.arc_off = p.g.arc_off, sh.bloom = p.g.bloom, sh.bloom_mask = p.g.bloom_mask, sh.K = p.g.bloom_k;
-		sh.hmask = (uint32_t)p.bw.hs - 1, sh.nb = p.bw.nb;
-	}
-	{
-		int4 *const h4 = (int4 *)(wsb + p.bw.hash);
-#pragma unroll 1
-		for (int32_t j = lane; j < p.bw.hs / 2; j += 32) h4[j] = make_int4(-1, -1, -1, -1);
-	}
-	__syncwarp();
+	bw_init(p.g, p.bw, wsb);
 #pragma unroll 1
 	for (int32_t guard = 0; guard < p.n_order + 1; ++guard) {
 		int32_t qi = 0;
-		if (lane == 0) qi = atomicAdd(p.head, 1);
+		if (threadIdx.x == 0) qi = atomicAdd(p.head, 1);
 		qi = __shfl_sync(FULL, qi, 0);
 		if (qi >= p.n_order) break;
-		align_read_blocks(p, p.order[qi], wsb);
+		align_read_blocks<false>(p, p.order[qi], wsb);
+	}
+}
+
+// The same with all warps of a CTA on one read.
+__global__ void __launch_bounds__(512, 2) k_align_blocks_mw(const __grid_constant__ KParams p)
+{
+	BwShm &sh = bw_sh();
+	uint8_t *const wsb = p.ws + (int64_t)blockIdx.x * p.bw.total;
+	bw_init(p.g, p.bw, wsb);
+#pragma unroll 1
+	for (int32_t guard = 0; guard < p.n_order + 1; ++guard) {
+		if (threadIdx.x == 0) sh.claim = atomicAdd(p.head, 1);
+		__syncthreads();
+		const int32_t qi = sh.claim;
+		__syncthreads(); // every thread has the claim before the next one is written
+		if (qi >= p.n_order) break;
+		align_read_blocks<true>(p, p.order[qi], wsb);
+		__syncthreads();
 	}
 }
 #endif

@@ -13,7 +13,7 @@
 // takes each branch as a whole. Long candidate lists are radix-sorted with one histogram per
 // warp (stable in the warp order), the same dense-key mapping as warp_radix_sort.
 #pragma once
-#include "gwf_kernels.cuh"
+#include "gwf_blocks.cuh"
 
 namespace gwfb {
 
@@ -948,23 +948,27 @@ __device__ __forceinline__ void run_class(const KParams &p, const ClassParams &c
 }
 
 #ifndef GWF_KERNELS_DECL_ONLY
-// Serving form with groups of NW warps: k_serve's claim, pack, align and completion steps, with
-// one read per group. The group's first thread claims (the same bounded, backed-off polling and
-// closing rule as k_serve, the leader group closing the kernel), the group packs the read and
-// aligns it with align_read_grp, and the first thread writes the completion record.
+// Serving form, one CTA of NW warps per read. The CTA's first thread claims the next published queue
+// position (bounded, backed-off polling of device memory), the CTA packs the read that the host
+// copied into its arena and aligns it: in the block form, or, where the host marked it so (a target
+// vertex, lag pruning, graphs that the block form does not take, the largest arena classes), in the
+// sorted form. The first thread writes a completion record into host-mapped memory (an arena
+// overflow comes back as GWF_E_CAPACITY; the host re-queues the read in a larger arena).
+// The kernel ends as a whole: the leader CTA marks q_head closed after idle_ns with nothing queued
+// and no CTA busy (any CTA does after max_idle_ns), and every CTA leaves when it sees the mark. A
+// CTA counts itself busy before it tries to claim, so the leader never closes under a claim in
+// progress. The host relaunches the kernel when positions are queued and it has ended.
 template <int NW>
-__global__ void __launch_bounds__(256, 3) k_serve_grp(const __grid_constant__ SrvParams p)
+__global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constant__ SrvParams p)
 {
-	__shared__ GrpShm gsh[4];
-	if (threadIdx.x < 4 * 8) ((uint32_t *)gsh[threadIdx.x >> 3].ctr)[threadIdx.x & 7] = 0;
-	__syncthreads();
-	const int gi = (threadIdx.x >> 5) / NW;
-	Grp<NW> G;
-	G.init(gsh + gi, gi);
+	__shared__ GrpShm gsh;
+	__shared__ int32_t impure;
 	constexpr int GS = 32 * NW;
-	const bool leader = blockIdx.x == 0 && gi == 0;
+	if (threadIdx.x < 8) gsh.ctr[threadIdx.x] = 0;
+	__syncthreads();
+	const bool leader = blockIdx.x == 0, first = threadIdx.x == 0;
 	for (int64_t guard = 0; guard < (1LL << 40); ++guard) {
-		if (G.rank == 0) {
+		if (first) {
 			long long h = -1;
 			const uint64_t t0 = globaltimer_ns();
 			uint32_t ns = 128;
@@ -985,23 +989,24 @@ __global__ void __launch_bounds__(256, 3) k_serve_grp(const __grid_constant__ Sr
 				const int64_t idle = (int64_t)(globaltimer_ns() - t0);
 				if (idle > p.max_idle_ns ||
 				    (leader && idle > p.idle_ns && *(volatile const int32_t *)p.busy == 0)) {
-					atomicCAS(p.q_head, head, head | SRV_CLOSED);
+					atomicCAS(p.q_head, head, head | SRV_CLOSED); // fails if a read was claimed
 					continue;
 				}
 				__nanosleep(ns);
 				if (ns < 32768) ns *= 2;
 			}
-			gsh[gi].claim64 = h;
+			gsh.claim64 = h;
+			impure = 0;
 		}
-		G.sync();
-		const long long h = *(volatile long long *)&gsh[gi].claim64;
-		G.sync(); // every thread has the claim before the next one is written
+		__syncthreads();
+		const long long h = *(volatile long long *)&gsh.claim64;
+		__syncthreads(); // every thread has the claim before the next one is written
 		if (h < 0) break;
 		asm volatile("fence.acq_rel.gpu;" ::: "memory");
 		const SrvEntry *ep = p.q + (h & p.qmask);
 		const uint32_t seq = __ldcg((const unsigned int *)&ep->seq);
-		if (seq != (uint32_t)(h + 1)) {
-			if (G.rank == 0) {
+		if (seq != (uint32_t)(h + 1)) { // cannot happen while the host keeps its ring bounds
+			if (first) {
 				atomicOr(p.err, SRV_ERR_SEQ);
 				atomicOr(p.q_head, SRV_CLOSED);
 				atomicSub(p.busy, 1);
@@ -1009,17 +1014,18 @@ __global__ void __launch_bounds__(256, 3) k_serve_grp(const __grid_constant__ Sr
 			break;
 		}
 		const int32_t tag = __ldcg(&ep->tag), ql = __ldcg(&ep->ql), v0 = __ldcg(&ep->v0);
-		const int32_t v1 = __ldcg(&ep->v1), level = __ldcg(&ep->level);
+		const int32_t v1 = __ldcg(&ep->v1), level = __ldcg(&ep->level), blocks = __ldcg(&ep->blocks);
 		const long long aoff = __ldcg((const long long *)&ep->arena_off);
 		const long long abytes = __ldcg((const long long *)&ep->arena_bytes);
 		uint8_t *ab = p.arena + aoff;
 		SrvHdr *hdr = (SrvHdr *)ab;
 		uint64_t *pk = (uint64_t *)(ab + 256);
 		const uint8_t *raw = ab + 256 + srv_pk_bytes(ql);
+		// pack as k_pack_reads does; the raw bytes came by DMA, so they are read from L2
 		const int32_t L = ql > 0 ? ql : 0;
 		const int32_t nwords = (L + 31) / 32 + 2;
 		bool ok = true;
-		for (int32_t w = G.rank; w < nwords; w += GS) {
+		for (int32_t w = threadIdx.x; w < nwords; w += GS) {
 			uint64_t word = 0;
 			for (int32_t t = 0; t < 32; ++t) {
 				const int32_t i = w * 32 + t;
@@ -1031,18 +1037,20 @@ __global__ void __launch_bounds__(256, 3) k_serve_grp(const __grid_constant__ Sr
 			}
 			pk[w] = word;
 		}
-		const bool pure = G.or_bits(ok ? 0u : 1u) == 0;
-		if (G.rank == 0) {
-			hdr->zero = 0, hdr->ql = ql, hdr->v0 = v0, hdr->pure = pure ? 1 : 0;
+		if (!ok) impure = 1;
+		__syncthreads();
+		if (first) {
+			hdr->zero = 0, hdr->ql = ql, hdr->v0 = v0, hdr->pure = impure ? 0 : 1;
 			hdr->dist = -1, hdr->status = ST_CAPACITY;
 		}
-		G.sync();
+		__syncthreads();
 		int32_t dist = -1, st = ST_CAPACITY;
 		const int64_t qb = srv_qbytes(ql);
-		const Caps c = caps_for(ql, level, p.dens_milli);
-		if (qb + ws_layout(c).total <= abytes) {
-			KParams lp;
-			memset(&lp, 0, sizeof lp);
+		KParams lp;
+		memset(&lp, 0, sizeof lp);
+		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli);
+		const int64_t need = blocks ? lp.bw.total : ws_layout(caps_for(ql, level, p.dens_milli)).total;
+		if (qb + need <= abytes) { // the host sized it so; else report capacity
 			lp.g = p.g;
 			lp.r.pk = pk;
 			lp.r.pk_off = &hdr->zero;
@@ -1058,13 +1066,20 @@ __global__ void __launch_bounds__(256, 3) k_serve_grp(const __grid_constant__ Sr
 			lp.max_lag = p.max_lag;
 			lp.dist = &hdr->dist;
 			lp.status = &hdr->status;
-			if (p.max_lag > 0) align_read_grp<NW, true>(lp, 0, ab + qb, ql, level, gsh + gi, gi);
-			else align_read_grp<NW, false>(lp, 0, ab + qb, ql, level, gsh + gi, gi);
-			G.sync();
+			if (blocks) {
+				bw_init(lp.g, lp.bw, ab + qb);
+				align_read_blocks<(NW > 1)>(lp, 0, ab + qb);
+			} else if constexpr (NW == 1)
+				align_read(lp, 0, ab + qb, ql, level);
+			else if (p.max_lag > 0)
+				align_read_grp<NW, true>(lp, 0, ab + qb, ql, level, &gsh, 0);
+			else
+				align_read_grp<NW, false>(lp, 0, ab + qb, ql, level, &gsh, 0);
+			__syncthreads();
 			dist = *(volatile int32_t *)&hdr->dist;
 			st = *(volatile int32_t *)&hdr->status;
 		}
-		if (G.rank == 0) {
+		if (first) {
 			const unsigned long long pos = atomicAdd(p.cq_tail, 1ULL);
 			volatile SrvDone *d = p.cq + (pos & p.cmask);
 			d->tag = tag, d->dist = dist, d->status = st;
@@ -1072,7 +1087,7 @@ __global__ void __launch_bounds__(256, 3) k_serve_grp(const __grid_constant__ Sr
 			d->gen = (int32_t)((pos >> p.cq_shift) + 1);
 			atomicSub(p.busy, 1);
 		}
-		G.sync();
+		__syncthreads();
 	}
 }
 

@@ -12,14 +12,17 @@ struct BwLay {
 	int64_t total;
 };
 
-// Arena for reads of up to ql bases at retry class level (0, 1) on a graph of dens_milli vertices
-// per 1000 bases. Pruned runs of 10 kbp reads at 5% on the dense benchmark graph make ~1,000
-// blocks (34,000 unpruned), 20 kbp reads at 10% ~33,000, 1 kbp reads on the sparse graph ~50.
+// Arena for reads of up to ql bases at retry class level on a graph of dens_milli vertices per 1000
+// bases. Pruned runs of 10 kbp reads at 5% on the dense benchmark graph make ~1,000 blocks (34,000
+// unpruned), 20 kbp reads at 10% ~33,000, 1 kbp reads on the sparse graph ~50, random 1 kbp reads
+// ~400. Class 0 (serving's first, where arenas share a budget) leaves out what reads unlike the
+// graph need, class 1 holds it (the first of a batch), class 2 is 8 times as large.
 __host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli)
 {
 	const int64_t q = ql < 64 ? 64 : ql;
-	int64_t nb = 128 + q / 2 + (int64_t)dens_milli * q * q / 400000 + (int64_t)dens_milli * q * 8 / 1000;
-	if (level > 0) nb *= 8;
+	int64_t nb = 128 + (int64_t)dens_milli * q * q / 400000 + (int64_t)dens_milli * q * 8 / 1000;
+	if (level > 0) nb += q / 2;
+	if (level > 1) nb *= 8;
 	if (nb > (1 << 22)) nb = 1 << 22;
 	BwLay o;
 	o.nb = (int32_t)nb, o.hs = pow2ceil_i(2 * o.nb);
@@ -73,14 +76,15 @@ struct KParams {
 //   [0, 256)              SrvHdr
 //   [256, 256 + pkb)      2-bit packed read, written by the warp
 //   [.., + rawb)          raw read bytes (+16 padding), copied in by the host before publication
-//   [srv_qbytes(ql), ..)  wavefront workspace for caps_for(ql, level)
+//   [srv_qbytes(ql), ..)  workspace: bw_layout(ql, level) in the block form, else for caps_for(ql, level)
 struct SrvEntry {         // queue entry, 48 bytes
 	uint32_t seq;         // queue position + 1 (checks that the entry is the one claimed)
 	int32_t tag;          // host slot of the read
 	int64_t arena_off;    // byte offset of the read's arena in the pool
 	int64_t arena_bytes;
 	int32_t ql, v0, v1, level;
-	int32_t pad[2];
+	int32_t blocks;       // 1: block form, the arena laid out by bw_layout(ql, level)
+	int32_t pad;
 };
 struct SrvDone {          // completion record in host-mapped memory
 	int32_t tag, dist, status, gen; // gen = pass over the ring + 1, written last
@@ -96,7 +100,7 @@ struct SrvParams {
 	const unsigned long long *q_tail;  // published by the host (device memory)
 	unsigned long long *q_head;        // next position to claim
 	const int32_t *stop;               // host sets 1 to end the kernel
-	int32_t *busy;                     // warps holding a read
+	int32_t *busy;                     // groups holding a read
 	unsigned long long *cq_tail;       // next completion position
 	SrvDone *cq;                       // host-mapped ring, cmask + 1 records
 	int32_t *err;                      // host-mapped error bits (SRV_ERR_*)
@@ -1008,130 +1012,6 @@ __device__ __forceinline__ int32_t ld_acquire_s32(const int32_t *p)
 	int32_t v;
 	asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
 	return v;
-}
-
-// Serving form. A warp claims the next published queue position (bounded, backed-off polling of
-// device memory), packs the read that the host copied into its arena, aligns it at the entry's
-// capacity class, and writes a completion record into host-mapped memory (an arena overflow
-// comes back as GWF_E_CAPACITY; the host re-queues the read in a larger arena).
-// The kernel ends as a whole: one leader warp marks q_head closed after idle_ns with nothing
-// queued and no warp busy (any warp does after max_idle_ns), and every warp leaves when it sees
-// the mark. A warp counts itself busy before it tries to claim, so the leader never closes
-// under a claim in progress. The host relaunches the kernel when positions are queued and it
-// has ended.
-__global__ void __launch_bounds__(256, 3) k_serve(const __grid_constant__ SrvParams p)
-{
-	const int lane = threadIdx.x & 31;
-	const bool leader = blockIdx.x == 0 && (threadIdx.x >> 5) == 0;
-	for (int64_t guard = 0; guard < (1LL << 40); ++guard) {
-		long long h = -1;
-		if (lane == 0) {
-			const uint64_t t0 = globaltimer_ns();
-			uint32_t ns = 128;
-			for (int64_t spin = 0; spin < (1LL << 32); ++spin) {
-				if (ld_acquire_s32(p.stop)) break;
-				const unsigned long long head = *(volatile const unsigned long long *)p.q_head;
-				if (head & SRV_CLOSED) break;
-				const unsigned long long tail = ld_acquire_u64(p.q_tail);
-				if (head < tail) {
-					atomicAdd(p.busy, 1);
-					if (atomicCAS(p.q_head, head, head + 1) == head) {
-						h = (long long)head;
-						break;
-					}
-					atomicSub(p.busy, 1);
-					continue;
-				}
-				const int64_t idle = (int64_t)(globaltimer_ns() - t0);
-				if (idle > p.max_idle_ns ||
-				    (leader && idle > p.idle_ns && *(volatile const int32_t *)p.busy == 0)) {
-					atomicCAS(p.q_head, head, head | SRV_CLOSED); // fails if a read was claimed
-					continue;
-				}
-				__nanosleep(ns);
-				if (ns < 32768) ns *= 2;
-			}
-		}
-		h = __shfl_sync(FULL, h, 0);
-		if (h < 0) break;
-		__syncwarp();
-		asm volatile("fence.acq_rel.gpu;" ::: "memory");
-		const SrvEntry *ep = p.q + (h & p.qmask);
-		const uint32_t seq = __ldcg((const unsigned int *)&ep->seq);
-		if (seq != (uint32_t)(h + 1)) { // cannot happen while the host keeps its ring bounds
-			if (lane == 0) {
-				atomicOr(p.err, SRV_ERR_SEQ);
-				atomicOr(p.q_head, SRV_CLOSED);
-				atomicSub(p.busy, 1);
-			}
-			break;
-		}
-		const int32_t tag = __ldcg(&ep->tag), ql = __ldcg(&ep->ql), v0 = __ldcg(&ep->v0);
-		const int32_t v1 = __ldcg(&ep->v1), level = __ldcg(&ep->level);
-		const long long aoff = __ldcg((const long long *)&ep->arena_off);
-		const long long abytes = __ldcg((const long long *)&ep->arena_bytes);
-		uint8_t *ab = p.arena + aoff;
-		SrvHdr *hdr = (SrvHdr *)ab;
-		uint64_t *pk = (uint64_t *)(ab + 256);
-		const uint8_t *raw = ab + 256 + srv_pk_bytes(ql);
-		// pack as k_pack_reads does; the raw bytes came by DMA, so they are read from L2
-		const int32_t L = ql > 0 ? ql : 0;
-		const int32_t nw = (L + 31) / 32 + 2;
-		bool ok = true;
-		for (int32_t w = lane; w < nw; w += 32) {
-			uint64_t word = 0;
-			for (int32_t t = 0; t < 32; ++t) {
-				const int32_t i = w * 32 + t;
-				if (i < L) {
-					const uint8_t ch = (uint8_t)__ldcg((const unsigned char *)raw + i);
-					ok &= (ch == 'A' || ch == 'C' || ch == 'G' || ch == 'T');
-					word |= (uint64_t)((ch >> 1) & 3) << (2 * t);
-				}
-			}
-			pk[w] = word;
-		}
-		ok = __all_sync(FULL, ok);
-		if (lane == 0) {
-			hdr->zero = 0, hdr->ql = ql, hdr->v0 = v0, hdr->pure = ok ? 1 : 0;
-			hdr->dist = -1, hdr->status = ST_CAPACITY;
-		}
-		__syncwarp();
-		int32_t dist = -1, st = ST_CAPACITY;
-		const int64_t qb = srv_qbytes(ql);
-		const Caps c = caps_for(ql, level, p.dens_milli);
-		if (qb + ws_layout(c).total <= abytes) { // the host sized it so; else report capacity
-			KParams lp;
-			memset(&lp, 0, sizeof lp);
-			lp.g = p.g;
-			lp.r.pk = pk;
-			lp.r.pk_off = &hdr->zero;
-			lp.r.raw = raw;
-			lp.r.raw_off = &hdr->zero;
-			lp.r.ql = &hdr->ql;
-			lp.r.v0 = &hdr->v0;
-			lp.r.pure = &hdr->pure;
-			lp.r.v1 = v1;
-			lp.r.n = 1;
-			lp.dens_milli = p.dens_milli;
-			lp.flags = p.flags;
-			lp.max_lag = p.max_lag;
-			lp.dist = &hdr->dist;
-			lp.status = &hdr->status;
-			align_read(lp, 0, ab + qb, ql, level);
-			__syncwarp();
-			dist = *(volatile int32_t *)&hdr->dist;
-			st = *(volatile int32_t *)&hdr->status;
-		}
-		if (lane == 0) {
-			const unsigned long long pos = atomicAdd(p.cq_tail, 1ULL);
-			volatile SrvDone *d = p.cq + (pos & p.cmask);
-			d->tag = tag, d->dist = dist, d->status = st;
-			__threadfence_system();
-			d->gen = (int32_t)((pos >> p.cq_shift) + 1);
-			atomicSub(p.busy, 1);
-		}
-		__syncwarp();
-	}
 }
 
 // IUPAC complement (upper and lower case; other bytes map to themselves), as the GFA loader

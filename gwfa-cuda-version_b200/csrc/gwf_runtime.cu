@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -366,6 +367,9 @@ Engine::~Engine()
 	for (cudaEvent_t e : stage_ev)
 		if (e) cudaEventDestroy(e);
 	if (stream) cudaStreamDestroy(stream);
+	if (stream2) cudaStreamDestroy(stream2);
+	if (fork) cudaEventDestroy(fork);
+	if (join) cudaEventDestroy(join);
 	if (ev0) cudaEventDestroy(ev0);
 	if (ev1) cudaEventDestroy(ev1);
 }
@@ -382,6 +386,9 @@ Engine *gwf_engine(int dev)
 	E->device = dev;
 	cudaSetDevice(dev);
 	if (cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking) != cudaSuccess ||
+	    cudaStreamCreateWithFlags(&E->stream2, cudaStreamNonBlocking) != cudaSuccess ||
+	    cudaEventCreateWithFlags(&E->fork, cudaEventDisableTiming) != cudaSuccess ||
+	    cudaEventCreateWithFlags(&E->join, cudaEventDisableTiming) != cudaSuccess ||
 	    cudaEventCreate(&E->ev0) != cudaSuccess || cudaEventCreate(&E->ev1) != cudaSuccess ||
 	    !std::all_of(std::begin(E->stage_ev), std::end(E->stage_ev), [](cudaEvent_t &e) {
 		    return cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
@@ -401,7 +408,7 @@ Engine *gwf_engine(int dev)
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_persistent<false>, 256, 0);
 	E->persistent_ctas_per_sm = occ > 0 ? occ : 1;
 	occ = 0;
-	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_blocks, 32, sizeof(BwShm));
+	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_blocks, 32, bw_shm_bytes(1));
 	E->blocks_warps_per_sm = occ > 0 ? occ : 1;
 	occ = 0;
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_align_classes, 256, 0);
@@ -664,36 +671,85 @@ static int enqueue_persistent(Engine &E, KParams p, const PersistPlan &pl, const
 // ---- block form (gwf_blocks.cuh): the persistent queue on block wavefronts. It takes every read
 // that ends at the query's end (no target vertex) on a graph whose in-arcs share one overlap per
 // vertex; lag pruning as an option, targets and mixed overlaps stay with the sorted form.
-static bool blocks_ok(const KParams &p) { return p.r.v1 < 0 && p.max_lag == 0 && p.g.arc_key == nullptr && p.g.arcx != nullptr; }
+static bool blocks_ok(const KParams &p) { return p.r.v1 < 0 && p.max_lag == 0 && gwf_blocks_graph(p.g); }
 
-static int plan_blocks(Engine &E, KParams *p, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
-                       PersistPlan *pl)
+// A launch of the block form over a queue that is ordered longest read first: its first n_mw reads
+// with mw warps each (k_align_blocks_mw), the rest with one, the two kernels side by side.
+struct BlocksPlan {
+	int32_t n_mw = 0, mw = 0;
+	int64_t ctas_mw = 0, ctas = 0;
+	BwLay lay_mw, lay;
+};
+
+// Several warps for a read pay where its own time would set the batch's end: where it costs more
+// than kMwShare even shares of the batch's work (ql^2, as plan_classes) over the warp slots. With
+// the device full a warp runs about a third as fast as alone, hence 3 (3,001 reads of 0.5-10 kbp on
+// the sparse graph, 18.0 ms with one warp each). nw > 0: that many for every read.
+static const double kMwShare = 3.0;
+static const int32_t kMwMinQl = 1500; // shorter reads have no more than a few blocks at a time
+
+static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
+                       int32_t nw, int32_t dens_milli, BlocksPlan *pl)
 {
-	p->bw = bw_layout(ql_cap, level, p->dens_milli);
-	int64_t warps = std::min<int64_t>((int64_t)E.sm_count * warps_per_sm, n_order);
+	const int64_t slots = (int64_t)E.sm_count * warps_per_sm;
+	int32_t cap = ql_cap;
+	*pl = BlocksPlan();
+	if (nw > 1) pl->n_mw = n_order, pl->mw = nw;
+	else if (nw == 0 && B) {
+		double total = 0;
+		for (int32_t i = 0; i < B->n; ++i) total += (double)B->h_ql[(size_t)i] * (double)B->h_ql[(size_t)i];
+		const double from = std::max(sqrt(kMwShare * total / (double)slots), (double)kMwMinQl);
+		const int32_t bucket = from < 2e9 ? (int32_t)from >> 6 : INT32_MAX; // the queue's order is by ql >> 6
+		cap = 0;
+		for (int32_t i = 0; i < B->n; ++i) {
+			const int32_t q = B->h_ql[(size_t)i];
+			if (q >> 6 > bucket) ++pl->n_mw;
+			else cap = std::max(cap, q);
+		}
+		if (pl->n_mw) pl->mw = pl->n_mw <= E.sm_count ? 16 : 8;
+	}
+	pl->lay_mw = bw_layout(ql_cap, level, dens_milli), pl->lay = bw_layout(cap, level, dens_milli);
 	const int64_t budget = std::max<int64_t>(E.mem_budget, (int64_t)E.ws.cap);
-	warps = std::min(warps, budget / p->bw.total);
-	if (warps < 1) {
-		gwf_set_errorf("arena of %lld bytes per warp does not fit the device", (long long)p->bw.total);
+	const int32_t n_one = n_order - pl->n_mw;
+	if (pl->n_mw) pl->ctas_mw = std::min<int64_t>(pl->n_mw, std::max<int64_t>(1, slots / pl->mw));
+	pl->ctas = std::min<int64_t>(n_one, slots);
+	while (pl->ctas_mw > 1 && pl->ctas_mw * pl->lay_mw.total > budget / 2) --pl->ctas_mw;
+	const int64_t left = budget - pl->ctas_mw * pl->lay_mw.total;
+	if (pl->ctas * pl->lay.total > left) pl->ctas = left / pl->lay.total;
+	if (left < 0 || (n_one > 0 && pl->ctas < 1)) {
+		gwf_set_errorf("arenas of %lld and %lld bytes do not fit the device", (long long)pl->lay_mw.total,
+		               (long long)pl->lay.total);
 		return GWF_E_NOMEM;
 	}
 	int rc;
-	if ((rc = E.ws.ensure((size_t)(warps * p->bw.total)))) return rc;
-	if ((rc = E.head.ensure(16))) return rc;
-	pl->ctas = (int)warps;
-	pl->slot = p->bw.total;
-	return 0;
+	if ((rc = E.ws.ensure((size_t)(pl->ctas_mw * pl->lay_mw.total + pl->ctas * pl->lay.total)))) return rc;
+	return E.head.ensure(16);
 }
 
-static int enqueue_blocks(Engine &E, KParams p, const PersistPlan &pl, const int32_t *d_order, int32_t n_order)
+static int enqueue_blocks(Engine &E, KParams p, const BlocksPlan &pl, const int32_t *d_order, int32_t n_order)
 {
-	CK(cudaMemsetAsync(E.head.p, 0, 4, E.stream));
-	p.order = d_order;
-	p.n_order = n_order;
-	p.head = (int32_t *)E.head.p;
-	p.ws = (uint8_t *)E.ws.p;
-	k_align_blocks<<<pl.ctas, 32, sizeof(BwShm), E.stream>>>(p);
-	CK(cudaGetLastError());
+	CK(cudaMemsetAsync(E.head.p, 0, 8, E.stream));
+	const bool two = pl.n_mw > 0 && pl.n_mw < n_order;
+	if (pl.n_mw > 0) {
+		const cudaStream_t s = two ? E.stream2 : E.stream;
+		if (two) {
+			CK(cudaEventRecord(E.fork, E.stream));
+			CK(cudaStreamWaitEvent(s, E.fork, 0));
+		}
+		KParams q = p;
+		q.order = d_order, q.n_order = pl.n_mw, q.head = (int32_t *)E.head.p + 1;
+		q.ws = (uint8_t *)E.ws.p, q.bw = pl.lay_mw;
+		k_align_blocks_mw<<<(int)pl.ctas_mw, 32 * pl.mw, bw_shm_bytes(pl.mw), s>>>(q);
+		CK(cudaGetLastError());
+		if (two) CK(cudaEventRecord(E.join, s));
+	}
+	if (pl.n_mw < n_order) {
+		p.order = d_order + pl.n_mw, p.n_order = n_order - pl.n_mw, p.head = (int32_t *)E.head.p;
+		p.ws = (uint8_t *)E.ws.p + pl.ctas_mw * pl.lay_mw.total, p.bw = pl.lay;
+		k_align_blocks<<<(int)pl.ctas, 32, bw_shm_bytes(1), E.stream>>>(p);
+		CK(cudaGetLastError());
+		if (two) CK(cudaStreamWaitEvent(E.stream, E.join, 0));
+	}
 	return 0;
 }
 
@@ -919,13 +975,16 @@ static int enqueue_classes(Engine &E, KParams p, const ClassLaunch &cl)
 // Level-0 sequence of the persistent form as one CUDA graph: pack, clear the overflow count,
 // persistent kernel, copy the overflow count to the host. Captured once per batch contents and
 // launch shape, replayed on every run.
-static int launch_level0_graph(Engine &E, Batch &B, KParams &p, int ctas_per_sm, bool classes, bool blocks)
+static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_per_sm, bool classes, bool blocks,
+                               int32_t nw)
 {
 	PersistPlan pl;
+	BlocksPlan bp;
 	ClassLaunch cl;
 	int rc;
 	if (blocks) {
-		if ((rc = plan_blocks(E, &p, B.n, B.max_ql, 0, ctas_per_sm, &pl))) return rc;
+		if ((rc = plan_blocks(E, &B, B.n, B.max_ql, 1, ctas_per_sm, nw, p.dens_milli, &bp))) return rc;
+		pl.ctas = (int)bp.ctas, pl.slot = bp.lay.total;
 	} else if (classes) {
 		if ((rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl))) return rc;
 		pl.ctas = cl.ctas, pl.slot = cl.cp.cta_bytes;
@@ -935,13 +994,13 @@ static int launch_level0_graph(Engine &E, Batch &B, KParams &p, int ctas_per_sm,
 	                         (uint64_t)(uint32_t)p.flags | (uint64_t)(uint32_t)p.max_lag << 32,
 	                         (uint64_t)(uintptr_t)B.res.p,
 	                         (uint64_t)(uintptr_t)E.h_small.p, (uint64_t)(uintptr_t)E.retry_list.p,
-	                         blocks ? ~1ULL : classes ? B.cls_key ^ B.cls_gen << 40 : ~0ULL};
+	                         blocks ? ~(1ULL | (uint64_t)bp.n_mw << 8 | (uint64_t)bp.mw << 40 | (uint64_t)bp.ctas_mw << 46) : classes ? B.cls_key ^ B.cls_gen << 40 : ~0ULL};
 	if (!B.gexec || memcmp(key, B.gkey, sizeof key) != 0) {
 		if (B.gexec) cudaGraphExecDestroy(B.gexec), B.gexec = nullptr;
 		CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
 		int erc = enqueue_pack(E, B);
 		if (!erc && cudaMemsetAsync(B.d_count, 0, 4, E.stream) != cudaSuccess) erc = GWF_E_CUDA;
-		if (!erc) erc = blocks ? enqueue_blocks(E, p, pl, B.d_order, B.n)
+		if (!erc) erc = blocks ? enqueue_blocks(E, p, bp, B.d_order, B.n)
 		                : classes ? enqueue_classes(E, p, cl)
 		                        : enqueue_persistent(E, p, pl, B.d_order, B.n, B.max_ql, 0);
 		if (!erc && cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream) != cudaSuccess)
@@ -996,8 +1055,9 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		if (gwf_tune_lookup(E.device, B.dom_bucket, &f, &c)) mode = f, ctas_per_sm = c;
 	}
 	bool classes = false;
-	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p) &&
-	                    *std::max_element(nw_b, nw_b + GWF_TUNE_NBUCKETS) <= 1;
+	// the block form takes one count for the batch: forced, tuned for its dominant bucket, or by rule
+	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p);
+	const int32_t nw_blocks = nw_b[B.dom_bucket];
 	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;
@@ -1009,7 +1069,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	bool count_copied = false;
 	if (ms) CK(cudaEventRecord(E.ev0, E.stream));
 	if (use_graph && mode != GWF_MODE_PLAIN) {
-		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks))) return rc;
+		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks, nw_blocks))) return rc;
 		launches += 2;
 		count_copied = true;
 	} else {
@@ -1018,10 +1078,10 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		if (mode == GWF_MODE_PLAIN) rc = launch_plain(E, p, B, &launches);
 		else if (blocks) {
-			PersistPlan pl;
-			if (!(rc = plan_blocks(E, &p, B.n, B.max_ql, 0, warps_per_sm, &pl)) &&
+			BlocksPlan pl;
+			if (!(rc = plan_blocks(E, &B, B.n, B.max_ql, 1, warps_per_sm, nw_blocks, p.dens_milli, &pl)) &&
 			    !(rc = enqueue_blocks(E, p, pl, B.d_order, B.n)))
-				++launches;
+				launches += 1 + (pl.n_mw > 0 && pl.n_mw < B.n);
 		} else if (classes) {
 			ClassLaunch cl;
 			if (!(rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl)) && !(rc = enqueue_classes(E, p, cl)))
@@ -1058,8 +1118,8 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		KParams q = p;
 		if (level == 0) {
-			PersistPlan pl;
-			if ((rc = plan_blocks(E, &q, nr, cap, 1, warps_per_sm, &pl)) ||
+			BlocksPlan pl; // few reads, and the longest: a group of warps each
+			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, 8, p.dens_milli, &pl)) ||
 			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr)))
 				return rc;
 			++launches;
@@ -1110,13 +1170,14 @@ cudaError_t gwf_launch_persistent(const KParams &p, int ctas, int threads, cudaS
 	return cudaGetLastError();
 }
 
-cudaError_t gwf_launch_serve(const SrvParams &p, int ctas, int threads, cudaStream_t s, int warps_per_read)
+cudaError_t gwf_launch_serve(const SrvParams &p, int ctas, cudaStream_t s, int warps_per_read)
 {
+	const size_t shm = bw_shm_bytes(warps_per_read);
 	switch (warps_per_read) {
-	case 2: k_serve_grp<2><<<ctas, threads, 0, s>>>(p); break;
-	case 4: k_serve_grp<4><<<ctas, threads, 0, s>>>(p); break;
-	case 8: k_serve_grp<8><<<ctas, threads, 0, s>>>(p); break;
-	default: k_serve<<<ctas, threads, 0, s>>>(p); break;
+	case 1: k_serve<1><<<ctas, 32, shm, s>>>(p); break;
+	case 2: k_serve<2><<<ctas, 64, shm, s>>>(p); break;
+	case 4: k_serve<4><<<ctas, 128, shm, s>>>(p); break;
+	default: k_serve<8><<<ctas, 256, shm, s>>>(p); break;
 	}
 	return cudaGetLastError();
 }
@@ -1124,12 +1185,13 @@ cudaError_t gwf_launch_serve(const SrvParams &p, int ctas, int threads, cudaStre
 int gwf_serve_ctas_per_sm(int warps_per_read)
 {
 	int occ = 0;
+	const size_t shm = bw_shm_bytes(warps_per_read);
 	cudaError_t e;
 	switch (warps_per_read) {
-	case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve_grp<2>, 256, 0); break;
-	case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve_grp<4>, 256, 0); break;
-	case 8: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve_grp<8>, 256, 0); break;
-	default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve, 256, 0); break;
+	case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve<1>, 32, shm); break;
+	case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve<2>, 64, shm); break;
+	case 4: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve<4>, 128, shm); break;
+	default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_serve<8>, 256, shm); break;
 	}
 	if (e != cudaSuccess) {
 		cudaGetLastError();

@@ -46,7 +46,8 @@ struct Engine { // per-device launch state: stream, events, warp arenas
 	int classes_ctas_per_sm = 1;
 	int blocks_warps_per_sm = 1;
 	int64_t mem_budget = 0; // device bytes the arenas may take
-	cudaStream_t stream = nullptr;
+	cudaStream_t stream = nullptr, stream2 = nullptr; // stream2: reads with several warps, beside the rest
+	cudaEvent_t fork = nullptr, join = nullptr;
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 	DBuf order, head, retry_list, ws, slot_off;
 	HBuf h_small;
@@ -96,9 +97,10 @@ struct KParams;
 struct SrvParams;
 }
 cudaError_t gwf_launch_persistent(const gwfb::KParams &p, int ctas, int threads, cudaStream_t s);
-cudaError_t gwf_launch_serve(const gwfb::SrvParams &p, int ctas, int threads, cudaStream_t s,
-                             int warps_per_read = 1);
-int gwf_serve_ctas_per_sm(int warps_per_read = 1);
+cudaError_t gwf_launch_serve(const gwfb::SrvParams &p, int ctas, cudaStream_t s, int warps_per_read);
+int gwf_serve_ctas_per_sm(int warps_per_read);
+// the block form takes graphs whose in-arcs share one overlap per vertex, of the sizes of its arc records
+inline bool gwf_blocks_graph(const gwfb::DevGraph &g) { return g.arc_key == nullptr && g.arcx != nullptr; }
 
 #include <mutex>
 std::mutex &gwf_batch_mutex();   // serialises batch calls (one engine per device)

@@ -1,16 +1,16 @@
 // gwf_serve.cu — continuous-batching request loop on a device-resident graph.
 //
-// One resident kernel (k_serve) runs on the device; its warps pull single reads from a queue in
-// device memory. A host pump thread does everything else:
+// One resident kernel (k_serve) runs on the device; its CTAs, one group of warps each, pull single
+// reads from a queue in device memory. A host pump thread does everything else:
 //   * admission: reads of queued requests are admitted in FIFO order while a slot is free and the
 //     arena pool (a fixed device-memory budget) has room for the read's wavefront arena, sized for
 //     its own length; the read's bases are copied into its arena and its queue entry published;
 //   * completion: the kernel writes one record per read into host-mapped memory; the pump frees
 //     the arena and the slot, and completes a request when its last read is done;
 //   * retry: a read that overflows its arena comes back with GWF_E_CAPACITY and is queued again
-//     in a 4x larger arena (up to three times), ahead of new reads;
+//     in a larger arena (up to three times), ahead of new reads;
 //   * liveness: the kernel closes as a whole a few milliseconds after the queue runs dry with no
-//     warp busy; the pump relaunches it when positions are queued and it has ended.
+//     group busy; the pump relaunches it when positions are queued and it has ended.
 // Reads that arrive while others are on the device therefore start as soon as a warp and arena
 // memory are free, and results do not depend on what else is in flight.
 #include <cuda_runtime.h>
@@ -126,6 +126,7 @@ struct gwf_srv_s {
 	const gwf_graph_t *g = nullptr;
 	GraphDev *G = nullptr;
 	int device = 0, sm_count = 0, ctas = 0;
+	bool blocks = false; // reads may take the block form
 	int32_t flags = 0, max_lag = 0, nw = 1; // nw: warps that align one read together
 	int64_t budget = 0;
 	uint32_t qcap = 0, ccap = 0;
@@ -173,10 +174,23 @@ int32_t *stop_dev(gwf_srv_s *S) { return (int32_t *)((unsigned long long *)S->ct
 unsigned long long *cq_tail_dev(gwf_srv_s *S) { return (unsigned long long *)((char *)S->ctl.p + 128); }
 int32_t *busy_dev(gwf_srv_s *S) { return (int32_t *)((char *)S->ctl.p + 256); }
 
-int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, int32_t level)
+// The block form takes reads without a target vertex and without lag pruning, in its three arena
+// classes; the sorted form the rest.
+bool block_form(const gwf_srv_s *S, int32_t v1, int32_t level)
 {
-	const gwfb::Caps c = gwfb::caps_for(ql, level, S->G->dens_milli);
-	return gwfb::srv_al256(gwfb::srv_qbytes(ql) + gwfb::ws_layout(c).total);
+	return S->blocks && v1 < 0 && level < 3;
+}
+
+// Arena of a read, -1 when it can never be served: when the sorted form's, which it may come to
+// need, is larger than the whole budget.
+int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, int32_t v1, int32_t level)
+{
+	const int32_t dens = S->G->dens_milli;
+	int64_t ws = gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
+	if (gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws) > S->pool.cap()) return -1;
+	if (block_form(S, v1, level)) ws = gwfb::bw_layout(ql, level, dens).total;
+	const int64_t bytes = gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws);
+	return bytes <= S->pool.cap() ? bytes : -1;
 }
 
 // Called with S->mu held.
@@ -251,8 +265,8 @@ int admit(gwf_srv_s *S)
 	auto place = [&](int32_t tag) -> int {
 		Slot &sl = S->slots[(size_t)tag];
 		const int32_t ql = sl.r->ql[(size_t)sl.read];
-		const int64_t bytes = arena_bytes(S, ql, sl.level);
-		if (bytes > S->pool.cap()) return -1; // can never fit
+		const int64_t bytes = arena_bytes(S, ql, sl.r->v1, sl.level);
+		if (bytes < 0) return -1; // can never fit
 		const int64_t off = S->pool.alloc(bytes);
 		if (off < 0) return 0;
 		sl.off = off, sl.bytes = bytes;
@@ -325,6 +339,7 @@ int admit(gwf_srv_s *S)
 		e.v0 = r.v0[(size_t)sl.read];
 		e.v1 = r.v1;
 		e.level = sl.level;
+		e.blocks = block_form(S, r.v1, sl.level);
 		++S->q_pos;
 	}
 	// queue entries (two copies when the range wraps), then the tail that publishes them
@@ -374,7 +389,7 @@ int launch(gwf_srv_s *S)
 	p.max_lag = S->max_lag;
 	p.idle_ns = kIdleNs;
 	p.max_idle_ns = kMaxIdleNs;
-	if (gwf_launch_serve(p, S->ctas, 256, S->kstream, S->nw) != cudaSuccess) return -1;
+	if (gwf_launch_serve(p, S->ctas, S->kstream, S->nw) != cudaSuccess) return -1;
 	if (cudaEventRecord(S->kdone, S->kstream) != cudaSuccess) return -1;
 	S->kernel_running = true;
 	++S->launches;
@@ -476,6 +491,7 @@ extern "C" gwf_srv_t *gwf_srv_create(const gwf_graph_t *g, const gwf_srv_opts_t 
 		return nullptr;
 	}
 	S->max_lag = opt && (opt->flags & GWF_F_MAX_LAG) && opt->max_lag > 0 ? opt->max_lag : 0;
+	S->blocks = S->max_lag == 0 && gwf_blocks_graph(G->view());
 	size_t fr = 0, tot = 0;
 	cudaMemGetInfo(&fr, &tot);
 	S->budget = opt && opt->arena_budget_bytes > 0 ? opt->arena_budget_bytes : (int64_t)(fr / 4);

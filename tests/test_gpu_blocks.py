@@ -10,10 +10,13 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _check(G, O, seqs, arcs, reads, v0, flags=0):
+def _check(G, O, seqs, arcs, reads, v0, flags=0, nw=(1, 2, 8)):
     g = G.Graph.from_arrays(seqs, arcs)
     g.index()
     d, st = g.ed_batch(reads, v0, mode=G.MODE_PERSISTENT, flags=flags)
+    for k in nw:
+        d2, st2 = g.ed_batch(reads, v0, mode=G.MODE_PERSISTENT, flags=flags, warps_per_read=k)
+        assert np.array_equal(d2, d) and np.array_equal(st2, st)
     og = O.OracleGraph(seqs, arcs)
     ref, skip = [], []
     for q, v in zip(reads, v0):
@@ -102,6 +105,28 @@ def test_dead_ends_and_unlike_reads(G, O):
     reads = [_walk(rng, seqs, out, 0, 2000) + _rand_seq(rng, n) for n in (0, 3, 200, 700)]
     reads += [_rand_seq(rng, n) for n in (600, 900, 2500)]
     _check(G, O, seqs, arcs, reads, [0] * len(reads))
+
+
+def test_long_and_short_reads_side_by_side(G, O):
+    """A batch whose longest reads get several warps and run beside the rest, launched and
+    replayed as a graph, on new reads of the same resident shape."""
+    w = G.load_workload("config3", n=400)
+    long_ = G.load_workload("config3", n=6000)
+    pick = np.argsort(long_["lens"])[-3:]
+    reads = [bytes(w["cat"][o:o + l]) for o, l in zip(w["offs"], w["lens"])]
+    reads += [bytes(long_["cat"][long_["offs"][i]:long_["offs"][i] + long_["lens"][i]]) for i in pick]
+    v0 = np.concatenate([w["v0"], long_["v0"][pick]])
+    g = w["graph"]
+    g.index()
+    cat, offs, lens = G.pack_reads(reads)
+    og = O.OracleGraph.from_graph(g)
+    ref, _, _ = og.ed_batch(cat, offs, lens, v0, stats=False)
+    rb = G.ResidentBatch(g, cat, offs, lens, v0, mode=G.MODE_PERSISTENT)
+    for graph in (0, 1, 1):
+        rb.run(use_graph=graph)
+        d, st = rb.results()
+        assert (st == 0).all() and np.array_equal(d, ref)
+    rb.close()
 
 
 def test_long_reads_on_a_dense_graph(G, O):
