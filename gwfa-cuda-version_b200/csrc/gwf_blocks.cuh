@@ -149,12 +149,15 @@ struct BwShm {
 	int32_t n_blk;             // blocks in use
 	int32_t ovf;               // a buffer is full
 	// of a step (bw_step_begin)
-	int32_t s, imin;           // score; query position behind which the lag run drops states
+	int32_t s, imin;           // score; query position behind which a lag run drops states
+	int32_t lag;               // the caller's max_lag, 0 = none
+	int32_t far_c;             // with it: the furthest query position of a candidate
 	int32_t n_nxt, n_e;        // lengths of nxt and e
 	int32_t next;              // next entry of the live list to be taken
 	int32_t any, found, far;   // a state lives, one reached the query's end, furthest query position
 	int32_t n_n[2], n_f[2];    // of a wave, by its parity
 	int32_t claim;             // MW: queue position of the group's read
+	int32_t pad;
 };
 __device__ __forceinline__ BwShm &bw_sh()
 {
@@ -635,6 +638,7 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 	BwShm &sh = bw_sh();
 	const int lane = threadIdx.x & 31, gr = lane >> 3, l = lane & 7;
 	const int32_t ql = sh.ql, kmin1 = sh.quirk ? 0 : -1;
+	const int32_t user = sh.lag;
 	int32_t s = sh.s, imin = sh.imin;
 	const bool has = gr < n_cur;
 	const int32_t id = cur[has ? gr : 0];
@@ -665,6 +669,7 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 		k = max(max(nu ? BW_NONE : up, max(k, nd ? BW_NONE : dn) + 1), c);
 		dead |= k >= vl; // at the first step only: later ones follow no vertex end
 		live = !dead && k >= lo;
+		if (user) imin = max(__reduce_max_sync(FULL, live ? d + k : INT32_MIN), INT32_MIN / 2) - user;
 		const int32_t hv = sh.h[live ? ql - 1 - d - k : 0]; // any value below BW_INF while T is BW_INF
 		live = live && s + hv < T && d + k >= imin;
 		k = bw_ext(sh, (uint32_t)b0.x, d, k, vl, live);
@@ -699,6 +704,36 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 	if (__any_sync(FULL, act)) bw_side<MW>(act, id, l, np);
 }
 
+// The furthest query position of a candidate of this step (the caller's lag pruning,
+// gwf-ed.cu:1286-1287, drops what lags it by more than max_lag), as bw_fill forms them, into far_c.
+template <bool MW>
+static __device__ __noinline__ void bw_far(const int32_t *cur, int32_t n_cur, int par, int32_t kmin)
+{
+	BwShm &sh = bw_sh();
+	const int lane = threadIdx.x & 31, np = par ^ 1, l = lane & 7;
+	const int32_t wid = MW ? threadIdx.x >> 5 : 0, nw = MW ? blockDim.x >> 5 : 1;
+	int32_t far = INT32_MIN / 2;
+#pragma unroll 1
+	for (int32_t base = 4 * wid; base < n_cur; base += 4 * nw) { // a lane per diagonal
+		const bool in = base + (lane >> 3) < n_cur;
+		const BwBlock *const B = sh.blk + cur[in ? base + (lane >> 3) : base];
+		const int32_t nid = l == 0 ? B->left : B->right, kk = B->row[np][l];
+		int32_t up = __shfl_up_sync(FULL, kk, 1), dn = __shfl_down_sync(FULL, kk, 1), ek = BW_NONE;
+		if ((l == 0 || l == 7) && nid >= 0) ek = sh.blk[nid].row[np][7 - l];
+		if (l == 0) up = ek;
+		if (l == 7) dn = ek;
+		const int32_t k = max(max(up, max(kk, dn) + 1), B->c[l] >> 1);
+		if (in && k >= kmin && k < B->vl && !(B->ended >> l & 1)) far = max(far, B->db + l + k);
+	}
+	far = __reduce_max_sync(FULL, far);
+	if constexpr (MW) {
+		if (lane == 0) atomicMax(&sh.far_c, far);
+		__syncthreads();
+	} else
+		sh.far_c = far;
+	__syncwarp();
+}
+
 // Step 1 for more blocks: bw_fill's diagonals through the warp's queue, so that the extension runs on
 // full warps (of a dense graph's diagonals in live blocks one in four lives).
 template <bool MW>
@@ -707,8 +742,13 @@ __device__ __forceinline__ void bw_wide(const int32_t *cur, int32_t n_cur, int32
 	BwShm &sh = bw_sh();
 	const uint2 *const queue = bw_queue();
 	const int lane = threadIdx.x & 31;
-	const int32_t ql = sh.ql, s = sh.s, imin = sh.imin, ne = sh.nb;
+	const int32_t ql = sh.ql, s = sh.s, ne = sh.nb;
 	const int par = s & 1;
+	int32_t imin = sh.imin;
+	if (sh.lag) {
+		bw_far<MW>(cur, n_cur, par, s == 0 || !sh.quirk ? -1 : 0);
+		imin = sh.far_c - sh.lag;
+	}
 	bool found = false, any = false;
 	int32_t far = INT32_MIN;
 	int2 at = make_int2(1, 0); // more blocks, queued diagonals
@@ -924,7 +964,7 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 	int32_t *const list0 = (int32_t *)(wsb + p.bw.list0), *const list1 = (int32_t *)(wsb + p.bw.list1);
 	if (lead) {
 		sh.qpk = p.r.pk + p.r.pk_off[r], sh.qraw = p.r.raw + p.r.raw_off[r];
-		sh.ql = ql, sh.packed = g.pure && p.r.pure[r], sh.quirk = !(p.flags & 1);
+		sh.ql = ql, sh.packed = g.pure && p.r.pure[r], sh.quirk = !(p.flags & 1), sh.lag = p.max_lag;
 	}
 	bw_bar<MW>();
 	const int32_t max_steps = (ql < 64 ? 64 : ql) * 4 + 1024;
@@ -934,7 +974,7 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 	bool attained = false; // an alignment of T edits exists
 	bool lag = false;      // the run that looks for such a T
 	int32_t h0 = 0;
-	if (g.bloom && ql >= kPruneMinQl) {
+	if (g.bloom && ql >= kPruneMinQl && p.max_lag == 0) {
 		h0 = bw_seeds<MW>(g.bloom_k);
 		// nearly all windows at their largest cost: the read is unlike the graph, and no bound helps
 		lag = (float)h0 < 1.7f * (float)(ql / g.bloom_k);
@@ -957,7 +997,7 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 			if (lead) {
 				sh.nxt = s & 1 ? list0 : list1;
 				sh.n_nxt = 0, sh.n_e = 0, sh.next = 0, sh.any = 0, sh.found = 0, sh.far = INT32_MIN;
-				sh.n_n[0] = 0, sh.n_f[0] = 0;
+				sh.n_n[0] = 0, sh.n_f[0] = 0, sh.far_c = INT32_MIN / 2;
 			}
 			bw_bar<MW>();
 			if (s >= max_steps) {

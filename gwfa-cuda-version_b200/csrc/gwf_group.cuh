@@ -951,7 +951,7 @@ __device__ __forceinline__ void run_class(const KParams &p, const ClassParams &c
 // Serving form, one CTA of NW warps per read. The CTA's first thread claims the next published queue
 // position (bounded, backed-off polling of device memory), the CTA packs the read that the host
 // copied into its arena and aligns it: in the block form, or, where the host marked it so (a target
-// vertex, lag pruning, graphs that the block form does not take, the largest arena classes), in the
+// vertex, graphs that the block form does not take, the largest arena class), in the
 // sorted form. The first thread writes a completion record into host-mapped memory (an arena
 // overflow comes back as GWF_E_CAPACITY; the host re-queues the read in a larger arena).
 // The kernel ends as a whole: the leader CTA marks q_head closed after idle_ns with nothing queued

@@ -670,8 +670,8 @@ static int enqueue_persistent(Engine &E, KParams p, const PersistPlan &pl, const
 
 // ---- block form (gwf_blocks.cuh): the persistent queue on block wavefronts. It takes every read
 // that ends at the query's end (no target vertex) on a graph whose in-arcs share one overlap per
-// vertex; lag pruning as an option, targets and mixed overlaps stay with the sorted form.
-static bool blocks_ok(const KParams &p) { return p.r.v1 < 0 && p.max_lag == 0 && gwf_blocks_graph(p.g); }
+// vertex; targets and mixed overlaps stay with the sorted form.
+static bool blocks_ok(const KParams &p) { return p.r.v1 < 0 && gwf_blocks_graph(p.g); }
 
 // A launch of the block form over a queue that is ordered longest read first: its first n_mw reads
 // with mw warps each (k_align_blocks_mw), the rest with one, the two kernels side by side.

@@ -174,8 +174,8 @@ int32_t *stop_dev(gwf_srv_s *S) { return (int32_t *)((unsigned long long *)S->ct
 unsigned long long *cq_tail_dev(gwf_srv_s *S) { return (unsigned long long *)((char *)S->ctl.p + 128); }
 int32_t *busy_dev(gwf_srv_s *S) { return (int32_t *)((char *)S->ctl.p + 256); }
 
-// The block form takes reads without a target vertex and without lag pruning, in its three arena
-// classes; the sorted form the rest.
+// The block form takes reads without a target vertex, in its three arena classes; the sorted form
+// the rest.
 bool block_form(const gwf_srv_s *S, int32_t v1, int32_t level)
 {
 	return S->blocks && v1 < 0 && level < 3;
@@ -491,7 +491,7 @@ extern "C" gwf_srv_t *gwf_srv_create(const gwf_graph_t *g, const gwf_srv_opts_t 
 		return nullptr;
 	}
 	S->max_lag = opt && (opt->flags & GWF_F_MAX_LAG) && opt->max_lag > 0 ? opt->max_lag : 0;
-	S->blocks = S->max_lag == 0 && gwf_blocks_graph(G->view());
+	S->blocks = gwf_blocks_graph(G->view());
 	size_t fr = 0, tot = 0;
 	cudaMemGetInfo(&fr, &tot);
 	S->budget = opt && opt->arena_budget_bytes > 0 ? opt->arena_budget_bytes : (int64_t)(fr / 4);

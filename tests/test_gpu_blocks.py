@@ -148,3 +148,21 @@ def test_long_reads_on_a_dense_graph(G, O):
     rb.run()
     assert np.array_equal(rb.steps(), ref + 1)
     rb.close()
+
+
+@pytest.mark.parametrize("lag", [3, 60, 400])
+def test_lag_pruning_in_registers_and_in_lists(G, O, lag):
+    """The caller's lag pruning on a dense graph: a small lag keeps to a few blocks, a large one goes
+    through the lists, with one warp and with several."""
+    sg = G.SynthGraph(30_000, 50, 0.7, 20, 10_000, 200, 800, seed=19)
+    g = G.Graph.from_gfa_text(sg.gfa)
+    g.index()
+    r = sg.reads(8, 2, 700, 2000, 700, 2000, 0.02, 0.12, seed=20)
+    s2v = g.vertex_of_segment()
+    v0 = np.array([s2v[int(o)] for o in r["origin_seg"]], dtype=np.int32)
+    og = O.OracleGraph.from_graph(g)
+    ref = [og.ed(bytes(r["cat"][o:o + n]), int(v), max_lag=lag)[0] for o, n, v in zip(r["offs"], r["lens"], v0)]
+    for nw in (0, 1, 8):
+        d, st = g.ed_batch((r["cat"], r["offs"], r["lens"]), v0, mode=G.MODE_PERSISTENT, flags=G.GWF_F_MAX_LAG,
+                           max_lag=lag, warps_per_read=nw)
+        assert (st == 0).all() and list(d) == ref
