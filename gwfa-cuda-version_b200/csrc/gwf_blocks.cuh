@@ -41,13 +41,26 @@ struct __align__(128) BwBlock {
 	int32_t db;        // diagonal of cell 0 (a multiple of 8)
 	int32_t vl;
 	int32_t left, right; // neighbouring blocks, -1 = none yet
-	uint8_t ended;     // diagonals past the vertex end
-	uint8_t has_c;     // some cell has an arc-side candidate
-	uint8_t inl[2];    // in the live list of even / odd steps
+	uint32_t flags;    // BwBits
 	int32_t row[2][8];
-	int32_t c[8];      // arc-side candidate of the next step, k << 1 | arrived
+	int32_t c[8];      // arc-side candidate of the next step: k << 1 | arrived with one warp, k with several
 };
 static_assert(sizeof(BwBlock) == 128, "one line per block");
+
+// Bits of a block's flags: diagonals past the vertex end (0 to 7), an arc-side candidate is there, in
+// the live list of even / odd steps. With one warp per read the lists and the candidate flag have a
+// byte each, which lanes store without a read; with several warps (MW) they are bits set by
+// atomicOr, and bits 8 to 15 are the cells that an arc has reached, so that one atomicOr takes an
+// arrival, flags its candidate and lists the block.
+template <bool MW>
+struct BwBits {
+	static constexpr uint32_t ended = 0xff, has_c = MW ? 1u << 18 : 0x100u, clear_c = MW ? 1u << 18 : 0xff00u;
+	static __device__ __forceinline__ uint32_t inl(int par) { return 0x10000u << (MW ? par : 8 * par); }
+	static __device__ __forceinline__ uint32_t drop(int par) { return clear_c | (MW ? 0x10000u << par : 0xff0000u << (8 * par)); }
+	static constexpr int32_t none = MW ? BW_NONE : 2 * BW_NONE;
+	static __device__ __forceinline__ int32_t k(int32_t c) { return MW ? c : c >> 1; }
+	static __device__ __forceinline__ int32_t taken(int32_t c) { return MW ? BW_NONE : 2 * BW_NONE | (c & 1); }
+};
 
 // Words and bits of a 16-mer in the graph's filter (4 bits of one 64-bit word).
 __host__ __device__ inline uint32_t bloom_word(uint32_t x, uint32_t mask)
@@ -66,7 +79,7 @@ __host__ __device__ inline uint64_t bloom_bits(uint32_t x)
 
 #ifndef GWF_KERNELS_DECL_ONLY
 constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few steps cost less than a bound
-constexpr int32_t kPruneLag = 12;    // lag of the run that gives an upper bound
+constexpr int32_t kPruneLag = 10;    // lag of the run that gives an upper bound
 
 // The filter's build: every string of K = bloom_k bases that a walk of the graph spells, from
 // every position. One warp per vertex, one start per lane; walks branch through a stack (fewer than
@@ -427,7 +440,7 @@ static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, u
 				int4 *q = (int4 *)(blk + id);
 				q[1] = make_int4(vl, -1, -1, 0);
 				const int4 none = make_int4(BW_NONE, BW_NONE, BW_NONE, BW_NONE);
-				const int4 nonec = make_int4(2 * BW_NONE, 2 * BW_NONE, 2 * BW_NONE, 2 * BW_NONE);
+				const int4 nonec = make_int4(BwBits<MW>::none, BwBits<MW>::none, BwBits<MW>::none, BwBits<MW>::none);
 				q[2] = none, q[3] = none, q[4] = none, q[5] = none, q[6] = nonec, q[7] = nonec;
 				q[0] = make_int4((int)gb, (int)__ldg(sh.varcs + v), (int)v, 8 * bi);
 				sh.slot[id] = sl;
@@ -471,21 +484,24 @@ static __device__ __noinline__ int32_t bw_get(bool on, uint32_t v, int32_t bi, u
 	return max(id, 0);
 }
 
-// Puts block id into the next live list, once (several lanes may name one block). np: the parity of
-// the next step.
+// Puts block id into the next live list, once (several lanes may name one block), and flags its
+// candidates where they have some (has_c). np: the parity of the next step.
 template <bool MW>
-static __device__ __noinline__ void bw_push(bool on, int32_t id, int np)
+static __device__ __noinline__ void bw_push(bool on, int32_t id, int np, bool has_c)
 {
 	BwShm &sh = bw_sh();
-	const uint32_t same = __match_any_sync(FULL, on ? id : -1 - (int)(threadIdx.x & 31));
-	bool app = on && (same & lanemask_lt()) == 0;
-	uint8_t *const f = &sh.blk[id].inl[np];
-	app = app && !*f;
+	uint32_t *const f = &sh.blk[id].flags;
+	bool app;
 	if constexpr (MW) {
-		const uint32_t bit = 0x10000u << (8 * np);
-		if (app) app = !(atomicOr((uint32_t *)(sh.blk + id) + 7, bit) & bit);
-	} else if (app)
-		*f = 1;
+		const uint32_t bit = BwBits<MW>::inl(np);
+		app = on && !(atomicOr(f, bit | (has_c ? BwBits<MW>::has_c : 0u)) & bit);
+	} else {
+		if (on && has_c) ((uint8_t *)f)[1] = 1;
+		const uint32_t same = __match_any_sync(FULL, on ? id : -1 - (int)(threadIdx.x & 31));
+		uint8_t *const in = (uint8_t *)f + 2 + np;
+		app = on && (same & lanemask_lt()) == 0 && !*in;
+		if (app) *in = 1;
+	}
 	const uint32_t m = __ballot_sync(FULL, app);
 	if (m) {
 		const int32_t at = bw_append<MW>(&sh.n_nxt, m);
@@ -494,35 +510,26 @@ static __device__ __noinline__ void bw_push(bool on, int32_t id, int np)
 	__syncwarp();
 }
 
-// Arc-side candidate k for cell c (k << 1 | arrived); MW: other warps may change it
+// Arc-side candidate k for a cell (lanes of a warp that meet on one cell bring the same k)
 template <bool MW>
 __device__ __forceinline__ void bw_raise(int32_t *c, int32_t k)
 {
-	int32_t c0 = MW ? *(volatile int32_t *)c : *c;
-	if constexpr (MW) {
-#pragma unroll 1
-		while (c0 >> 1 < k) { // each retry means that another lane raised it
-			const int32_t was = atomicCAS(c, c0, k << 1 | (c0 & 1));
-			if (was == c0) break;
-			c0 = was;
-		}
-	} else if (c0 >> 1 < k)
-		*c = k << 1 | (c0 & 1);
+	if constexpr (MW) atomicMax(c, k);
+	else {
+		const int32_t c0 = *c;
+		if (c0 >> 1 < k) *c = k << 1 | (c0 & 1);
+	}
 }
 
-// Arc-side candidate k for diagonal d of vertex v at the next step (lanes of a warp that meet on one
-// diagonal bring the same k).
+// Arc-side candidate k for diagonal d of vertex v at the next step
 template <bool MW>
 static __device__ __noinline__ void bw_cand(bool on, uint32_t v, int32_t d, uint32_t gb, int32_t vl, int32_t k, int np)
 {
 	BwShm &sh = bw_sh();
 	const int32_t id = bw_get<MW>(on, v, d >> 3, gb, vl);
-	if (sh.ovf) return;
-	if (on) {
-		bw_raise<MW>(sh.blk[id].c + (d & 7), k);
-		sh.blk[id].has_c = 1;
-	}
-	bw_push<MW>(on, id, np);
+	if (__any_sync(FULL, sh.ovf != 0)) return;
+	if (on) bw_raise<MW>(sh.blk[id].c + (d & 7), k);
+	bw_push<MW>(on, id, np, true);
 }
 
 // A live edge diagonal (act: block id, cell l) gives the neighbouring block a candidate at the next
@@ -541,7 +548,7 @@ static __device__ __noinline__ void bw_side(bool act, int32_t id, int32_t l, int
 		if (__any_sync(FULL, sh.ovf != 0)) return;
 		if (miss) u = w;
 	}
-	bw_push<MW>(act, act ? u : 0, np);
+	bw_push<MW>(act, act ? u : 0, np, false);
 }
 
 // Successors of the live blocks of the list cur (n_cur entries), two lanes per block and four
@@ -580,15 +587,14 @@ static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t n_cur, i
 		const int32_t lf = hf ? ok : ek, rt = hf ? ek : ok;
 		int32_t kq[4] = {max(lf, max(kk.x, kk.y) + 1), max(kk.x, max(kk.y, kk.z) + 1),
 		                 max(kk.y, max(kk.z, kk.w) + 1), max(kk.z, max(kk.w, rt) + 1)};
-		if (__any_sync(FULL, (fl & 0xff00) != 0)) {
+		if (__any_sync(FULL, (fl & BwBits<MW>::clear_c) != 0)) {
 			int4 *const cp = (int4 *)B->c + hf;
 			const int4 c = *cp;
 			__syncwarp();
-			kq[0] = max(kq[0], c.x >> 1), kq[1] = max(kq[1], c.y >> 1);
-			kq[2] = max(kq[2], c.z >> 1), kq[3] = max(kq[3], c.w >> 1);
-			if (in)
-				*cp = make_int4(2 * BW_NONE | (c.x & 1), 2 * BW_NONE | (c.y & 1), 2 * BW_NONE | (c.z & 1),
-				                2 * BW_NONE | (c.w & 1));
+			typedef BwBits<MW> X;
+			kq[0] = max(kq[0], X::k(c.x)), kq[1] = max(kq[1], X::k(c.y));
+			kq[2] = max(kq[2], X::k(c.z)), kq[3] = max(kq[3], X::k(c.w));
+			if (in) *cp = make_int4(X::taken(c.x), X::taken(c.y), X::taken(c.z), X::taken(c.w));
 		}
 		uint32_t en = 0, up = 0;
 #pragma unroll
@@ -602,15 +608,15 @@ static __device__ __noinline__ int2 bw_fill(const int32_t *cur, int32_t n_cur, i
 		const bool stays = up != 0 || (in && max(max(kk.x, kk.y), max(kk.z, kk.w)) > BW_NONE);
 		const uint32_t w = en << (4 * hf) | (stays ? 0x100u : 0u);
 		const uint32_t w2 = w | __shfl_xor_sync(FULL, w, 1);
-		const uint32_t inb = 0x10000u << (8 * np);
+		const uint32_t inb = BwBits<MW>::inl(np);
 		const bool first = hf == 0 && in;
 		bool app = first && (w2 & 0x100) && !(fl & inb);
 		if (in) *((int4 *)B->row[par] + hf) = make_int4(BW_NONE, BW_NONE, BW_NONE, BW_NONE);
-		if constexpr (MW) { // other warps may list the block meanwhile: bytes, and a bit by atomicOr
-			if (first) B->ended = (uint8_t)(fl | w2), B->has_c = 0, B->inl[par] = 0;
-			if (app) app = !(atomicOr((uint32_t *)B + 7, inb) & inb);
+		if constexpr (MW) { // other warps may list the block meanwhile
+			if (first) atomicAnd(&B->flags, ~BwBits<MW>::drop(par));
+			if (first && (app || (w2 & 0xff & ~fl))) app = !(atomicOr(&B->flags, (w2 & 0xff) | (app ? inb : 0)) & inb) && app;
 		} else if (first)
-			*((uint32_t *)B + 7) = (fl & ~(0xff00u | 0xff0000u << (8 * par))) | (w2 & 0xff) | (app ? inb : 0);
+			B->flags = (fl & ~BwBits<MW>::drop(par)) | (w2 & 0xff) | (app ? inb : 0);
 		const uint32_t mp = __ballot_sync(FULL, app);
 		const int32_t at = bw_append<MW>(&sh.n_nxt, mp);
 		if (app) sh.nxt[at] = bid;
@@ -656,10 +662,10 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 	const int su = l == 0 ? max(src, 0) : lane - 1, sd = l == 7 ? max(src, 0) : lane + 1;
 	bool dead = !has || (fl >> l & 1); // absent, or past the vertex end
 	int32_t c = BW_NONE;               // the first step's arc-side candidates
-	if (__any_sync(FULL, has && (fl & 0xff00))) {
+	if (__any_sync(FULL, has && (fl & BwBits<MW>::clear_c))) {
 		const int32_t cw = B->c[l];
 		__syncwarp();
-		if (has) c = cw >> 1, B->c[l] = 2 * BW_NONE | (cw & 1);
+		if (has) c = BwBits<MW>::k(cw), B->c[l] = BwBits<MW>::taken(cw);
 	}
 	int32_t lo = s == 0 ? -1 : kmin1, i;
 	bool live, qend, vend;
@@ -687,7 +693,7 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 	const uint32_t ml = __ballot_sync(FULL, live);
 	if (has) B->row[par][l] = k, B->row[np][l] = BW_NONE;
 	const bool first = l == 0 && has, app = first && (ml >> (8 * gr) & 0xff) != 0;
-	if (first) *((uint32_t *)B + 7) = em | (app ? 0x10000u << (8 * np) : 0);
+	if (first) B->flags = (MW ? fl & 0xff00u : 0u) | em | (app ? BwBits<MW>::inl(np) : 0u); // MW: the cells reached stay
 	const uint32_t mp = __ballot_sync(FULL, app);
 	int32_t *const nxt = par ? list0 : list1; // the list at hand is in registers
 	if (app) nxt[__popc(mp & lanemask_lt())] = id;
@@ -722,8 +728,8 @@ static __device__ __noinline__ void bw_far(const int32_t *cur, int32_t n_cur, in
 		if ((l == 0 || l == 7) && nid >= 0) ek = sh.blk[nid].row[np][7 - l];
 		if (l == 0) up = ek;
 		if (l == 7) dn = ek;
-		const int32_t k = max(max(up, max(kk, dn) + 1), B->c[l] >> 1);
-		if (in && k >= kmin && k < B->vl && !(B->ended >> l & 1)) far = max(far, B->db + l + k);
+		const int32_t k = max(max(up, max(kk, dn) + 1), BwBits<MW>::k(B->c[l]));
+		if (in && k >= kmin && k < B->vl && !(B->flags >> l & 1)) far = max(far, B->db + l + k);
 	}
 	far = __reduce_max_sync(FULL, far);
 	if constexpr (MW) {
@@ -857,16 +863,27 @@ static __device__ __noinline__ void bw_waves(int32_t T)
 				if (!__any_sync(FULL, on)) continue;
 				const int32_t id2 = bw_get<MW>(on, w, dd >> 3, a.z, (int32_t)a.w);
 				if ((full = __any_sync(FULL, sh.ovf != 0))) break;
-				int32_t *const cp = blk[id2].c + (dd & 7);
+				BwBlock *const B = blk + id2;
+				const int cell = dd & 7;
 				bool neu, enter, two;
-				if constexpr (MW) { // of several lanes one sets the cell's arrival bit
-					neu = on && !(atomicOr(cp, 1) & 1);
+				if constexpr (MW) { // of several lanes one sets the cell's bit; a mismatch lists the block
+					const uint32_t inb = BwBits<MW>::inl(np);
+					uint32_t was = inb;
+					if (on) was = atomicOr(&B->flags, 0x100u << cell | (eq ? 0u : inb | BwBits<MW>::has_c));
+					neu = on && !(was >> (8 + cell) & 1);
 					enter = neu && eq, two = neu && !eq;
-					if (two) atomicMax(cp, ol << 1 | 1);
+					if (two) atomicMax(B->c + cell, ol);
+					const bool app = on && !eq && !(was & inb);
+					const uint32_t ma = __ballot_sync(FULL, app);
+					if (ma) {
+						const int32_t at = bw_append<MW>(&sh.n_nxt, ma);
+						if (app) sh.nxt[at] = id2;
+					}
 				} else {
+					int32_t *const cp = B->c + cell;
 					const int32_t cw = *cp;
 					neu = on && !(cw & 1);
-					const uint32_t same = __match_any_sync(FULL, neu ? (id2 << 3 | (dd & 7)) : -1 - lane);
+					const uint32_t same = __match_any_sync(FULL, neu ? (id2 << 3 | cell) : -1 - lane);
 					neu = neu && (same & lanemask_lt()) == 0;
 					enter = neu && eq, two = neu && !eq;
 					if (neu) *cp = (two ? max(cw >> 1, ol) : cw >> 1) << 1 | 1;
@@ -874,29 +891,34 @@ static __device__ __noinline__ void bw_waves(int32_t T)
 				const uint32_t mn = __ballot_sync(FULL, enter);
 				if (mn) {
 					const int32_t pn = bw_append<MW>(&sh.n_n[wave & 1], mn);
-					if (enter && pn < ne) sh.n[pn] = (uint32_t)id2 << 3 | (dd & 7), sh.nk[pn] = ol;
+					if (enter && pn < ne) sh.n[pn] = (uint32_t)id2 << 3 | cell, sh.nk[pn] = ol;
 				}
 				__syncwarp();
 				if (__any_sync(FULL, two)) {
-					if (two) blk[id2].has_c = 1;
-					bw_push<MW>(two, id2, np);
-					bw_cand<MW>(two && ha < T, w, dd - 1, a.z, (int32_t)a.w, ol, np);
-					if ((full = __any_sync(FULL, sh.ovf != 0))) break;
+					// the deletion: one diagonal below, most often in the same block
+					const bool del = two && ha < T, lo = del && cell == 0;
+					if (del && !lo) bw_raise<MW>(B->c + cell - 1, ol);
+					if constexpr (!MW) bw_push<MW>(two, id2, np, true);
+					if (__any_sync(FULL, lo)) {
+						bw_cand<MW>(lo, w, dd - 1, a.z, (int32_t)a.w, ol, np);
+						if ((full = __any_sync(FULL, sh.ovf != 0))) break;
+					}
 				}
 			}
 			// entered states that reached the vertex end: the diagonal has ended (gwf-ed.cu:1177-1183),
 			// and the insertion at the vertex end stays where an arc did not match
 			// (gwf-ed.cu:1225-1226). For the states of step 1 the successor rule does both.
 			if (wave > 0 && !full) {
-				const bool one = act && (lane & 3) == 0;
+				const bool one = act && (lane & 3) == 0, ins = one && (n_ext != deg || deg == 0), hi = ins && cl == 7;
 				if (one) {
-					if constexpr (MW) atomicMax(blk[id].c + cl, BW_ENDED << 1 | 1);
+					if constexpr (MW) atomicMax(blk[id].c + cl, BW_ENDED);
 					else blk[id].c[cl] = BW_ENDED << 1 | 1;
-					blk[id].has_c = 1;
 				}
 				__syncwarp();
-				bw_push<MW>(one, id, np);
-				bw_cand<MW>(one && (n_ext != deg || deg == 0), (uint32_t)b0.z, i - vl + 2, (uint32_t)b0.x, vl, vl - 1, np);
+				if (ins && !hi) bw_raise<MW>(blk[id].c + cl + 1, vl - 1);
+				bw_push<MW>(one, id, np, true);
+				if (__any_sync(FULL, hi))
+					bw_cand<MW>(hi, (uint32_t)b0.z, i - vl + 2, (uint32_t)b0.x, vl, vl - 1, np);
 			}
 			if (__any_sync(FULL, sh.ovf != 0)) break;
 		}
@@ -928,7 +950,7 @@ static __device__ __noinline__ void bw_waves(int32_t T)
 				if (toF) F[pf] = (uint32_t)id << 3 | cl;
 			}
 			if (__any_sync(FULL, in)) {
-				bw_push<MW>(in, id, np);
+				bw_push<MW>(in, id, np, false);
 				const bool eb = in && (cl == 0 || cl == 7);
 				if (__any_sync(FULL, eb)) bw_side<MW>(eb, id, cl, np);
 			}
@@ -986,7 +1008,11 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 		if (warp0) {
 			bw_get<MW>(lane == 0, (uint32_t)v0, 0, (uint32_t)__ldg(g.base + v0), (int32_t)__ldg(g.len + v0));
 			// the start state (v0, 0), k = -1, as an arc-side candidate (gwf-ed.cu:1303-1308)
-			if (lane == 0) sh.blk[0].c[0] = -2, sh.blk[0].has_c = 1, sh.blk[0].inl[0] = 1, list0[0] = 0;
+			if (lane == 0) {
+				sh.blk[0].c[0] = MW ? -1 : -2;
+				sh.blk[0].flags = BwBits<MW>::has_c | BwBits<MW>::inl(0);
+				list0[0] = 0;
+			}
 		}
 		const int32_t *cur = list0;
 		int32_t n_cur = 1, s = 0;
