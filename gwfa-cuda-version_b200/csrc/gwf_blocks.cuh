@@ -667,14 +667,17 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 		__syncwarp();
 		if (has) c = BwBits<MW>::k(cw), B->c[l] = BwBits<MW>::taken(cw);
 	}
-	int32_t lo = s == 0 ? -1 : kmin1, i;
+	int32_t i;
 	bool live, qend, vend;
+	auto successor = [&]() {
+		const int32_t up = __shfl_sync(FULL, k, su), dn = __shfl_sync(FULL, k, sd);
+		return max(nu ? BW_NONE : up, max(k, nd ? BW_NONE : dn) + 1);
+	};
+	k = max(successor(), c);
+	dead |= k >= vl; // later steps follow no vertex end
+	live = !dead && k >= (s == 0 ? -1 : kmin1);
 #pragma unroll 1
 	for (;;) {
-		const int32_t up = __shfl_sync(FULL, k, su), dn = __shfl_sync(FULL, k, sd);
-		k = max(max(nu ? BW_NONE : up, max(k, nd ? BW_NONE : dn) + 1), c);
-		dead |= k >= vl; // at the first step only: later ones follow no vertex end
-		live = !dead && k >= lo;
 		if (user) imin = max(__reduce_max_sync(FULL, live ? d + k : INT32_MIN), INT32_MIN / 2) - user;
 		const int32_t hv = sh.h[live ? ql - 1 - d - k : 0]; // any value below BW_INF while T is BW_INF
 		live = live && s + hv < T && d + k >= imin;
@@ -685,7 +688,9 @@ __device__ __forceinline__ void bw_narrow(const int32_t *cur, int32_t n_cur, int
 		const bool stop = qend || vend || (live && out) || s + 1 >= max_steps;
 		if (__any_sync(FULL, stop) || !__any_sync(FULL, live)) break;
 		if (lag) imin = __reduce_max_sync(FULL, i) - kPruneLag;
-		++s, lo = kmin1, c = BW_NONE;
+		++s;
+		k = successor();
+		live = !dead && k >= kmin1;
 	}
 	const int par = s & 1, np = par ^ 1;
 	// back to the blocks: both rows, the ended diagonals, the next list
@@ -1000,6 +1005,13 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 		h0 = bw_seeds<MW>(g.bloom_k);
 		// nearly all windows at their largest cost: the read is unlike the graph, and no bound helps
 		lag = (float)h0 < 1.7f * (float)(ql / g.bloom_k);
+		if (!lag && p.defer) { // such a read makes thousands of states per step: left to a group of warps
+			if (lead) {
+				p.dist[r] = -1, p.status[r] = ST_CAPACITY;
+				p.retry_list[atomicAdd(p.retry_n, 1)] = r;
+			}
+			return;
+		}
 	}
 #pragma unroll 1
 	for (;;) { // runs of the score loop

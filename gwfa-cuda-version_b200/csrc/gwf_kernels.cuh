@@ -67,7 +67,8 @@ struct KParams {
 	int32_t *path_v;        // path vertices from v0
 	int32_t *path_arc;      // arc index into path_v[j] (-1 for j = 0)
 	int32_t max_nv;
-	BwLay bw;               // block form: layout of a warp's arena
+	BwLay bw;               // block form: layout of a CTA's arena
+	int32_t defer;          // block form, one warp: reads unlike the graph go to the retry list
 };
 
 // ---- serving: one resident kernel, warps pull single reads from a device queue

@@ -746,6 +746,10 @@ static int enqueue_blocks(Engine &E, KParams p, const BlocksPlan &pl, const int3
 	if (pl.n_mw < n_order) {
 		p.order = d_order + pl.n_mw, p.n_order = n_order - pl.n_mw, p.head = (int32_t *)E.head.p;
 		p.ws = (uint8_t *)E.ws.p + pl.ctas_mw * pl.lay_mw.total, p.bw = pl.lay;
+		// with warps to spare, reads unlike the graph wait for the retry launch, where as many warps
+		// share each as there are (2,000 x 1 kbp and their reverse complements: 18.7 -> 14.0 ms with two
+		// warps for each of the latter, 22 with eight, in turns)
+		p.defer = p.retry_list && n_order <= (int64_t)E.sm_count * E.blocks_warps_per_sm;
 		k_align_blocks<<<(int)pl.ctas, 32, bw_shm_bytes(1), E.stream>>>(p);
 		CK(cudaGetLastError());
 		if (two) CK(cudaStreamWaitEvent(E.stream, E.join, 0));
@@ -1118,8 +1122,10 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		KParams q = p;
 		if (level == 0) {
-			BlocksPlan pl; // few reads, and the longest: a group of warps each
-			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, 8, p.dens_milli, &pl)) ||
+			BlocksPlan pl; // as many warps per read as keep all reads running at once
+			int32_t nw = 16;
+			while (nw > 1 && (int64_t)nw * nr > (int64_t)E.sm_count * warps_per_sm) nw >>= 1;
+			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p.dens_milli, &pl)) ||
 			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr)))
 				return rc;
 			++launches;
