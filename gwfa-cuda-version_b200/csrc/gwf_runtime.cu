@@ -681,11 +681,16 @@ struct BlocksPlan {
 	BwLay lay_mw, lay;
 };
 
-// Several warps for a read pay where its own time would set the batch's end: where it costs more
-// than kMwShare even shares of the batch's work (ql^2, as plan_classes) over the warp slots. With
-// the device full a warp runs about a third as fast as alone, hence 3 (3,001 reads of 0.5-10 kbp on
-// the sparse graph, 18.0 ms with one warp each). nw > 0: that many for every read.
-static const double kMwShare = 3.0;
+// Several warps for a read (nw = 0). Where lengths differ, so do costs, by more than ql^2 (a read's
+// error rate is not known here): the longest reads set the batch's end on one warp each, and the more
+// so the fewer reads there are per warp slot. Reads with ql^2 above kMwShare (n / slots)^2 times the
+// mean get 8 warps (16 where that few are as long). Measured, ms with that rule / with one warp
+// each / with 8 each: 3,001 reads of 0.5-10 kbp on the sparse graph 11.3 / 17.7 / 11.3, 8,000 12.8 /
+// 19.3 / 12.0, 20,000 19.8 / 21.5 / -, 50,000 28.5 / 28.3 / 73; 4,000 of 0.5-20 kbp on the dense
+// graph 149 / 403 / 131. Reads of one length (mean above kMwUniform of the largest ql^2) get as many
+// as keep all of them running at once: 1,500 x 10 kbp 22.4 with two / 24.5 / 39.1, 3,000 with one 29.1
+// / 29.1 / 69.9. nw > 0: that many for every read.
+static const double kMwShare = 0.2, kMwUniform = 0.67;
 static const int32_t kMwMinQl = 1500; // shorter reads have no more than a few blocks at a time
 
 static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
@@ -698,15 +703,22 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 	else if (nw == 0 && B) {
 		double total = 0;
 		for (int32_t i = 0; i < B->n; ++i) total += (double)B->h_ql[(size_t)i] * (double)B->h_ql[(size_t)i];
-		const double from = std::max(sqrt(kMwShare * total / (double)slots), (double)kMwMinQl);
-		const int32_t bucket = from < 2e9 ? (int32_t)from >> 6 : INT32_MAX; // the queue's order is by ql >> 6
+		const double mean = total / B->n, top = (double)B->max_ql * (double)B->max_ql;
+		const double per = (double)B->n / (double)slots;
+		int32_t all = 16; // warps per read with which all reads run at once
+		while (all > 1 && (int64_t)all * B->n > slots) all >>= 1;
+		double from = std::max(sqrt(kMwShare * per * per * mean), (double)kMwMinQl);
+		if (mean > kMwUniform * top) from = all > 1 && B->max_ql >= kMwMinQl ? 0 : 4e9;
 		cap = 0;
+		// the queue's order is by ql >> 6, longest first: the reads above a bucket are its head
+		const int64_t bucket = (int64_t)(from / 64) - (from == 0);
 		for (int32_t i = 0; i < B->n; ++i) {
 			const int32_t q = B->h_ql[(size_t)i];
 			if (q >> 6 > bucket) ++pl->n_mw;
 			else cap = std::max(cap, q);
 		}
-		if (pl->n_mw) pl->mw = pl->n_mw <= E.sm_count ? 16 : 8;
+		if (from == 0) pl->mw = all;
+		else if (pl->n_mw) pl->mw = 16LL * pl->n_mw <= slots ? 16 : 8;
 	}
 	pl->lay_mw = bw_layout(ql_cap, level, dens_milli), pl->lay = bw_layout(cap, level, dens_milli);
 	const int64_t budget = std::max<int64_t>(E.mem_budget, (int64_t)E.ws.cap);
@@ -1061,7 +1073,8 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	bool classes = false;
 	// the block form takes one count for the batch: forced, tuned for its dominant bucket, or by rule
 	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p);
-	const int32_t nw_blocks = nw_b[B.dom_bucket];
+	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp 7.5 ms, 10.1 with two)
+	const int32_t nw_blocks = nw_b[B.dom_bucket] == 0 && p.max_lag > 0 ? 1 : nw_b[B.dom_bucket];
 	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;
