@@ -958,6 +958,7 @@ __device__ __forceinline__ void run_class(const KParams &p, const ClassParams &c
 // and no CTA busy (any CTA does after max_idle_ns), and every CTA leaves when it sees the mark. A
 // CTA counts itself busy before it tries to claim, so the leader never closes under a claim in
 // progress. The host relaunches the kernel when positions are queued and it has ended.
+constexpr int32_t kServeMwMinQl = 1500; // shorter reads have few blocks at a time: one warp, without barriers
 template <int NW>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constant__ SrvParams p)
 {
@@ -1068,7 +1069,8 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constan
 			lp.status = &hdr->status;
 			if (blocks) {
 				bw_init(lp.g, lp.bw, ab + qb);
-				align_read_blocks<(NW > 1)>(lp, 0, ab + qb);
+				if (NW > 1 && ql >= kServeMwMinQl) align_read_blocks<(NW > 1)>(lp, 0, ab + qb);
+				else if (threadIdx.x < 32) align_read_blocks<false>(lp, 0, ab + qb);
 			} else if constexpr (NW == 1)
 				align_read(lp, 0, ab + qb, ql, level);
 			else if (p.max_lag > 0)
