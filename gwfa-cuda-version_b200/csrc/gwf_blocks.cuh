@@ -62,7 +62,7 @@ struct BwBits {
 	static __device__ __forceinline__ int32_t taken(int32_t c) { return MW ? BW_NONE : 2 * BW_NONE | (c & 1); }
 };
 
-// Words and bits of a 16-mer in the graph's filter (4 bits of one 64-bit word).
+// Word of a string in the graph's filter, and its bits there: two in each half of the word.
 __host__ __device__ inline uint32_t bloom_word(uint32_t x, uint32_t mask)
 {
 	x *= 0x9E3779B1u;
@@ -70,11 +70,10 @@ __host__ __device__ inline uint32_t bloom_word(uint32_t x, uint32_t mask)
 	x *= 0x2C1B3C6Du;
 	return (x ^ x >> 13) & mask;
 }
-__host__ __device__ inline uint64_t bloom_bits(uint32_t x)
+__host__ __device__ inline uint2 bloom_bits(uint32_t x)
 {
-	uint32_t y = (x ^ x >> 16) * 0x85EBCA6Bu;
-	y ^= y >> 13;
-	return 1ULL << (y & 63) | 1ULL << (y >> 6 & 63) | 1ULL << (y >> 12 & 63) | 1ULL << (y >> 18 & 63);
+	const uint32_t y = (x ^ x >> 16) * 0x85EBCA6Bu;
+	return make_uint2(1u << (y >> 27) | 1u << (y >> 22 & 31), 1u << (y >> 17 & 31) | 1u << (y >> 12 & 31));
 }
 
 #ifndef GWF_KERNELS_DECL_ONLY
@@ -87,6 +86,11 @@ constexpr int32_t kPruneLag = 10;    // lag of the run that gives an upper bound
 // enters all four extensions, so that a string of K - 1 bases may be looked up by extending it. A
 // start with more than kBloomLeaves walks sets *many, and the graph gets no filter.
 constexpr int32_t kBloomLeaves = 1024;
+__device__ __forceinline__ void bloom_put(unsigned long long *bloom, uint32_t mask, uint32_t x)
+{
+	const uint2 b = bloom_bits(x);
+	atomicOr(bloom + bloom_word(x, mask), (unsigned long long)b.y << 32 | b.x);
+}
 __global__ void __launch_bounds__(256) k_bloom(const __grid_constant__ DevGraph g, unsigned long long *bloom,
                                                int32_t *many)
 {
@@ -110,16 +114,13 @@ __global__ void __launch_bounds__(256) k_bloom(const __grid_constant__ DevGraph 
 			}
 			bool up = false;
 			if (n == K) {
-				atomicOr(bloom + bloom_word(x, mask), (unsigned long long)bloom_bits(x));
+				bloom_put(bloom, mask, x);
 				up = true;
 			} else {
 				const uint32_t a = __ldg(g.arc_off + v), e = __ldg(g.arc_off + v + 1);
 				if (a == e) {
 					if (n == K - 1)
-						for (uint32_t y = 0; y < 4; ++y) {
-							const uint32_t z = x | y << (2 * K - 2);
-							atomicOr(bloom + bloom_word(z, mask), (unsigned long long)bloom_bits(z));
-						}
+						for (uint32_t y = 0; y < 4; ++y) bloom_put(bloom, mask, x | y << (2 * K - 2));
 					up = true;
 				} else
 					st_x[depth] = x, st_n[depth] = n, st_a[depth] = a, st_e[depth] = e, ++depth;
@@ -212,30 +213,31 @@ __device__ __forceinline__ int32_t bw_append(int32_t *c, uint32_t m)
 
 __device__ __forceinline__ bool bloom_has(const BwShm &sh, uint32_t x)
 {
-	const uint64_t b = bloom_bits(x);
-	return (__ldg(sh.bloom + bloom_word(x, sh.bloom_mask)) & b) == b;
+	const uint2 b = bloom_bits(x), w = __ldg((const uint2 *)sh.bloom + bloom_word(x, sh.bloom_mask));
+	return ((b.x & ~w.x) | (b.y & ~w.y)) == 0;
 }
 
-// Does the graph (as its filter says) spell the K-base string y with one edit? code = kind << 8 |
-// a << 2 | t. Kind 0: another base (xor t) at a; 1: the base t inserted before a (K + 1 bases: the
-// first K and the last K); 2: the base at a taken out and t appended.
-static __device__ __noinline__ bool bw_edit(uint32_t y, int code)
+// Does the graph (as its filter says) spell the K-base string y with one edit at base a? Kind 0: the
+// base xor t; 1: the base t inserted before a (K + 1 bases: the first K and the last K); 2: the base
+// taken out and t appended.
+template <int KIND>
+__device__ __forceinline__ bool bw_edit(const BwShm &sh, uint32_t y, int a, uint32_t t)
 {
-	const BwShm &sh = bw_sh();
-	const int K = sh.K, kind = code >> 8, a2 = code >> 1 & 126;
-	const uint32_t t = code & 3, lo = y & ((1u << a2) - 1), hi = y >> a2, kmask = ~0u >> (32 - 2 * K);
-	uint32_t z = y ^ t << a2;
-	if (kind == 1) z = ((hi << 2 | t) << a2 | lo) & kmask;
-	if (kind == 2) z = hi >> 2 << a2 | lo | t << (2 * K - 2);
-	bool ok = bloom_has(sh, z);
-	if (ok && kind == 1) ok = bloom_has(sh, (uint32_t)(((uint64_t)(hi << 2 | t) << a2 | lo) >> 2));
+	const int K = sh.K, a2 = 2 * a;
+	if (KIND == 0) return bloom_has(sh, y ^ t << a2);
+	const uint32_t lo = y & ((1u << a2) - 1), hi = y >> a2;
+	if (KIND == 2) return bloom_has(sh, hi >> 2 << a2 | lo | t << (2 * K - 2));
+	const uint64_t z = (uint64_t)(hi << 2 | t) << a2 | lo;
+	bool ok = bloom_has(sh, (uint32_t)z & ~0u >> (32 - 2 * K));
+	if (ok) ok = bloom_has(sh, (uint32_t)(z >> 2));
 	return ok;
 }
 
 // Edits that the last rem bases of the query cannot avoid, rem = 0 .. ql, into h[rem]; returns
 // h[ql]. A window of K bases costs 0, 1 or 2 edits when the graph spells a string within 0, 1 or
 // more edits of it; windows that do not overlap add up, so h[rem] = max(h[rem - 1], h[rem - K] +
-// cost of the window that starts rem bases before the end). Windows start every `stride` bases.
+// cost of the window that starts rem bases before the end). Windows start every `stride` bases: K
+// (side by side, first) or 1 (after that, on the same read).
 // Lanes test 32 windows for exact presence. An absent one is looked up with one edit by the whole
 // warp (3 K substitutions, 4 (K - 1) insertions, 4 K deletions with any appended base); an edit
 // that is found is then tried on the other absent windows of the 32 that hold its position. A
@@ -246,11 +248,9 @@ static __device__ __noinline__ int32_t bw_seeds(int32_t stride)
 {
 	const BwShm &sh = bw_sh();
 	const int lane = threadIdx.x & 31;
-	const int32_t K = sh.K, ql = sh.ql, n_edit = 11 * K - 4;
+	const int32_t K = sh.K, ql = sh.ql;
 	uint16_t *const h = sh.h;
 	const int32_t wid = MW ? threadIdx.x >> 5 : 0, nw = MW ? blockDim.x >> 5 : 1;
-#pragma unroll 1
-	for (int32_t j = 32 * wid + lane; j <= ql; j += 32 * nw) h[j] = 0;
 	bw_bar<MW>();
 #pragma unroll 1
 	for (int32_t base = K + 32 * stride * wid; base <= ql; base += 32 * stride * nw) {
@@ -276,26 +276,63 @@ static __device__ __noinline__ int32_t bw_seeds(int32_t stride)
 		while (todo) {
 			const int src = __ffs(todo) - 1;
 			todo &= todo - 1;
-			uint32_t y = __shfl_sync(FULL, x, src), hit = 0;
+			const uint32_t y = __shfl_sync(FULL, x, src);
 			const int32_t sp = __shfl_sync(FULL, p, src);
-			int code = 0;
+			uint32_t hit = 0;
+			int kind = 0, code = 0; // a << 2 | t of the lane's last try
 #pragma unroll 1
-			for (int t0 = 0; t0 < n_edit && !hit; t0 += 32) {
-				const int t = t0 + lane, u = t - 3 * K, w = u - 4 * (K - 1);
-				code = t < 3 * K ? (t / 3) << 2 | (t % 3 + 1) : w < 0 ? 1 << 8 | (u + 4) : 2 << 8 | w;
-				hit = __ballot_sync(FULL, t < n_edit && bw_edit(y, code));
+			for (int t = lane; t < 3 * K + lane && !hit; t += 32) {
+				code = (t / 3) << 2 | (t % 3 + 1);
+				hit = __ballot_sync(FULL, t < 3 * K && bw_edit<0>(sh, y, code >> 2, code & 3));
+			}
+			if (!hit) kind = 1;
+#pragma unroll 1
+			for (int t = 4 + lane; t < 4 * K + lane && !hit; t += 32) {
+				code = t;
+				hit = __ballot_sync(FULL, t < 4 * K && bw_edit<1>(sh, y, code >> 2, code & 3));
+			}
+			if (!hit) kind = 2;
+#pragma unroll 1
+			for (int t = lane; t < 4 * K + lane && !hit; t += 32) {
+				code = t;
+				hit = __ballot_sync(FULL, t < 4 * K && bw_edit<2>(sh, y, code >> 2, code & 3));
 			}
 			if (!hit) continue;
-			// the same edit in this lane's window
-			const int c = __shfl_sync(FULL, code, __ffs(hit) - 1), kind = c >> 8;
-			const int a = sp + (c >> 2 & 63) - p;
-			const bool same = (todo >> lane & 1) && a >= (kind == 1) && a < K;
-			if (lane == src || (same && bw_edit(x, kind << 8 | a << 2 | (kind == 2 ? (int)nb : c & 3)))) cost = 1;
-			todo &= __ballot_sync(FULL, cost == 2);
+			if (lane == src) cost = 1;
+			if (todo && stride == 1) { // the same edit in this lane's window
+				const int c = __shfl_sync(FULL, code, __ffs(hit) - 1), a = sp + (c >> 2) - p;
+				bool same = (todo >> lane & 1) && a >= (kind == 1) && a < K;
+				if (same)
+					same = kind == 0 ? bw_edit<0>(sh, x, a, c & 3) : kind == 1 ? bw_edit<1>(sh, x, a, c & 3)
+					                                               : bw_edit<2>(sh, x, a, nb);
+				if (same) cost = 1;
+				todo &= __ballot_sync(FULL, cost == 2);
+			}
 		}
 		if (rem <= ql) h[rem] = (uint16_t)cost;
 	}
 	bw_bar<MW>();
+	if (stride == K) {
+		// windows side by side: h[rem] is the sum over the rem / K last of them
+		int32_t sum = 0;
+#pragma unroll 1
+		for (int32_t base = K; base <= ql && wid == 0; base += 32 * K) {
+			const int32_t rem = base + lane * K;
+			int32_t tot;
+			const int32_t c = rem <= ql ? (int32_t)h[rem] : 0, pre = sum + warp_excl_scan(c, &tot);
+			if (rem < ql + K)
+#pragma unroll 1
+				for (int32_t j = rem - K; j < rem && j <= ql; ++j) h[j] = (uint16_t)min(pre, 65535);
+			sum += tot;
+			__syncwarp();
+			if (rem <= ql && rem + K > ql)
+#pragma unroll 1
+				for (int32_t j = rem; j <= ql; ++j) h[j] = (uint16_t)min(pre + c, 65535);
+			__syncwarp();
+		}
+		bw_bar<MW>();
+		return (int32_t)h[ql];
+	}
 	// the maximum over disjoint windows, K entries at a time: lane l's entry takes its window after
 	// h[rem - K] of the pass before
 	int32_t prev = 0; // lane l < K: h[b - K + l]
