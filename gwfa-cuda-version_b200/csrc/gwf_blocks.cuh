@@ -19,11 +19,13 @@
 // configuration 4 962,000 -> 107,000, and 10,700 with windows from every base; the lag run needs
 // 600 and 2,300.
 //
-// What bounds it: instruction issue and fetch (ncu, 1 kbp reads: 0.49 issue slots active per cycle
-// at 32 warps per SM, a third of the stalls waiting for instructions), and the latency of one
-// read's chain of steps where a batch has few or unequal reads. Resident reads, graph replay,
-// kernel_ms against the sorted form: 100,000 x 1 kbp 26.1 -> 12.7 ms, 50,000 mixed 137 -> 27 ms,
-// 4,000 x 10 kbp on the dense graph 600 -> 33 ms, one 20 kbp read at 10% 374 -> 274 ms.
+// What bounds it: instruction fetch and issue (ncu, 20,000 mixed reads of at most 4 kbp: 0.37
+// instructions issued per cycle and scheduler at 32 warps per SM, 9.2 of a warp's 20.4 cycles per
+// instruction waiting for its next instruction, 4.6 for loads, 2.8 for fixed latencies; DRAM 0.76 GB
+// in 7.6 ms), and the latency of one read's chain of steps where a batch has few or unequal reads.
+// Resident reads, graph replay, kernel_ms against the sorted form: 100,000 x 1 kbp 26.1 -> 12.7 ms,
+// 50,000 mixed 137 -> 26 ms, 4,000 x 10 kbp on the dense graph 600 -> 30 ms, one 20 kbp read at 10%
+// 374 -> 69 ms (299 with one warp, 16 here).
 #pragma once
 #include "gwf_kernels.cuh"
 
@@ -54,7 +56,7 @@ static_assert(sizeof(BwBlock) == 128, "one line per block");
 // arrival, flags its candidate and lists the block.
 template <bool MW>
 struct BwBits {
-	static constexpr uint32_t ended = 0xff, has_c = MW ? 1u << 18 : 0x100u, clear_c = MW ? 1u << 18 : 0xff00u;
+	static constexpr uint32_t has_c = MW ? 1u << 18 : 0x100u, clear_c = MW ? 1u << 18 : 0xff00u;
 	static __device__ __forceinline__ uint32_t inl(int par) { return 0x10000u << (MW ? par : 8 * par); }
 	static __device__ __forceinline__ uint32_t drop(int par) { return clear_c | (MW ? 0x10000u << par : 0xff0000u << (8 * par)); }
 	static constexpr int32_t none = MW ? BW_NONE : 2 * BW_NONE;
@@ -138,7 +140,8 @@ __global__ void __launch_bounds__(256) k_bloom(const __grid_constant__ DevGraph 
 // State of a read's run, in the CTA's shared memory (a CTA aligns one read at a time, with one warp
 // or, MW, with several). The parts of the kernel that are not run at every step are functions of
 // their own that work on it: with everything inlined the kernel had 87 KB of code, its 32 warps per
-// SM stood in different parts of it, and the instruction cache held half of their cycles.
+// SM stood in different parts of it, and waits for instructions took 11 of 21 cycles per issue
+// (100,000 x 1 kbp 18.8 ms, 14.3 as functions). bw_ext stays inlined: 12.7 ms, 13.4 out of line.
 constexpr int kBwQueue = 31 + 16 * 8;
 struct BwShm {
 	BwBlock *blk;
@@ -162,7 +165,7 @@ struct BwShm {
 	int32_t ql, packed, quirk;
 	int32_t n_blk;             // blocks in use
 	int32_t ovf;               // a buffer is full
-	// of a step (bw_step_begin)
+	// of a step
 	int32_t s, imin;           // score; query position behind which a lag run drops states
 	int32_t lag;               // the caller's max_lag, 0 = none
 	int32_t far_c;             // with it: the furthest query position of a candidate
@@ -844,8 +847,8 @@ __device__ __forceinline__ void bw_wide(const int32_t *cur, int32_t n_cur, int32
 	__syncwarp();
 }
 
-// Inlined into the one-warp kernel (100,000 x 1 kbp: 14.3 -> 13.4 ms); out of line with several warps,
-// whose time is that of one read (20 kbp at 10%: 84.7 against 88.7 ms inlined)
+// Inlined into the one-warp kernel (100,000 x 1 kbp: 14.3 -> 13.4 ms when this was taken); out of line
+// with several warps, whose time is that of one read (20 kbp at 10%: 84.7 against 88.7 ms inlined)
 static __device__ __noinline__ void bw_narrow_mw(const int32_t *cur, int32_t n_cur, int32_t *list0, int32_t *list1,
                                                  int32_t T, bool lag, int32_t max_steps)
 {
@@ -1175,7 +1178,8 @@ __device__ __forceinline__ void bw_init(const DevGraph &g, const BwLay &bw, uint
 }
 
 // Persistent form: each one-warp CTA owns one arena (p.bw, sized for the longest read of the
-// launch) and pulls reads from the cost-ordered queue.
+// launch) and pulls reads from the cost-ordered queue. 32 warps per SM at 64 registers; 24 or 28
+// lose more on 1 kbp reads (2% and up) than they gain elsewhere.
 __global__ void __launch_bounds__(32, 32) k_align_blocks(const __grid_constant__ KParams p)
 {
 	uint8_t *const wsb = p.ws + (int64_t)blockIdx.x * p.bw.total;
@@ -1190,7 +1194,8 @@ __global__ void __launch_bounds__(32, 32) k_align_blocks(const __grid_constant__
 	}
 }
 
-// The same with all warps of a CTA on one read.
+// The same with all warps of a CTA on one read: one read of 20 kbp at 10% takes 299 ms with one warp,
+// 224 with 2, 138 with 4, 100 with 8 and 85 with 16 (68 since each arrival is one atomic).
 __global__ void __launch_bounds__(512, 2) k_align_blocks_mw(const __grid_constant__ KParams p)
 {
 	BwShm &sh = bw_sh();

@@ -938,13 +938,13 @@ __device__ __forceinline__ void align_read_body(const KParams &p, int32_t r, uin
 #undef BK
 #undef TLOG
 
-// Out-of-line copy of the read loop, for the kernels that hold it beside other work (serving,
-// read classes, traceback). The two batch kernels below inline the body, one instantiation per
+// Out-of-line copy of the read loop, for the kernels that hold it beside other work (read classes,
+// traceback, serving where the block form does not apply). The two batch kernels below inline the body, one instantiation per
 // kernel, and run four CTAs of 8 warps per SM at 64 registers. Inlined, the body spills less at a
 // given register count (-Xptxas -v at 80 registers: 200 B stack against 264 B out of line); at 64
 // registers it spills about as much as the out-of-line body did at 80, and the 32 warps per SM
 // hide more load latency than 24 (config 3: 438 -> 416 ms; config 2: 33.6 -> 32.2 ms; config 4
-// unchanged).
+// unchanged; measured before the block form took over these batches).
 template <bool TR, bool LAG>
 __device__ __noinline__ void align_read_t(const KParams &p, int32_t r, uint8_t *wsb, int32_t ql_cap, int32_t level)
 {

@@ -482,8 +482,8 @@ extern "C" gwf_srv_t *gwf_srv_create(const gwf_graph_t *g, const gwf_srv_opts_t 
 	S->g = g, S->G = G, S->device = dev;
 	S->flags = opt ? opt->flags : 0;
 	// serving is latency-first: a request waits for its slowest read, so by default each read gets
-	// a group of 8 warps (p99 at 70% of peak: 0.79 s against 4.66 s with one warp, on reads of
-	// 0.5-20 kbp on the 5 Mbp graph; peak 2,666 against 1,222 reads/s)
+	// a group of 8 warps, of which one aligns a short read (reads of 0.5-20 kbp on the 5 Mbp graph:
+	// p99 at 70% of peak 0.11 s, peak 20,400 reads/s; 0.64 s and 3,300 in the sorted form)
 	S->nw = opt && opt->warps_per_read > 0 ? opt->warps_per_read : 8;
 	if (S->nw != 1 && S->nw != 2 && S->nw != 4 && S->nw != 8) {
 		gwf_set_error("gwf_srv_create: warps_per_read must be 0, 1, 2, 4 or 8");
