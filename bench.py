@@ -410,10 +410,10 @@ def run_features(args):
 
 def run_case(args):
     """Small fixed cases, one kernel each, sized for profiler captures (a few GB on the device):
-    config3-4k   k_align_persistent: 20,000 config-3 reads of at most 4 kbp, one warp per read,
+    config3-4k   k_align_blocks: 20,000 config-3 reads of at most 4 kbp, one warp per read,
                  four launches;
-    classes      k_align_classes: 100 config-4 reads (10 kbp, 5 Mbp graph), warps per read by
-                 default (eight here), two batches;
+    classes      k_align_blocks_mw: 100 config-4 reads (10 kbp, 5 Mbp graph), warps per read by
+                 default (sixteen here), two batches;
     cigar        k_cigar: 400 config-2 reads with paths and CIGARs, two batches;
     serve        k_serve: four requests of ten config-5 reads on a one-warp server, 1 GiB budget."""
     G = pkg()

@@ -83,12 +83,15 @@ typedef struct {
 	int32_t flags;       /* GWF_F_* */
 	int32_t device;      /* CUDA device ordinal (-1 = current) */
 	int32_t warps_per_read; /* persistent form: warps that align one read together (1, 2, 4 or 8).
-	                           0 = per read: the gwf_tune value of its length bucket for
-	                           GWF_MODE_AUTO, else by its share of the batch's work (cost ql^2
-	                           against the persistent grid's warp slots) and by its arena size:
-	                           reads costing more than one slot's even share, or (in batches of
-	                           fewer than 3 reads per warp slot) whose arenas over every slot
-	                           would pass 16 GiB, get 2, 4 or 8 warps, the others one.
+	                           0 = the gwf_tune value of the length bucket that holds most of the
+	                           batch's work for GWF_MODE_AUTO, else by rule: in a batch of mixed
+	                           lengths the longest reads get 8 or 16 warps, the more of them the
+	                           fewer reads there are per warp slot; reads of one length get as
+	                           many (up to 16) as keep all of them running at once; the others,
+	                           and runs with lag pruning, one. With a target vertex (v1 >= 0), or
+	                           arcs into one vertex of different overlaps, per read: its bucket's
+	                           tuned value, or 2, 4 or 8 warps by its share of the batch's work
+	                           (cost ql^2) and its arena size.
 	                           The plain form uses one warp per read. */
 	int32_t ctas_per_sm;   /* persistent grid; 0 = the autotuned value for GWF_MODE_AUTO (see
 	                          gwf_tune), else the occupancy limit */
@@ -219,9 +222,9 @@ int gwf_ed_batch_noalloc(const gwf_graph_t *g, int32_t n, int32_t max_ql, const 
  * SM, and the plain form, on the given reads, separately for each read-length bucket (ql < 1500,
  * < 3000, < 6000, < 12000, longer; at most max_reads_per_bucket evenly spread reads each, 0 =
  * 8192), and keeps the fastest shape per bucket for the graph's device. Batch calls with mode
- * GWF_MODE_AUTO then align each read with the warps per read of its own bucket (warps_per_read =
- * 0), and take the form and CTAs per SM (ctas_per_sm = 0) of the bucket holding most of the
- * batch's work (sum of ql^2). json_path != NULL also writes the table as JSON; gwf_tune_load
+ * GWF_MODE_AUTO then take the warps per read (warps_per_read = 0), form and CTAs per SM
+ * (ctas_per_sm = 0) of the bucket holding most of the batch's work (sum of ql^2); with a target
+ * vertex, or arcs into one vertex of different overlaps, each read has its own bucket's warps. json_path != NULL also writes the table as JSON; gwf_tune_load
  * reads it back (device -1 = current). */
 #define GWF_TUNE_NBUCKETS 5
 int gwf_tune(const gwf_graph_t *g, int32_t n, const char *seqs, const int64_t *offs, const int32_t *ql,
@@ -239,8 +242,8 @@ void *gwf_pinned_alloc(int64_t bytes);
 void gwf_pinned_free(void *p);
 
 /* ---- serving: continuous batching on a resident graph ----
- * No reference counterpart. One resident kernel aligns reads pulled from a device queue, one
- * warp per read. Reads of queued requests are admitted in FIFO order while a slot is free and
+ * No reference counterpart. One resident kernel aligns reads pulled from a device queue, a group
+ * of warps per read (reads below 1,500 bases on one warp of it). Reads of queued requests are admitted in FIFO order while a slot is free and
  * the arena budget holds the read's wavefront arena (sized for its own length); a read that
  * overflows its arena is queued again in a 4x larger one, up to three times, ahead of new
  * reads. Results equal those of gwf_ed_batch for the same reads, whatever else is in flight. */
