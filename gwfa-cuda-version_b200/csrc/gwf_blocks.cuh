@@ -25,7 +25,7 @@
 // in 7.6 ms), and the latency of one read's chain of steps where a batch has few or unequal reads.
 // Resident reads, graph replay, kernel_ms against the sorted form: 100,000 x 1 kbp 26.1 -> 12.7 ms,
 // 50,000 mixed 137 -> 26 ms, 4,000 x 10 kbp on the dense graph 600 -> 30 ms, one 20 kbp read at 10%
-// 374 -> 69 ms (299 with one warp, 16 here).
+// 374 -> 69 ms (259 with one warp, 16 here).
 #pragma once
 #include "gwf_kernels.cuh"
 
@@ -1194,8 +1194,9 @@ __global__ void __launch_bounds__(32, 32) k_align_blocks(const __grid_constant__
 	}
 }
 
-// The same with all warps of a CTA on one read: one read of 20 kbp at 10% takes 299 ms with one warp,
-// 224 with 2, 138 with 4, 100 with 8 and 85 with 16 (68 since each arrival is one atomic).
+// The same with all warps of a CTA on one read: one read of 20 kbp at 10% takes 259 ms with one warp,
+// 178 with 2, 111 with 4, 81 with 8, 69 with 16 and 67 with 32; 100 reads of 10 kbp at 5% on the dense
+// graph 21.1, 18.0, 15.1, 14.5, 14.3 and 14.5 ms. So 16 is the most a read gets.
 __global__ void __launch_bounds__(512, 2) k_align_blocks_mw(const __grid_constant__ KParams p)
 {
 	BwShm &sh = bw_sh();
