@@ -738,7 +738,18 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 	return E.head.ensure(16);
 }
 
-static int enqueue_blocks(Engine &E, KParams p, const BlocksPlan &pl, const int32_t *d_order, int32_t n_order)
+// With warps to spare, and their number left to the library, reads unlike the graph wait for the
+// retry launch, where as many warps share each as there are (2,000 x 1 kbp and their reverse
+// complements: 18.7 -> 14.0 ms with two warps for each of the latter, 22 with eight, in turns).
+static bool defer_unlike(const Engine &E, int32_t n, int warps_per_sm, int32_t nw)
+{
+	return nw == 0 && n <= (int64_t)E.sm_count * warps_per_sm;
+}
+
+// defer: reads unlike the graph leave the one-warp kernel through the retry list. Never in the retry
+// launch itself, which would hand them to the sorted form without a step in the block form.
+static int enqueue_blocks(Engine &E, KParams p, const BlocksPlan &pl, const int32_t *d_order, int32_t n_order,
+                          bool defer)
 {
 	CK(cudaMemsetAsync(E.head.p, 0, 8, E.stream));
 	const bool two = pl.n_mw > 0 && pl.n_mw < n_order;
@@ -758,10 +769,7 @@ static int enqueue_blocks(Engine &E, KParams p, const BlocksPlan &pl, const int3
 	if (pl.n_mw < n_order) {
 		p.order = d_order + pl.n_mw, p.n_order = n_order - pl.n_mw, p.head = (int32_t *)E.head.p;
 		p.ws = (uint8_t *)E.ws.p + pl.ctas_mw * pl.lay_mw.total, p.bw = pl.lay;
-		// with warps to spare, reads unlike the graph wait for the retry launch, where as many warps
-		// share each as there are (2,000 x 1 kbp and their reverse complements: 18.7 -> 14.0 ms with two
-		// warps for each of the latter, 22 with eight, in turns)
-		p.defer = p.retry_list && n_order <= (int64_t)E.sm_count * E.blocks_warps_per_sm;
+		p.defer = defer && p.retry_list;
 		k_align_blocks<<<(int)pl.ctas, 32, bw_shm_bytes(1), E.stream>>>(p);
 		CK(cudaGetLastError());
 		if (two) CK(cudaStreamWaitEvent(E.stream, E.join, 0));
@@ -998,6 +1006,7 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 	BlocksPlan bp;
 	ClassLaunch cl;
 	int rc;
+	const bool defer = blocks && defer_unlike(E, B.n, ctas_per_sm, nw);
 	if (blocks) {
 		if ((rc = plan_blocks(E, &B, B.n, B.max_ql, 1, ctas_per_sm, nw, p.dens_milli, &bp))) return rc;
 		pl.ctas = (int)bp.ctas, pl.slot = bp.lay.total;
@@ -1010,13 +1019,16 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 	                         (uint64_t)(uint32_t)p.flags | (uint64_t)(uint32_t)p.max_lag << 32,
 	                         (uint64_t)(uintptr_t)B.res.p,
 	                         (uint64_t)(uintptr_t)E.h_small.p, (uint64_t)(uintptr_t)E.retry_list.p,
-	                         blocks ? ~(1ULL | (uint64_t)bp.n_mw << 8 | (uint64_t)bp.mw << 40 | (uint64_t)bp.ctas_mw << 46) : classes ? B.cls_key ^ B.cls_gen << 40 : ~0ULL};
+	                         blocks ? ~(1ULL | (uint64_t)defer << 1 | (uint64_t)bp.n_mw << 8 | (uint64_t)bp.mw << 40 |
+	                                    (uint64_t)bp.ctas_mw << 46)
+	                         : classes ? B.cls_key ^ B.cls_gen << 40
+	                                   : ~0ULL};
 	if (!B.gexec || memcmp(key, B.gkey, sizeof key) != 0) {
 		if (B.gexec) cudaGraphExecDestroy(B.gexec), B.gexec = nullptr;
 		CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
 		int erc = enqueue_pack(E, B);
 		if (!erc && cudaMemsetAsync(B.d_count, 0, 4, E.stream) != cudaSuccess) erc = GWF_E_CUDA;
-		if (!erc) erc = blocks ? enqueue_blocks(E, p, bp, B.d_order, B.n)
+		if (!erc) erc = blocks ? enqueue_blocks(E, p, bp, B.d_order, B.n, defer)
 		                : classes ? enqueue_classes(E, p, cl)
 		                        : enqueue_persistent(E, p, pl, B.d_order, B.n, B.max_ql, 0);
 		if (!erc && cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream) != cudaSuccess)
@@ -1097,7 +1109,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		else if (blocks) {
 			BlocksPlan pl;
 			if (!(rc = plan_blocks(E, &B, B.n, B.max_ql, 1, warps_per_sm, nw_blocks, p.dens_milli, &pl)) &&
-			    !(rc = enqueue_blocks(E, p, pl, B.d_order, B.n)))
+			    !(rc = enqueue_blocks(E, p, pl, B.d_order, B.n, defer_unlike(E, B.n, warps_per_sm, nw_blocks))))
 				launches += 1 + (pl.n_mw > 0 && pl.n_mw < B.n);
 		} else if (classes) {
 			ClassLaunch cl;
@@ -1139,7 +1151,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 			int32_t nw = 16;
 			while (nw > 1 && (int64_t)nw * nr > (int64_t)E.sm_count * warps_per_sm) nw >>= 1;
 			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p.dens_milli, &pl)) ||
-			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr)))
+			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr, false)))
 				return rc;
 			++launches;
 			continue;
