@@ -8,7 +8,7 @@
 //   * completion: the kernel writes one record per read into host-mapped memory; the pump frees
 //     the arena and the slot, and completes a request when its last read is done;
 //   * retry: a read that overflows its arena comes back with GWF_E_CAPACITY and is queued again
-//     in a larger arena (up to three times), ahead of new reads;
+//     in a larger arena (next_class), ahead of new reads;
 //   * liveness: the kernel closes as a whole a few milliseconds after the queue runs dry with no
 //     group busy; the pump relaunches it when positions are queued and it has ended.
 // Reads that arrive while others are on the device therefore start as soon as a warp and arena
@@ -45,7 +45,8 @@ double now_s()
 	return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-constexpr int kMaxLevel = 3;         // arena classes 1x, 4x, 16x, 64x, as the batch path
+constexpr int kBlockLevels = 3;      // arena classes of the block form (bw_layout)
+constexpr int kMaxLevel = 3;         // the sorted form's are 1x, 4x, 16x, 64x
 constexpr int64_t kIdleNs = 5000000; // 5 ms
 constexpr int64_t kMaxIdleNs = 120LL * 1000000000LL;
 
@@ -117,6 +118,7 @@ struct Request {
 struct Slot {
 	std::shared_ptr<Request> r;
 	int32_t read = 0, level = 0;
+	bool blocks = false; // level is a class of the block form
 	int64_t off = -1, bytes = 0;
 };
 
@@ -174,23 +176,36 @@ int32_t *stop_dev(gwf_srv_s *S) { return (int32_t *)((unsigned long long *)S->ct
 unsigned long long *cq_tail_dev(gwf_srv_s *S) { return (unsigned long long *)((char *)S->ctl.p + 128); }
 int32_t *busy_dev(gwf_srv_s *S) { return (int32_t *)((char *)S->ctl.p + 256); }
 
-// The block form takes reads without a target vertex, in its three arena classes; the sorted form
-// the rest.
-bool block_form(const gwf_srv_s *S, int32_t v1, int32_t level)
-{
-	return S->blocks && v1 < 0 && level < 3;
-}
-
-// Arena of a read, -1 when it can never be served: when the sorted form's, which it may come to
-// need, is larger than the whole budget.
-int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, int32_t v1, int32_t level)
+// Arena of a read in a class of the block form or of the sorted form; -1 when it is larger than the
+// whole budget.
+int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, bool blocks, int32_t level)
 {
 	const int32_t dens = S->G->dens_milli;
-	int64_t ws = gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
-	if (gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws) > S->pool.cap()) return -1;
-	if (block_form(S, v1, level)) ws = gwfb::bw_layout(ql, level, dens).total;
+	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens).total : gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
 	const int64_t bytes = gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws);
 	return bytes <= S->pool.cap() ? bytes : -1;
+}
+
+// Arena classes of a read, in turn. Reads without a target vertex take the block form's, as long as
+// they fit the budget, then the sorted form's from 4x on (as the batch path), or from 1x where 4x does
+// not fit; the others take the sorted form's. A read whose first sorted arena does not fit is not
+// served. Both return false when no class is left.
+bool first_class(const gwf_srv_s *S, Slot &sl)
+{
+	const int32_t ql = sl.r->ql[(size_t)sl.read];
+	sl.level = 0;
+	sl.blocks = S->blocks && sl.r->v1 < 0 && arena_bytes(S, ql, true, 0) >= 0;
+	return arena_bytes(S, ql, false, 0) >= 0;
+}
+bool next_class(const gwf_srv_s *S, Slot &sl)
+{
+	const int32_t ql = sl.r->ql[(size_t)sl.read];
+	if (sl.blocks) {
+		if (++sl.level < kBlockLevels && arena_bytes(S, ql, true, sl.level) >= 0) return true;
+		sl.blocks = false, sl.level = arena_bytes(S, ql, false, 1) >= 0 ? 1 : 0;
+		return true;
+	}
+	return ++sl.level <= kMaxLevel && arena_bytes(S, ql, false, sl.level) >= 0;
 }
 
 // Called with S->mu held.
@@ -244,8 +259,7 @@ int drain(gwf_srv_s *S)
 		Slot &sl = S->slots[(size_t)tag];
 		S->pool.release(sl.off, sl.bytes);
 		sl.off = -1;
-		if (st == GWF_E_CAPACITY && sl.level < kMaxLevel) {
-			++sl.level;
+		if (st == GWF_E_CAPACITY && next_class(S, sl)) {
 			++S->retries;
 			S->retry.push_back(tag); // keeps its slot; re-admitted with a larger arena
 			continue;
@@ -262,27 +276,18 @@ int admit(gwf_srv_s *S)
 {
 	std::vector<int32_t> batch;
 	const uint64_t first = S->q_pos;
-	auto place = [&](int32_t tag) -> int {
+	auto place = [&](int32_t tag) -> bool { // the read's class fits the budget
 		Slot &sl = S->slots[(size_t)tag];
-		const int32_t ql = sl.r->ql[(size_t)sl.read];
-		const int64_t bytes = arena_bytes(S, ql, sl.r->v1, sl.level);
-		if (bytes < 0) return -1; // can never fit
+		const int64_t bytes = arena_bytes(S, sl.r->ql[(size_t)sl.read], sl.blocks, sl.level);
 		const int64_t off = S->pool.alloc(bytes);
-		if (off < 0) return 0;
+		if (off < 0) return false;
 		sl.off = off, sl.bytes = bytes;
-		return 1;
+		return true;
 	};
 	while (!S->retry.empty()) {
 		const int32_t tag = S->retry.front();
-		const int rc = place(tag);
-		if (rc == 0) break;
+		if (!place(tag)) break;
 		S->retry.pop_front();
-		if (rc < 0) {
-			Slot &sl = S->slots[(size_t)tag];
-			finish_read(S, sl.r, sl.read, -1, GWF_E_CAPACITY);
-			release_slot(S, tag);
-			continue;
-		}
 		batch.push_back(tag);
 	}
 	while (S->retry.empty() && !S->pending.empty() && !S->free_slots.empty()) {
@@ -293,19 +298,17 @@ int admit(gwf_srv_s *S)
 		} else {
 			const int32_t tag = S->free_slots.back();
 			Slot &sl = S->slots[(size_t)tag];
-			sl.r = r, sl.read = i, sl.level = 0;
-			const int rc = place(tag);
-			if (rc == 0) {
+			sl.r = r, sl.read = i;
+			if (!first_class(S, sl)) {
+				sl.r.reset();
+				finish_read(S, r, i, -1, GWF_E_CAPACITY);
+			} else if (place(tag)) {
+				S->free_slots.pop_back();
+				++S->in_flight;
+				batch.push_back(tag);
+			} else {
 				sl.r.reset();
 				break; // wait for arena memory
-			}
-			S->free_slots.pop_back();
-			++S->in_flight;
-			if (rc < 0) {
-				finish_read(S, r, i, -1, GWF_E_CAPACITY);
-				release_slot(S, tag);
-			} else {
-				batch.push_back(tag);
 			}
 		}
 		if (r->t_admit == 0) r->t_admit = now_s();
@@ -339,7 +342,7 @@ int admit(gwf_srv_s *S)
 		e.v0 = r.v0[(size_t)sl.read];
 		e.v1 = r.v1;
 		e.level = sl.level;
-		e.blocks = block_form(S, r.v1, sl.level);
+		e.blocks = sl.blocks;
 		++S->q_pos;
 	}
 	// queue entries (two copies when the range wraps), then the tail that publishes them
