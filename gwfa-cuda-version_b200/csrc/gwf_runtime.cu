@@ -176,7 +176,7 @@ static uint8_t code2(uint8_t c) { return (uint8_t)((c >> 1) & 3); } // A0 C1 T2 
 // none.
 static int build_bloom(GraphDev *G)
 {
-	if (!G->pure || G->total_len > (1ULL << 26)) return 0;
+	if (!G->pure || G->n_vtx == 0 || G->total_len > (1ULL << 26)) return 0;
 	uint32_t words = 1024;
 	while (words < G->total_len) words <<= 1;
 	if (words <= (1u << 20)) words <<= 1; // half a string per word where that stays small
