@@ -86,10 +86,11 @@ constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few 
 constexpr int32_t kPruneLag = 10;
 
 // The filter's build: every string of K = bloom_k bases that a walk of the graph spells, from
-// every position. One warp per vertex, one start per lane; walks branch through a stack (fewer than
-// K levels, as each vertex gives at least one base). A walk that dead-ends after K - 1 bases
-// enters all four extensions, so that a string of K - 1 bases may be looked up by extending it. A
-// start with more than kBloomLeaves walks sets *many, and the graph gets no filter.
+// every position, one start per thread (its vertex by binary search, so that a long vertex is as
+// many threads as it has bases); walks branch through a stack (fewer than K levels, as each vertex
+// gives at least one base). A walk that dead-ends after K - 1 bases enters all four extensions, so
+// that a string of K - 1 bases may be looked up by extending it. A start with more than kBloomLeaves
+// walks sets *many, the graph gets no filter, and threads that start later have nothing to do.
 constexpr int32_t kBloomLeaves = 1024;
 __device__ __forceinline__ void bloom_put(unsigned long long *bloom, uint32_t mask, uint32_t x)
 {
@@ -99,45 +100,47 @@ __device__ __forceinline__ void bloom_put(unsigned long long *bloom, uint32_t ma
 __global__ void __launch_bounds__(256) k_bloom(const __grid_constant__ DevGraph g, unsigned long long *bloom,
                                                int32_t *many)
 {
-	const int lane = threadIdx.x & 31;
+	const uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+	if (p0 >= g.total_len || *(volatile const int32_t *)many) return;
 	const int32_t K = g.bloom_k;
 	const uint32_t mask = g.bloom_mask;
-	const uint32_t v0 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-	if (v0 >= g.n_vtx) return;
-	const uint32_t l0 = __ldg(g.len + v0);
-	for (uint32_t o0 = lane; o0 < l0; o0 += 32) {
-		uint32_t st_x[17], st_a[17], st_e[17];
-		int32_t st_n[17];
-		int32_t depth = 0, n = 0, leaves = 0;
-		uint32_t v = v0, o = o0, x = 0;
-		for (int64_t guard = 0; guard < 64LL * kBloomLeaves; ++guard) {
-			const uint32_t vl = __ldg(g.len + v);
-			const uint64_t gb = __ldg(g.base + v);
-			for (; o < vl && n < K; ++o, ++n) {
-				const uint64_t p = gb + o;
-				x |= (uint32_t)(__ldg(g.pk + (p >> 5)) >> (2 * (p & 31)) & 3) << (2 * n);
-			}
-			bool up = false;
-			if (n == K) {
-				bloom_put(bloom, mask, x);
-				up = true;
-			} else {
-				const uint32_t a = __ldg(g.arc_off + v), e = __ldg(g.arc_off + v + 1);
-				if (a == e) {
-					if (n == K - 1)
-						for (uint32_t y = 0; y < 4; ++y) bloom_put(bloom, mask, x | y << (2 * K - 2));
-					up = true;
-				} else
-					st_x[depth] = x, st_n[depth] = n, st_a[depth] = a, st_e[depth] = e, ++depth;
-			}
-			if (up && ++leaves > kBloomLeaves) break;
-			while (depth > 0 && st_a[depth - 1] == st_e[depth - 1]) --depth;
-			if (depth == 0) break;
-			const uint2 arc = __ldg(g.arc + st_a[depth - 1]++);
-			v = arc.x, o = arc.y, x = st_x[depth - 1], n = st_n[depth - 1];
-		}
-		if (leaves > kBloomLeaves || depth > 0) *many = 1;
+	uint32_t v = 0; // the last vertex that begins at or before p0
+	for (uint32_t hi = g.n_vtx; hi - v > 1;) {
+		const uint32_t mid = v + (hi - v) / 2;
+		if (__ldg(g.base + mid) <= p0) v = mid;
+		else hi = mid;
 	}
+	uint32_t st_x[17], st_a[17], st_e[17];
+	int32_t st_n[17];
+	int32_t depth = 0, n = 0, leaves = 0;
+	uint32_t o = (uint32_t)(p0 - __ldg(g.base + v)), x = 0;
+	for (int64_t guard = 0; guard < 64LL * kBloomLeaves; ++guard) {
+		const uint32_t vl = __ldg(g.len + v);
+		const uint64_t gb = __ldg(g.base + v);
+		for (; o < vl && n < K; ++o, ++n) {
+			const uint64_t p = gb + o;
+			x |= (uint32_t)(__ldg(g.pk + (p >> 5)) >> (2 * (p & 31)) & 3) << (2 * n);
+		}
+		bool up = false;
+		if (n == K) {
+			bloom_put(bloom, mask, x);
+			up = true;
+		} else {
+			const uint32_t a = __ldg(g.arc_off + v), e = __ldg(g.arc_off + v + 1);
+			if (a == e) {
+				if (n == K - 1)
+					for (uint32_t y = 0; y < 4; ++y) bloom_put(bloom, mask, x | y << (2 * K - 2));
+				up = true;
+			} else
+				st_x[depth] = x, st_n[depth] = n, st_a[depth] = a, st_e[depth] = e, ++depth;
+		}
+		if (up && ++leaves > kBloomLeaves) break;
+		while (depth > 0 && st_a[depth - 1] == st_e[depth - 1]) --depth;
+		if (depth == 0) break;
+		const uint2 arc = __ldg(g.arc + st_a[depth - 1]++);
+		v = arc.x, o = arc.y, x = st_x[depth - 1], n = st_n[depth - 1];
+	}
+	if (leaves > kBloomLeaves || depth > 0) *many = 1;
 }
 
 // State of a read's run, in the CTA's shared memory (a CTA aligns one read at a time, with one warp

@@ -192,7 +192,7 @@ static int build_bloom(GraphDev *G)
 	if (e == cudaSuccess) e = cudaMemset(many.p, 0, 4);
 	if (e == cudaSuccess) {
 		DevGraph v = G->view();
-		k_bloom<<<(G->n_vtx + 7) / 8, 256>>>(v, (unsigned long long *)G->bloom.p, (int32_t *)many.p);
+		k_bloom<<<(unsigned)((G->total_len + 255) / 256), 256>>>(v, (unsigned long long *)G->bloom.p, (int32_t *)many.p);
 		e = cudaGetLastError();
 	}
 	if (e == cudaSuccess) e = cudaMemcpy(&h_many, many.p, 4, cudaMemcpyDeviceToHost);
