@@ -297,8 +297,8 @@ class Graph:
     def ed_batch(self, reads, v0, v1=-1, mode=MODE_AUTO, flags=0, concat=True, max_lag=0, use_graph=0,
                  warps_per_read=0):
         """Batch alignment. reads: list of bytes, or (cat, offs, lens). Returns (dist, status).
-        warps_per_read: 1, 2, 4 or 8 warps align each read of the persistent form (0 = per
-        length bucket: tuned for MODE_AUTO, else the library's default)."""
+        warps_per_read: 1, 2, 4 or 8 warps align each read of the persistent form (0 = the library's
+        rule; with a target vertex the tuned count of the read's length bucket for MODE_AUTO)."""
         if isinstance(reads, tuple):
             cat, offs, lens = reads
         else:

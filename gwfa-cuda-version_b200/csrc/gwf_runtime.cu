@@ -1070,8 +1070,8 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		return rc;
 	KParams p = base_params(E, G, B, flags);
 	p.max_lag = max_lag > 0 ? max_lag : 0;
-	// warps per read of each length bucket (persistent form): forced, tuned (GWF_MODE_AUTO), or
-	// 0: by the read's share of the batch's work (plan_classes)
+	// warps per read of each length bucket (sorted form): forced, tuned (GWF_MODE_AUTO), or 0: by the
+	// read's share of the batch's work (plan_classes)
 	int32_t nw_b[GWF_TUNE_NBUCKETS];
 	for (int b = 0; b < GWF_TUNE_NBUCKETS; ++b) {
 		int32_t nw = warps_per_read > 0 ? warps_per_read : 0;
@@ -1083,10 +1083,12 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		if (gwf_tune_lookup(E.device, B.dom_bucket, &f, &c)) mode = f, ctas_per_sm = c;
 	}
 	bool classes = false;
-	// the block form takes one count for the batch: forced, tuned for its dominant bucket, or by rule
+	// the block form: forced, or by rule (plan_blocks). Not the tuned counts: those are a bucket's, on
+	// a sample of its reads, and a count for a whole batch switches off its split by length (30,000
+	// mixed reads: 153 ms with the count tuned on 300 reads a bucket, 22 by rule)
 	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p);
 	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp 7.5 ms, 10.1 with two)
-	const int32_t nw_blocks = nw_b[B.dom_bucket] == 0 && p.max_lag > 0 ? 1 : nw_b[B.dom_bucket];
+	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 ? 1 : 0;
 	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;

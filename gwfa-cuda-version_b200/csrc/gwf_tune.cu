@@ -2,12 +2,17 @@
 //
 // The cost of a read grows with ql^2 x error, and the arena a warp needs grows with ql, so the
 // best launch shape depends on the lengths in a batch. gwf_tune times, on the caller's own reads
-// and separately for each length bucket, the persistent form with 1, 2, 4 and 8 warps per read at
-// every CTAs-per-SM count up to the occupancy limit, and the plain form, and keeps the fastest
-// per bucket in a per-device table. A batch run with mode GWF_MODE_AUTO then aligns each read
-// with the warps per read of its own bucket (one launch, read classes longest first) and takes
-// the form and CTAs per SM of the bucket that carries most of its work (sum of ql^2). The table
-// can be written to and read from a small JSON file, so a tuned setting survives the process.
+// and separately for each length bucket, the persistent form at every CTAs-per-SM count up to the
+// occupancy limit and with 1, 2, 4 and 8 warps per read, and the plain form, and keeps the fastest
+// per bucket in a per-device table. A batch run with mode GWF_MODE_AUTO then takes the form and CTAs
+// per SM of the bucket that carries most of its work (sum of ql^2). In the sorted form (target
+// vertices, mixed overlaps) each read gets the warps of its own bucket (one launch, read classes
+// longest first); in the block form the warps per read stay with the rule of the whole batch, so
+// that form is timed with it, and with fewer CTAs per SM only where the sample has more reads than
+// the device has warp slots, and where they gain 2%: on a smaller sample fewer are as good or better,
+// and a larger batch needs them all (30,000 mixed reads after tuning on 300 a bucket: 24.8 ms with the
+// one CTA that won there, 22.2 untuned). The table can be written to and read from a small JSON file,
+// so a tuned setting survives the process.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -150,26 +155,44 @@ extern "C" int gwf_tune(const gwf_graph_t *g, int32_t n, const char *seqs, const
 			int32_t form, cps, nw;
 		};
 		std::vector<Cand> cand;
+		const bool blocks = v1 < 0 && gwf_blocks_graph(G->view());
+		const int full = E->persistent_ctas_per_sm;
+		for (int c = full; blocks && c >= 1 && (c == full || k > 8 * full * E->sm_count); --c)
+			cand.push_back({GWF_MODE_PERSISTENT, c, 0});
 		for (int nw : {1, 2, 4, 8}) {
+			if (blocks) break;
 			const int occ = nw == 1 ? E->persistent_ctas_per_sm : E->classes_ctas_per_sm;
 			for (int c = 1; c <= occ; ++c) cand.push_back({GWF_MODE_PERSISTENT, c, nw});
 		}
 		cand.push_back({GWF_MODE_PLAIN, 0, 1});
-		for (const Cand &fc : cand) {
+		auto time_shape = [&](const Cand &fc, float *rps) -> int {
 			float best_ms = 0;
 			for (int rep = 0; rep < 3; ++rep) { // one warm-up, then the faster of two timed runs
 				float ms = 0;
-				if ((rc = gwf_batch_exec(*E, *G, B, fc.form, 0, fc.cps, &ms, nullptr, 0, 0, fc.nw))) {
-					B.release();
-					return rc;
-				}
+				const int e = gwf_batch_exec(*E, *G, B, fc.form, 0, fc.cps, &ms, nullptr, 0, 0, fc.nw);
+				if (e) return e;
 				if (rep == 1 || (rep == 2 && ms < best_ms)) best_ms = ms;
 			}
-			const float rps = best_ms > 0 ? (float)k / (best_ms / 1000.0f) : 0.0f;
-			if (!best.valid || rps > best.rps)
+			*rps = best_ms > 0 ? (float)k / (best_ms / 1000.0f) : 0.0f;
+			return 0;
+		};
+		for (const Cand &fc : cand) {
+			float rps = 0;
+			if ((rc = time_shape(fc, &rps))) break;
+			if (!best.valid || rps > best.rps * (blocks ? 1.02f : 1.0f))
 				best.valid = 1, best.form = fc.form, best.cps = fc.cps, best.nw = fc.nw, best.rps = rps;
 		}
+		if (!rc && best.nw == 0) { // the block form: its fastest count, for runs that take the sorted form
+			float top = 0;
+			for (int nw : {1, 2, 4, 8}) {
+				float rps = 0;
+				if ((rc = time_shape({GWF_MODE_PERSISTENT, best.cps, nw}, &rps))) break;
+				if (rps > top) top = rps, best.nw = nw;
+			}
+			if (best.nw == 0) best.nw = 1;
+		}
 		B.release();
+		if (rc) return rc;
 		std::lock_guard<std::mutex> lk(g_tune_mu);
 		g_tune[dev][b] = best;
 	}

@@ -83,14 +83,13 @@ typedef struct {
 	int32_t flags;       /* GWF_F_* */
 	int32_t device;      /* CUDA device ordinal (-1 = current) */
 	int32_t warps_per_read; /* persistent form: warps that align one read together (1, 2, 4 or 8).
-	                           0 = the gwf_tune value of the length bucket that holds most of the
-	                           batch's work for GWF_MODE_AUTO, else by rule: in a batch of mixed
-	                           lengths the longest reads get 8 or 16 warps, the more of them the
-	                           fewer reads there are per warp slot; reads of one length get as
-	                           many (up to 16) as keep all of them running at once; the others,
-	                           and runs with lag pruning, one. With a target vertex (v1 >= 0), or
-	                           arcs into one vertex of different overlaps, per read: its bucket's
-	                           tuned value, or 2, 4 or 8 warps by its share of the batch's work
+	                           0 = by rule: in a batch of mixed lengths the longest reads get 8 or
+	                           16 warps, the more of them the fewer reads there are per warp slot;
+	                           reads of one length get as many (up to 16) as keep all of them
+	                           running at once; the others, and runs with lag pruning, one. With a
+	                           target vertex (v1 >= 0), or arcs into one vertex of different
+	                           overlaps, per read: the gwf_tune value of its length bucket for
+	                           GWF_MODE_AUTO, else 2, 4 or 8 warps by its share of the batch's work
 	                           (cost ql^2) and its arena size.
 	                           The plain form uses one warp per read. */
 	int32_t ctas_per_sm;   /* persistent grid; 0 = the autotuned value for GWF_MODE_AUTO (see
@@ -218,13 +217,14 @@ int gwf_ed_batch_noalloc(const gwf_graph_t *g, int32_t n, int32_t max_ql, const 
                          void *stream);
 
 /* ---- autotuner (no reference counterpart) ----
- * Times the persistent form with 1, 2, 4 and 8 warps per read at 1..(occupancy limit) CTAs per
- * SM, and the plain form, on the given reads, separately for each read-length bucket (ql < 1500,
+ * Times the persistent form at 1..(occupancy limit) CTAs per SM, with 1, 2, 4 and 8 warps per read,
+ * and the plain form, on the given reads, separately for each read-length bucket (ql < 1500,
  * < 3000, < 6000, < 12000, longer; at most max_reads_per_bucket evenly spread reads each, 0 =
  * 8192), and keeps the fastest shape per bucket for the graph's device. Batch calls with mode
- * GWF_MODE_AUTO then take the warps per read (warps_per_read = 0), form and CTAs per SM
- * (ctas_per_sm = 0) of the bucket holding most of the batch's work (sum of ql^2); with a target
- * vertex, or arcs into one vertex of different overlaps, each read has its own bucket's warps. json_path != NULL also writes the table as JSON; gwf_tune_load
+ * GWF_MODE_AUTO then take the form and CTAs per SM (ctas_per_sm = 0) of the bucket holding most of
+ * the batch's work (sum of ql^2); with a target vertex, or arcs into one vertex of different overlaps,
+ * each read has its own bucket's warps (tune with such calls for them), and in the other calls the
+ * warps per read stay with the rule. json_path != NULL also writes the table as JSON; gwf_tune_load
  * reads it back (device -1 = current). */
 #define GWF_TUNE_NBUCKETS 5
 int gwf_tune(const gwf_graph_t *g, int32_t n, const char *seqs, const int64_t *offs, const int32_t *ql,

@@ -36,3 +36,25 @@ def test_unlike_reads_stay_in_the_block_form(G, O, n):
     pick = np.arange(0, n, 50)
     ref, _, _ = og.ed_batch(cat, offs[pick], lens[pick], np.zeros(len(pick), np.int32), stats=False)
     assert np.array_equal(d[pick], ref)
+
+
+def test_tuned_counts_leave_the_split_by_length(G, tmp_path):
+    """A table with eight warps for every bucket: GWF_MODE_AUTO still gives groups of warps to the longest
+    reads only (two kernels side by side), as an untuned run does."""
+    w = G.load_workload("config3", n=1500)
+    w["graph"].index()
+    b = G.ResidentBatch(w["graph"], w["cat"], w["offs"], w["lens"], w["v0"], mode=G.MODE_AUTO)
+    path = tmp_path / "tune.json"
+    path.write_text('{"buckets": [' + ",".join(
+        '\n {"bucket": %d, "ql_max": 0, "form": "persistent", "ctas_per_sm": 4, "reads_per_s": 1.0, '
+        '"warps_per_read": 8}' % k for k in range(5)) + "]}")
+    b.run()
+    d, launches = b.results()[0], b.launches()
+    assert launches == 3  # packing, one warp per read, several warps per read
+    try:
+        G.tune_load(str(path))
+        b.run()
+        assert b.launches() == launches and np.array_equal(b.results()[0], d)
+    finally:
+        G.tune_clear()
+        b.close()
