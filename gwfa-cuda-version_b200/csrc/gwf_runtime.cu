@@ -1000,7 +1000,7 @@ static int enqueue_classes(Engine &E, KParams p, const ClassLaunch &cl)
 // persistent kernel, copy the overflow count to the host. Captured once per batch contents and
 // launch shape, replayed on every run.
 static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_per_sm, bool classes, bool blocks,
-                               int32_t nw)
+                               int32_t nw, int *launches)
 {
 	PersistPlan pl;
 	BlocksPlan bp;
@@ -1052,6 +1052,7 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 		memcpy(B.gkey, key, sizeof key);
 	}
 	CK(cudaGraphLaunch(B.gexec, E.stream));
+	*launches += 2 + (blocks && bp.n_mw > 0 && bp.n_mw < B.n); // packing and the batch's kernels
 	return 0;
 }
 
@@ -1100,8 +1101,8 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	bool count_copied = false;
 	if (ms) CK(cudaEventRecord(E.ev0, E.stream));
 	if (use_graph && mode != GWF_MODE_PLAIN) {
-		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks, nw_blocks))) return rc;
-		launches += 2;
+		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks, nw_blocks, &launches)))
+			return rc;
 		count_copied = true;
 	} else {
 		if ((rc = enqueue_pack(E, B))) return rc;

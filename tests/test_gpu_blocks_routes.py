@@ -58,3 +58,14 @@ def test_tuned_counts_leave_the_split_by_length(G, tmp_path):
     finally:
         G.tune_clear()
         b.close()
+
+
+def test_launches_of_a_replayed_graph(G):
+    """The launch count of a replay is that of the kernels in it: packing and both batch kernels."""
+    w = G.load_workload("config3", n=1500)
+    w["graph"].index()
+    b = G.ResidentBatch(w["graph"], w["cat"], w["offs"], w["lens"], w["v0"], mode=G.MODE_PERSISTENT)
+    for use_graph, nw, want in ((0, 0, 3), (1, 0, 3), (1, 0, 3), (1, 1, 2), (1, 8, 2)):
+        b.run(use_graph=use_graph, warps_per_read=nw)
+        assert b.launches() == want
+    b.close()
