@@ -79,7 +79,6 @@ __host__ __device__ inline uint2 bloom_bits(uint32_t x)
 }
 
 #ifndef GWF_KERNELS_DECL_ONLY
-constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few steps cost less than a bound
 // Lag of the run that gives an upper bound. A larger one costs more states (24: 2,000 x 10 kbp at 10%
 // 97.6 -> 102.0 ms), a smaller one loses the read's path sooner, and the bound with it (6: 4,000 x
 // 10 kbp at 5% on the dense graph 29.7 -> 238 ms, 8: 29.7).

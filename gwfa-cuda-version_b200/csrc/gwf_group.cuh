@@ -1049,7 +1049,7 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constan
 		const int64_t qb = srv_qbytes(ql);
 		KParams lp;
 		memset(&lp, 0, sizeof lp);
-		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli);
+		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli, bw_free(p.g.bloom, p.max_lag));
 		const int64_t need = blocks ? lp.bw.total : ws_layout(caps_for(ql, level, p.dens_milli)).total;
 		if (qb + need <= abytes) { // the host sized it so; else report capacity
 			lp.g = p.g;

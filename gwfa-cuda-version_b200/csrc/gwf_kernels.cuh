@@ -12,17 +12,26 @@ struct BwLay {
 	int64_t total;
 };
 
+constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few steps cost less than a bound
+constexpr int32_t kFreeLag = 300;    // the caller's lag pruning from here on keeps many blocks
+
+// Do reads run without a bound (free), and without a small lag of the caller's?
+__host__ __device__ inline bool bw_free(bool bloom, int32_t max_lag) { return max_lag > 0 ? max_lag >= kFreeLag : !bloom; }
+
 // Arena for reads of up to ql bases at retry class level on a graph of dens_milli vertices per 1000
-// bases. Pruned runs of 10 kbp reads at 5% on the dense benchmark graph make ~1,000 blocks (34,000
-// unpruned), 20 kbp reads at 10% ~33,000, 1 kbp reads on the sparse graph ~50, random 1 kbp reads
-// ~400. Class 0 (serving's first, where arenas share a budget) leaves out what reads unlike the
-// graph need, class 1 holds it (the first of a batch), class 2 is 8 times as large.
-__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli)
+// bases. Blocks that reads make, in units of u = dens_milli ql^2 / 10^6 (64 reads each of 1, 3 and 10
+// kbp, graphs of 5 to 550 vertices per 1000 bases): with a bound 0.4 to 5.7 at 2 to 10% errors, the
+// upper end short reads, which the other terms hold; free 3 to 26, or lag 2000 up to 17, 600 up to 7;
+// reads unlike the graph 90 to 110. Class 0 (serving's first, where arenas share a budget) leaves out
+// the last, class 1 (the first of a batch) holds short ones of them, class 2 all (reads of 3 kbp on
+// the dense benchmark graph that met no such class ended in the sorted form).
+__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli, bool free)
 {
-	const int64_t q = ql < 64 ? 64 : ql;
-	int64_t nb = 128 + (int64_t)dens_milli * q * q / 400000 + (int64_t)dens_milli * q * 8 / 1000;
+	const int64_t q = ql < 64 ? 64 : ql, u10 = (int64_t)dens_milli * q * q / 100000;
+	int64_t nb = 128 + (int64_t)dens_milli * q * 8 / 1000 + u10 / 4;
 	if (level > 0) nb += q / 2;
-	if (level > 1) nb *= 8;
+	if (level > 1) nb = 8 * nb + 13 * u10;
+	else if (free || q < kPruneMinQl) nb += 5 * u10 / 2;
 	if (nb > (1 << 22)) nb = 1 << 22;
 	BwLay o;
 	o.nb = (int32_t)nb, o.hs = pow2ceil_i(2 * o.nb);

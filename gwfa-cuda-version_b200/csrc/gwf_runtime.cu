@@ -694,7 +694,7 @@ static const double kMwShare = 0.2, kMwUniform = 0.67;
 static const int32_t kMwMinQl = 1500; // shorter reads have no more than a few blocks at a time
 
 static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
-                       int32_t nw, int32_t dens_milli, BlocksPlan *pl)
+                       int32_t nw, const KParams &p, BlocksPlan *pl)
 {
 	const int64_t slots = (int64_t)E.sm_count * warps_per_sm;
 	int32_t cap = ql_cap;
@@ -720,7 +720,8 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 		if (from == 0) pl->mw = all;
 		else if (pl->n_mw) pl->mw = 16LL * pl->n_mw <= slots ? 16 : 8;
 	}
-	pl->lay_mw = bw_layout(ql_cap, level, dens_milli), pl->lay = bw_layout(cap, level, dens_milli);
+	const bool free = bw_free(p.g.bloom, p.max_lag);
+	pl->lay_mw = bw_layout(ql_cap, level, p.dens_milli, free), pl->lay = bw_layout(cap, level, p.dens_milli, free);
 	const int64_t budget = std::max<int64_t>(E.mem_budget, (int64_t)E.ws.cap);
 	const int32_t n_one = n_order - pl->n_mw;
 	if (pl->n_mw) pl->ctas_mw = std::min<int64_t>(pl->n_mw, std::max<int64_t>(1, slots / pl->mw));
@@ -1008,7 +1009,7 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 	int rc;
 	const bool defer = blocks && defer_unlike(E, B.n, ctas_per_sm, nw);
 	if (blocks) {
-		if ((rc = plan_blocks(E, &B, B.n, B.max_ql, 1, ctas_per_sm, nw, p.dens_milli, &bp))) return rc;
+		if ((rc = plan_blocks(E, &B, B.n, B.max_ql, 1, ctas_per_sm, nw, p, &bp))) return rc;
 		pl.ctas = (int)bp.ctas, pl.slot = bp.lay.total;
 	} else if (classes) {
 		if ((rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl))) return rc;
@@ -1111,7 +1112,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		if (mode == GWF_MODE_PLAIN) rc = launch_plain(E, p, B, &launches);
 		else if (blocks) {
 			BlocksPlan pl;
-			if (!(rc = plan_blocks(E, &B, B.n, B.max_ql, 1, warps_per_sm, nw_blocks, p.dens_milli, &pl)) &&
+			if (!(rc = plan_blocks(E, &B, B.n, B.max_ql, 1, warps_per_sm, nw_blocks, p, &pl)) &&
 			    !(rc = enqueue_blocks(E, p, pl, B.d_order, B.n, defer_unlike(E, B.n, warps_per_sm, nw_blocks))))
 				launches += 1 + (pl.n_mw > 0 && pl.n_mw < B.n);
 		} else if (classes) {
@@ -1153,7 +1154,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 			BlocksPlan pl; // as many warps per read as keep all reads running at once
 			int32_t nw = 16;
 			while (nw > 1 && (int64_t)nw * nr > (int64_t)E.sm_count * warps_per_sm) nw >>= 1;
-			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p.dens_milli, &pl)) ||
+			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p, &pl)) ||
 			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr, false)))
 				return rc;
 			++launches;

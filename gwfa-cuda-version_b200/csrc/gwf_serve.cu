@@ -181,7 +181,8 @@ int32_t *busy_dev(gwf_srv_s *S) { return (int32_t *)((char *)S->ctl.p + 256); }
 int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, bool blocks, int32_t level)
 {
 	const int32_t dens = S->G->dens_milli;
-	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens).total : gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
+	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens, gwfb::bw_free(S->G->bloom.p, S->max_lag)).total
+	                          : gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
 	const int64_t bytes = gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws);
 	return bytes <= S->pool.cap() ? bytes : -1;
 }

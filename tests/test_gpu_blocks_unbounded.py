@@ -1,0 +1,71 @@
+"""The block form where no bound prunes it: graphs without a filter (a byte other than A/C/G/T, too many
+walks), reads unlike the graph, the caller's lag pruning with a large lag. The oracle gives every
+distance (tolerance 0); launch counts show that arenas are large enough at the first try."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(G, n, site=50, lower=False, seed=31):
+    """A seeded graph of n bases with a variant every `site` bases; lower: one lower-case base, so that it
+    has no filter and every compare takes bytes."""
+    sg = G.SynthGraph(n, site, 0.7, 4, 0, 0, 0, seed=seed)
+    text = sg.gfa
+    if lower:
+        i = text.index(b"\tA") + 1
+        text = text[:i] + b"a" + text[i + 1:]
+    g = G.Graph.from_gfa_text(text)
+    g.index()
+    s2v = g.vertex_of_segment()
+    return sg, g, s2v
+
+
+def _reads(sg, s2v, *a, **kw):
+    r = sg.reads(*a, **kw)
+    return r["cat"], r["offs"], r["lens"], np.array([s2v[int(o)] for o in r["origin_seg"]], dtype=np.int32)
+
+
+def _revcomp(cat, offs, lens):
+    t = np.arange(256, dtype=np.uint8)
+    for x, y in (b"AT", b"CG", b"GC", b"TA"):
+        t[x] = y
+    out = cat.copy()
+    for o, n in zip(offs, lens):
+        out[o:o + n] = t[cat[o:o + n][::-1]]
+    return out
+
+
+@pytest.mark.parametrize("site", [12, 50, 500])
+def test_graphs_without_a_filter(G, O, site):
+    """Reads of 0.6 to 6 kbp at 2 to 10%: the first arena holds them, with one warp and with eight."""
+    sg, g, s2v = _dense(G, 60_000, site, lower=True)
+    cat, offs, lens, v0 = _reads(sg, s2v, 24, 2, 600, 6000, 600, 6000, 0.02, 0.10, seed=site)
+    ref, _, _ = O.OracleGraph.from_graph(g).ed_batch(cat, offs, lens, v0, stats=False)
+    b = G.ResidentBatch(g, cat, offs, lens, v0, mode=G.MODE_PERSISTENT)
+    for nw in (1, 8):
+        b.run(warps_per_read=nw)
+        d, st = b.results()
+        assert (st == 0).all() and np.array_equal(d, ref)
+        assert b.launches() == 2  # packing and the batch
+    b.run()
+    assert np.array_equal(b.results()[0], ref)
+    b.close()
+
+
+@pytest.mark.parametrize("site", [12, 50])
+def test_reads_unlike_a_dense_graph(G, O, site):
+    """Reverse complements, left to the retry launch: its arena holds them, the sorted form is not
+    reached."""
+    sg, g, s2v = _dense(G, 60_000, site)
+    cat, offs, lens, v0 = _reads(sg, s2v, 12, 2, 700, 3000, 700, 3000, 0.02, 0.10, seed=site)
+    cat = _revcomp(cat, offs, lens)
+    ref, _, _ = O.OracleGraph.from_graph(g).ed_batch(cat, offs, lens, v0, stats=False)
+    b = G.ResidentBatch(g, cat, offs, lens, v0, mode=G.MODE_PERSISTENT)
+    b.run()
+    d, st = b.results()
+    assert (st == 0).all() and np.array_equal(d, ref)
+    assert b.launches() <= 4  # packing, one warp and several warps per read, the retry
+    b.run(warps_per_read=1)
+    assert np.array_equal(b.results()[0], ref) and b.launches() <= 3
+    b.close()
