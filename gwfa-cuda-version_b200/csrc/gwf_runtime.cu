@@ -1089,8 +1089,12 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	// a sample of its reads, and a count for a whole batch switches off its split by length (30,000
 	// mixed reads: 153 ms with the count tuned on 300 reads a bucket, 22 by rule)
 	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p);
-	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp 7.5 ms, 10.1 with two)
-	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 ? 1 : 0;
+	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp at lag 20 7.5 ms, 10.1 with two.
+	// From kWideLag on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the dense graph
+	// at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 / 62; 200 reads of 0.5-20 kbp at lag 60
+	// 21 / 21, 200 42 / 32, 2000 470 / 96)
+	const int32_t kWideLag = 200;
+	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 && p.max_lag < kWideLag ? 1 : 0;
 	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;

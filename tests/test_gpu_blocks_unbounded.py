@@ -1,6 +1,8 @@
 """The block form where no bound prunes it: graphs without a filter (a byte other than A/C/G/T, too many
 walks), reads unlike the graph, the caller's lag pruning with a large lag. The oracle gives every
 distance (tolerance 0); launch counts show that arenas are large enough at the first try."""
+import time
+
 import numpy as np
 import pytest
 
@@ -69,3 +71,23 @@ def test_reads_unlike_a_dense_graph(G, O, site):
     b.run(warps_per_read=1)
     assert np.array_equal(b.results()[0], ref) and b.launches() <= 3
     b.close()
+
+
+def test_large_lag_gets_warps_by_rule(G):
+    """A lag of 2,000 on a dense graph prunes little: few long reads get groups of warps as they do
+    without it (the time of eight warps each, with a factor to spare; with one it was several times)."""
+    sg, g, s2v = _dense(G, 200_000, 20)
+    cat, offs, lens, v0 = _reads(sg, s2v, 60, 0, 6000, 0, 6000, 6000, 0.08, 0.08, seed=3)
+
+    def best(nw):
+        t = []
+        for _ in range(4):
+            t0 = time.perf_counter()
+            d, st = g.ed_batch((cat, offs, lens), v0, mode=G.MODE_PERSISTENT, flags=G.GWF_F_MAX_LAG, max_lag=2000,
+                               warps_per_read=nw)
+            t.append(time.perf_counter() - t0)
+            assert (st == 0).all()
+        return min(t), d
+
+    (t8, d8), (t0, d0) = best(8), best(0)
+    assert np.array_equal(d0, d8) and t0 < 1.6 * t8
