@@ -1053,7 +1053,7 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 		if (!lag && p.defer) { // such a read makes thousands of states per step: left to a group of warps
 			if (lead) {
 				p.dist[r] = -1, p.status[r] = ST_CAPACITY;
-				p.retry_list[atomicAdd(p.retry_n, 1)] = r;
+				if (p.retry_list) p.retry_list[atomicAdd(p.retry_n, 1)] = r;
 			}
 			return;
 		}

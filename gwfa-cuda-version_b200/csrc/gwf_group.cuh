@@ -958,7 +958,10 @@ __device__ __forceinline__ void run_class(const KParams &p, const ClassParams &c
 // and no CTA busy (any CTA does after max_idle_ns), and every CTA leaves when it sees the mark. A
 // CTA counts itself busy before it tries to claim, so the leader never closes under a claim in
 // progress. The host relaunches the kernel when positions are queued and it has ended.
-constexpr int32_t kServeMwMinQl = 1500; // shorter reads have few blocks at a time: one warp, without barriers
+// Shorter reads with a bound, or a small lag, have few blocks at a time: one warp, without barriers;
+// without a bound, those below one unit of bw_layout. Reads unlike the graph are given up in the first
+// arena class, which does not hold them, before a step is made; the group aligns them in a larger one.
+constexpr int32_t kServeMwMinQl = 1500;
 template <int NW>
 __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constant__ SrvParams p)
 {
@@ -1049,7 +1052,7 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constan
 		const int64_t qb = srv_qbytes(ql);
 		KParams lp;
 		memset(&lp, 0, sizeof lp);
-		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli, bw_free(p.g.bloom, p.max_lag));
+		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli, bw_open(p.g.bloom, ql, p.max_lag));
 		const int64_t need = blocks ? lp.bw.total : ws_layout(caps_for(ql, level, p.dens_milli)).total;
 		if (qb + need <= abytes) { // the host sized it so; else report capacity
 			lp.g = p.g;
@@ -1068,9 +1071,13 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constan
 			lp.dist = &hdr->dist;
 			lp.status = &hdr->status;
 			if (blocks) {
+				lp.defer = level == 0;
 				bw_init(lp.g, lp.bw, ab + qb);
-				if (NW > 1 && ql >= kServeMwMinQl) align_read_blocks<(NW > 1)>(lp, 0, ab + qb);
-				else if (threadIdx.x < 32) align_read_blocks<false>(lp, 0, ab + qb);
+				const bool open = bw_open(p.g.bloom, ql, p.max_lag) && bw_u10(ql, p.dens_milli) >= 10;
+				if (NW > 1 && (level > 0 || ql >= kServeMwMinQl || open))
+					align_read_blocks<(NW > 1)>(lp, 0, ab + qb);
+				else if (threadIdx.x < 32)
+					align_read_blocks<false>(lp, 0, ab + qb);
 			} else if constexpr (NW == 1)
 				align_read(lp, 0, ab + qb, ql, level);
 			else if (p.max_lag > 0)

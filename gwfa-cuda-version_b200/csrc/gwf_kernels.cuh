@@ -13,25 +13,39 @@ struct BwLay {
 };
 
 constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few steps cost less than a bound
-constexpr int32_t kFreeLag = 300;    // the caller's lag pruning from here on keeps many blocks
+constexpr int32_t kFreeLag = 300;    // the caller's lag pruning from here on keeps many states
 
-// Do reads run without a bound (free), and without a small lag of the caller's?
-__host__ __device__ inline bool bw_free(bool bloom, int32_t max_lag) { return max_lag > 0 ? max_lag >= kFreeLag : !bloom; }
+// Does a read run without a bound, and without a small lag of the caller's?
+__host__ __device__ inline bool bw_open(bool bloom, int32_t ql, int32_t max_lag)
+{
+	return max_lag > 0 ? max_lag >= kFreeLag : !bloom || ql < kPruneMinQl;
+}
+
+// A read's size in tenths of the unit u of bw_layout
+__host__ __device__ inline int64_t bw_u10(int32_t ql, int32_t dens_milli) { return (int64_t)dens_milli * ql * ql / 100000; }
+
+// Groups of warps pay for open reads (bw_open) from shorter lengths on, and on graphs with fewer than
+// kSparse vertices per 1000 bases, whose long vertices make long lists of diagonals, the sorted form's
+// groups are the faster ones below kSparseU10. Up to 200 reads each, ms, sorted form / block form with
+// one warp / with eight: sparse graph (5 vertices per 1000 bases), 1.4 kbp 1.5 / 1.75 / 1.5, 3 kbp 5.0 /
+// - / 4.5, 500 bases 0.18 / 0.20 / 0.26 and their reverse complements 1.2 / 1.9 / 1.5; dense one (49),
+// 500 bases 1.1 / 1.5 / 1.0, 1.4 kbp 4.8 / 8.7 / 3.6.
+constexpr int32_t kSparse = 20, kSparseU10 = 120;
 
 // Arena for reads of up to ql bases at retry class level on a graph of dens_milli vertices per 1000
 // bases. Blocks that reads make, in units of u = dens_milli ql^2 / 10^6 (64 reads each of 1, 3 and 10
 // kbp, graphs of 5 to 550 vertices per 1000 bases): with a bound 0.4 to 5.7 at 2 to 10% errors, the
-// upper end short reads, which the other terms hold; free 3 to 26, or lag 2000 up to 17, 600 up to 7;
+// upper end short reads, which the other terms hold; open 3 to 26, or lag 2000 up to 17, 600 up to 7;
 // reads unlike the graph 90 to 110. Class 0 (serving's first, where arenas share a budget) leaves out
 // the last, class 1 (the first of a batch) holds short ones of them, class 2 all (reads of 3 kbp on
 // the dense benchmark graph that met no such class ended in the sorted form).
-__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli, bool free)
+__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli, bool open)
 {
-	const int64_t q = ql < 64 ? 64 : ql, u10 = (int64_t)dens_milli * q * q / 100000;
+	const int64_t q = ql < 64 ? 64 : ql, u10 = bw_u10((int32_t)q, dens_milli);
 	int64_t nb = 128 + (int64_t)dens_milli * q * 8 / 1000 + u10 / 4;
 	if (level > 0) nb += q / 2;
 	if (level > 1) nb = 8 * nb + 13 * u10;
-	else if (free || q < kPruneMinQl) nb += 5 * u10 / 2;
+	else if (open) nb += 5 * u10 / 2;
 	if (nb > (1 << 22)) nb = 1 << 22;
 	BwLay o;
 	o.nb = (int32_t)nb, o.hs = pow2ceil_i(2 * o.nb);
@@ -77,7 +91,7 @@ struct KParams {
 	int32_t *path_arc;      // arc index into path_v[j] (-1 for j = 0)
 	int32_t max_nv;
 	BwLay bw;               // block form: layout of a CTA's arena
-	int32_t defer;          // block form, one warp: reads unlike the graph go to the retry list
+	int32_t defer;          // block form, one warp: reads unlike the graph are given up (GWF_E_CAPACITY)
 };
 
 // ---- serving: one resident kernel, warps pull single reads from a device queue

@@ -720,8 +720,8 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 		if (from == 0) pl->mw = all;
 		else if (pl->n_mw) pl->mw = 16LL * pl->n_mw <= slots ? 16 : 8;
 	}
-	const bool free = bw_free(p.g.bloom, p.max_lag);
-	pl->lay_mw = bw_layout(ql_cap, level, p.dens_milli, free), pl->lay = bw_layout(cap, level, p.dens_milli, free);
+	pl->lay_mw = bw_layout(ql_cap, level, p.dens_milli, bw_open(p.g.bloom, ql_cap, p.max_lag));
+	pl->lay = bw_layout(cap, level, p.dens_milli, bw_open(p.g.bloom, cap, p.max_lag));
 	const int64_t budget = std::max<int64_t>(E.mem_budget, (int64_t)E.ws.cap);
 	const int32_t n_one = n_order - pl->n_mw;
 	if (pl->n_mw) pl->ctas_mw = std::min<int64_t>(pl->n_mw, std::max<int64_t>(1, slots / pl->mw));

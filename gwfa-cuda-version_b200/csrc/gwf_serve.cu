@@ -45,8 +45,7 @@ double now_s()
 	return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
 }
 
-constexpr int kBlockLevels = 3;      // arena classes of the block form (bw_layout)
-constexpr int kMaxLevel = 3;         // the sorted form's are 1x, 4x, 16x, 64x
+constexpr int kMaxLevel = 3;         // arena classes of the sorted form: 1x, 4x, 16x, 64x
 constexpr int64_t kIdleNs = 5000000; // 5 ms
 constexpr int64_t kMaxIdleNs = 120LL * 1000000000LL;
 
@@ -181,28 +180,35 @@ int32_t *busy_dev(gwf_srv_s *S) { return (int32_t *)((char *)S->ctl.p + 256); }
 int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, bool blocks, int32_t level)
 {
 	const int32_t dens = S->G->dens_milli;
-	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens, gwfb::bw_free(S->G->bloom.p, S->max_lag)).total
+	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens, gwfb::bw_open(S->G->bloom.p, ql, S->max_lag)).total
 	                          : gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
 	const int64_t bytes = gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws);
 	return bytes <= S->pool.cap() ? bytes : -1;
 }
 
-// Arena classes of a read, in turn. Reads without a target vertex take the block form's, as long as
-// they fit the budget, then the sorted form's from 4x on (as the batch path), or from 1x where 4x does
+// Arena classes of a read, in turn. Reads without a target vertex, but for short ones without a bound
+// on sparse graphs, take the block form's 0 and 2 (1 where 2 does not fit the budget), as long as they
+// fit, then the sorted form's from 4x on (as the batch path), or from 1x where 4x does
 // not fit; the others take the sorted form's. A read whose first sorted arena does not fit is not
 // served. Both return false when no class is left.
 bool first_class(const gwf_srv_s *S, Slot &sl)
 {
 	const int32_t ql = sl.r->ql[(size_t)sl.read];
+	const int32_t dens = S->G->dens_milli;
 	sl.level = 0;
-	sl.blocks = S->blocks && sl.r->v1 < 0 && arena_bytes(S, ql, true, 0) >= 0;
+	sl.blocks = S->blocks && sl.r->v1 < 0 && arena_bytes(S, ql, true, 0) >= 0 &&
+	            !(dens < gwfb::kSparse && gwfb::bw_open(S->G->bloom.p, ql, S->max_lag) &&
+	              gwfb::bw_u10(ql, dens) < gwfb::kSparseU10);
 	return arena_bytes(S, ql, false, 0) >= 0;
 }
 bool next_class(const gwf_srv_s *S, Slot &sl)
 {
 	const int32_t ql = sl.r->ql[(size_t)sl.read];
 	if (sl.blocks) {
-		if (++sl.level < kBlockLevels && arena_bytes(S, ql, true, sl.level) >= 0) return true;
+		if (sl.level == 0) { // most often a read unlike the graph
+			sl.level = arena_bytes(S, ql, true, 2) >= 0 ? 2 : 1;
+			if (arena_bytes(S, ql, true, sl.level) >= 0) return true;
+		}
 		sl.blocks = false, sl.level = arena_bytes(S, ql, false, 1) >= 0 ? 1 : 0;
 		return true;
 	}

@@ -45,3 +45,28 @@ def test_sorted_form_where_the_block_arena_does_not_fit(G):
     solo, _ = g.ed_batch(reads, v0)
     assert (st == 0).all() and np.array_equal(d, solo)
     assert stats["retries"] == 0
+
+
+@pytest.mark.parametrize("lower", [False, True])
+def test_unlike_reads_and_missing_filters_cost_one_retry_at_most(G, lower):
+    """Both strands of reads on a dense graph: the reverse complements leave the first arena class before
+    a step is made, and the class after it holds them. With one lower-case base the graph has no filter
+    that could tell them apart; they still go straight to the class that holds them."""
+    sg = G.SynthGraph(60_000, 50, 0.7, 4, 0, 0, 0, seed=41)
+    text = sg.gfa
+    if lower:
+        i = text.index(b"\tA") + 1
+        text = text[:i] + b"a" + text[i + 1:]
+    g = G.Graph.from_gfa_text(text)
+    g.index()
+    s2v = g.vertex_of_segment()
+    r = sg.reads(16, 2, 300, 2500, 300, 2500, 0.01, 0.1, seed=5)
+    v0 = np.array([s2v[int(o)] for o in r["origin_seg"]], dtype=np.int32)
+    reads = (r["cat"], r["offs"], r["lens"])
+    d, st, stats = _serve(G, g, reads, v0, flags=G.GWF_F_BOTH_STRANDS, arena_budget_bytes=2 << 30)
+    solo, st2, _ = g.ed_strand(reads, v0)
+    assert np.array_equal(d, solo) and np.array_equal(st, st2) and (st == 0).all()
+    assert stats["retries"] <= 16
+    d, st, stats = _serve(G, g, reads, v0, arena_budget_bytes=2 << 30)
+    assert (st == 0).all() and np.array_equal(d, g.ed_batch(reads, v0)[0])
+    assert stats["retries"] == 0
