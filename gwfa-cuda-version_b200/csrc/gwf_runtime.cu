@@ -691,7 +691,18 @@ struct BlocksPlan {
 // as keep all of them running at once: 1,500 x 10 kbp 22.4 with two / 24.5 / 39.1, 3,000 with one 29.1
 // / 29.1 / 69.9. nw > 0: that many for every read.
 static const double kMwShare = 0.2, kMwUniform = 0.67;
-static const int32_t kMwMinQl = 1500; // shorter reads have no more than a few blocks at a time
+
+// Shortest read that gets several warps: shorter ones have no more than a few blocks at a time. With a
+// bound 1,500 bases, on a dense graph 40 units of bw_layout (1 kbp reads, 49 units, one warp / several:
+// 200 reads 3.4 / 2.5 ms, 16 1.6 / 1.4, but one read 1.1 / 1.3); open reads 1 unit, on a sparse graph 4
+// (1,000 reads of 500 bases, 1.3 units: 0.22 / 0.27 ms, of 1.4 kbp, 11 units: 2.2 / 1.8).
+static double mw_min_ql(const KParams &p, const Batch &B)
+{
+	const double unit = 1e6 / p.dens_milli;
+	const bool sparse = p.dens_milli < kSparse;
+	if (bw_open(p.g.bloom, B.max_ql, p.max_lag)) return sqrt(sparse ? 4 * unit : unit);
+	return sparse || B.n < 8 ? 1500 : std::min(1500.0, sqrt(40 * unit));
+}
 
 static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
                        int32_t nw, const KParams &p, BlocksPlan *pl)
@@ -707,8 +718,12 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 		const double per = (double)B->n / (double)slots;
 		int32_t all = 16; // warps per read with which all reads run at once
 		while (all > 1 && (int64_t)all * B->n > slots) all >>= 1;
-		double from = std::max(sqrt(kMwShare * per * per * mean), (double)kMwMinQl);
-		if (mean > kMwUniform * top) from = all > 1 && B->max_ql >= kMwMinQl ? 0 : 4e9;
+		// at least four where reads without a bound make that many states (dense graph, one warp / four:
+		// 5,000 x 3 kbp 89 / 65 ms, 6,000 x 10 kbp 1190 / 830, 79 and 1080 in the sorted form)
+		if (all < 4 && p.max_lag == 0 && bw_open(p.g.bloom, B->max_ql, 0) && bw_u10(B->max_ql, p.dens_milli) >= 3000) all = 4;
+		const double min_ql = mw_min_ql(p, *B);
+		double from = std::max(sqrt(kMwShare * per * per * mean), min_ql);
+		if (mean > kMwUniform * top) from = all > 1 && B->max_ql >= min_ql ? 0 : 4e9;
 		cap = 0;
 		// the queue's order is by ql >> 6, longest first: the reads above a bucket are its head
 		const int64_t bucket = (int64_t)(from / 64) - (from == 0);
@@ -762,7 +777,7 @@ static int enqueue_blocks(Engine &E, KParams p, const BlocksPlan &pl, const int3
 		}
 		KParams q = p;
 		q.order = d_order, q.n_order = pl.n_mw, q.head = (int32_t *)E.head.p + 1;
-		q.ws = (uint8_t *)E.ws.p, q.bw = pl.lay_mw;
+		q.ws = (uint8_t *)E.ws.p, q.bw = pl.lay_mw, q.defer = defer && p.retry_list;
 		k_align_blocks_mw<<<(int)pl.ctas_mw, 32 * pl.mw, bw_shm_bytes(pl.mw), s>>>(q);
 		CK(cudaGetLastError());
 		if (two) CK(cudaEventRecord(E.join, s));
@@ -1088,13 +1103,17 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	// the block form: forced, or by rule (plan_blocks). Not the tuned counts: those are a bucket's, on
 	// a sample of its reads, and a count for a whole batch switches off its split by length (30,000
 	// mixed reads: 153 ms with the count tuned on 300 reads a bucket, 22 by rule)
-	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p);
+	// Few short reads without a bound on a sparse graph stay in the sorted form (bw_open): 200 x 500
+	// bases 0.18 ms, 0.20 in the block form, their reverse complements 1.2 and 1.9
+	const int64_t u10 = bw_u10(B.max_ql, p.dens_milli);
+	const bool few = warps_per_read <= 0 && p.dens_milli < kSparse && bw_open(p.g.bloom, B.max_ql, p.max_lag) &&
+	                 u10 >= 10 && u10 < kSparseU10 && 8LL * B.n <= (int64_t)E.sm_count * E.blocks_warps_per_sm;
+	const bool blocks = mode != GWF_MODE_PLAIN && !few && blocks_ok(p);
 	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp at lag 20 7.5 ms, 10.1 with two.
-	// From kWideLag on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the dense graph
-	// at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 / 62; 200 reads of 0.5-20 kbp at lag 60
-	// 21 / 21, 200 42 / 32, 2000 470 / 96)
-	const int32_t kWideLag = 200;
-	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 && p.max_lag < kWideLag ? 1 : 0;
+	// From kFreeLag on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the dense graph
+	// at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 / 62; 1,000 x 3 kbp on the sparse one at
+	// lag 200 2.3 / 2.6, 600 4.6 / 4.1)
+	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 && p.max_lag < kFreeLag ? 1 : 0;
 	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;

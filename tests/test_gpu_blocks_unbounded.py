@@ -91,3 +91,38 @@ def test_large_lag_gets_warps_by_rule(G):
 
     (t8, d8), (t0, d0) = best(8), best(0)
     assert np.array_equal(d0, d8) and t0 < 1.6 * t8
+
+
+def test_reads_without_a_filter_get_warps_by_rule(G):
+    """Reads of 1.4 kbp, few enough for a group each, on a dense graph without a filter: they get one (the
+    time of eight warps each, with a factor to spare; with one warp it was more than twice that)."""
+    sg, g, s2v = _dense(G, 200_000, 20, lower=True)
+    cat, offs, lens, v0 = _reads(sg, s2v, 200, 0, 1400, 0, 1400, 1400, 0.05, 0.05, seed=3)
+    b = G.ResidentBatch(g, cat, offs, lens, v0, mode=G.MODE_PERSISTENT)
+    ms, d = {}, {}
+    for nw in (8, 0):
+        ms[nw] = min(b.run(warps_per_read=nw) for _ in range(4))
+        d[nw] = b.results()[0]
+    b.close()
+    assert np.array_equal(d[0], d[8]) and ms[0] < 1.6 * ms[8]
+
+
+@pytest.mark.parametrize("ql", [400, 430, 500, 599, 600])
+@pytest.mark.parametrize("n", [3, 592, 593])
+def test_short_reads_on_a_sparse_graph(G, O, ql, n):
+    """Both sides of the lines between the sorted form and the block form for short reads: below and above
+    one unit of size (430 bases here), 600 bases, and a group of eight warps for each read or not. A fifth
+    of the reads are reverse complements; with and without a large lag."""
+    sg, g, s2v = _dense(G, 100_000, 500, seed=33)
+    cat, offs, lens, v0 = _reads(sg, s2v, n, 0, ql, 0, ql, ql, 0.0, 0.10, seed=ql)
+    un = _revcomp(cat, offs[::5], lens[::5])
+    og = O.OracleGraph.from_graph(g)
+    pick = np.unique(np.concatenate([np.arange(0, n, 40), np.arange(min(n, 3))]))
+    ref, _, _ = og.ed_batch(un, offs[pick], lens[pick], v0[pick], stats=False)
+    d, st = g.ed_batch((un, offs, lens), v0)
+    assert (st == 0).all() and np.array_equal(d[pick], ref)
+    d1, _ = g.ed_batch((un, offs, lens), v0, warps_per_read=1)
+    assert np.array_equal(d, d1)
+    lag, st = g.ed_batch((un, offs, lens), v0, flags=G.GWF_F_MAX_LAG, max_lag=300)
+    want = [og.ed(bytes(un[offs[i]:offs[i] + lens[i]]), int(v0[i]), max_lag=300)[0] for i in pick[:4]]
+    assert (st == 0).all() and list(lag[pick[:4]]) == want
