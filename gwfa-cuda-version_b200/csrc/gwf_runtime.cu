@@ -693,15 +693,17 @@ struct BlocksPlan {
 static const double kMwShare = 0.2, kMwUniform = 0.67;
 
 // Shortest read that gets several warps: shorter ones have no more than a few blocks at a time. With a
-// bound 1,500 bases, on a dense graph 40 units of bw_layout (1 kbp reads, 49 units, one warp / several:
-// 200 reads 3.4 / 2.5 ms, 16 1.6 / 1.4, but one read 1.1 / 1.3); open reads 1 unit, on a sparse graph 4
-// (1,000 reads of 500 bases, 1.3 units: 0.22 / 0.27 ms, of 1.4 kbp, 11 units: 2.2 / 1.8).
-static double mw_min_ql(const KParams &p, const Batch &B)
+// bound 1,500 bases; where all are of one length, on a dense graph, 40 units of bw_layout (1 kbp reads,
+// 49 units, one warp / several: 200 reads 3.4 / 2.5 ms, 16 1.6 / 1.4, but one read 1.1 / 1.3; 300 reads
+// of 0.5-8 kbp at 200 vertices per 1000 bases 39 with 1,500 bases, 45 with 40 units). Open reads 1 unit,
+// on a sparse graph 4 (1,000 reads of 500 bases, 1.3 units: 0.22 / 0.27 ms, of 1.4 kbp, 11 units: 2.2 /
+// 1.8).
+static double mw_min_ql(const KParams &p, const Batch &B, bool one_length)
 {
 	const double unit = 1e6 / p.dens_milli;
 	const bool sparse = p.dens_milli < kSparse;
 	if (bw_open(p.g.bloom, B.max_ql, p.max_lag)) return sqrt(sparse ? 4 * unit : unit);
-	return sparse || B.n < 8 ? 1500 : std::min(1500.0, sqrt(40 * unit));
+	return sparse || B.n < 8 || !one_length ? 1500 : std::min(1500.0, sqrt(40 * unit));
 }
 
 static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_cap, int32_t level, int warps_per_sm,
@@ -721,9 +723,10 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 		// at least four where reads without a bound make that many states (dense graph, one warp / four:
 		// 5,000 x 3 kbp 89 / 65 ms, 6,000 x 10 kbp 1190 / 830, 79 and 1080 in the sorted form)
 		if (all < 4 && p.max_lag == 0 && bw_open(p.g.bloom, B->max_ql, 0) && bw_u10(B->max_ql, p.dens_milli) >= 3000) all = 4;
-		const double min_ql = mw_min_ql(p, *B);
+		const bool one_length = mean > kMwUniform * top;
+		const double min_ql = mw_min_ql(p, *B, one_length);
 		double from = std::max(sqrt(kMwShare * per * per * mean), min_ql);
-		if (mean > kMwUniform * top) from = all > 1 && B->max_ql >= min_ql ? 0 : 4e9;
+		if (one_length) from = all > 1 && B->max_ql >= min_ql ? 0 : 4e9;
 		cap = 0;
 		// the queue's order is by ql >> 6, longest first: the reads above a bucket are its head
 		const int64_t bucket = (int64_t)(from / 64) - (from == 0);
