@@ -1075,6 +1075,24 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 	return 0;
 }
 
+// Batches of short reads without a bound that the sorted form aligns faster, ms sorted / block form:
+// - few on a sparse graph (bw_open): 200 x 500 bases 0.18 / 0.20, their reverse complements 1.2 / 1.9;
+// - many on a dense one, where a read meets few states and many vertices, each a block to make: up to
+//   kBulkShort bases, and up to kBulkQl as far as kBulkU10. 100,000 x 150 bases at up to 2% errors 1.2 /
+//   1.4, at 10% 3.2 / 3.2; x 300 2.5 / 3.0 and 10.2 / 8.9; at 550 vertices per 1000 bases x 150 7.6 / 12.8
+//   and 25.7 / 27.7, x 300 37 / 33 and 144 / 101; at 200 x 200 4.8 / 6.0 and 19.2 / 14.5. Not both
+//   strands: 2,000 reverse complements of 200 bases 4.7 / 2.2.
+static const int32_t kBulkShort = 160, kBulkQl = 320, kBulkU10 = 80;
+
+static bool sorted_is_faster(const Engine &E, const Batch &B, const KParams &p)
+{
+	if (!bw_open(p.g.bloom, B.max_ql, p.max_lag)) return false;
+	const int64_t slots = (int64_t)E.sm_count * E.blocks_warps_per_sm, u10 = bw_u10(B.max_ql, p.dens_milli);
+	if (p.dens_milli < kSparse) return u10 >= 10 && u10 < kSparseU10 && 8LL * B.n <= slots;
+	const bool brief = B.max_ql <= kBulkShort || (B.max_ql <= kBulkQl && u10 <= kBulkU10);
+	return p.max_lag == 0 && !B.both && brief && B.n > slots;
+}
+
 int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t flags,
                    int ctas_per_sm, float *ms, int *launches_out, int use_graph, int32_t max_lag,
                    int32_t warps_per_read, bool fetch)
@@ -1106,12 +1124,7 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	// the block form: forced, or by rule (plan_blocks). Not the tuned counts: those are a bucket's, on
 	// a sample of its reads, and a count for a whole batch switches off its split by length (30,000
 	// mixed reads: 153 ms with the count tuned on 300 reads a bucket, 22 by rule)
-	// Few short reads without a bound on a sparse graph stay in the sorted form (bw_open): 200 x 500
-	// bases 0.18 ms, 0.20 in the block form, their reverse complements 1.2 and 1.9
-	const int64_t u10 = bw_u10(B.max_ql, p.dens_milli);
-	const bool few = warps_per_read <= 0 && p.dens_milli < kSparse && bw_open(p.g.bloom, B.max_ql, p.max_lag) &&
-	                 u10 >= 10 && u10 < kSparseU10 && 8LL * B.n <= (int64_t)E.sm_count * E.blocks_warps_per_sm;
-	const bool blocks = mode != GWF_MODE_PLAIN && !few && blocks_ok(p);
+	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p) && (warps_per_read > 0 || !sorted_is_faster(E, B, p));
 	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp at lag 20 7.5 ms, 10.1 with two.
 	// From kFreeLag on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the dense graph
 	// at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 / 62; 1,000 x 3 kbp on the sparse one at

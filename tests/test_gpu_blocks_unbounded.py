@@ -126,3 +126,18 @@ def test_short_reads_on_a_sparse_graph(G, O, ql, n):
     lag, st = g.ed_batch((un, offs, lens), v0, flags=G.GWF_F_MAX_LAG, max_lag=300)
     want = [og.ed(bytes(un[offs[i]:offs[i] + lens[i]]), int(v0[i]), max_lag=300)[0] for i in pick[:4]]
     assert (st == 0).all() and list(lag[pick[:4]]) == want
+
+
+@pytest.mark.parametrize("ql", [40, 150, 305, 340])
+@pytest.mark.parametrize("n", [4736, 4737])
+def test_many_short_reads_on_a_dense_graph(G, O, ql, n):
+    """Both sides of the line between the block form and the sorted form for many short reads on a dense
+    graph: the warp slots of the device, and 320 bases."""
+    sg, g, s2v = _dense(G, 100_000, 50, seed=35)
+    cat, offs, lens, v0 = _reads(sg, s2v, n, 0, ql, 0, ql, ql, 0.0, 0.10, seed=ql)
+    d, st = g.ed_batch((cat, offs, lens), v0)
+    d1, st1 = g.ed_batch((cat, offs, lens), v0, warps_per_read=1)
+    assert (st == 0).all() and np.array_equal(d, d1) and np.array_equal(st, st1)
+    pick = np.arange(0, n, 100)
+    ref, _, _ = O.OracleGraph.from_graph(g).ed_batch(cat, offs[pick], lens[pick], v0[pick], stats=False)
+    assert np.array_equal(d[pick], ref)
