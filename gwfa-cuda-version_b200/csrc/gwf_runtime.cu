@@ -1018,17 +1018,14 @@ static int enqueue_classes(Engine &E, KParams p, const ClassLaunch &cl)
 // Level-0 sequence of the persistent form as one CUDA graph: pack, clear the overflow count,
 // persistent kernel, copy the overflow count to the host. Captured once per batch contents and
 // launch shape, replayed on every run.
-static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_per_sm, bool classes, bool blocks,
-                               int32_t nw, int *launches)
+static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_per_sm, bool classes,
+                               const BlocksPlan *bp, bool defer, int *launches)
 {
 	PersistPlan pl;
-	BlocksPlan bp;
 	ClassLaunch cl;
 	int rc;
-	const bool defer = blocks && defer_unlike(E, B.n, ctas_per_sm, nw);
-	if (blocks) {
-		if ((rc = plan_blocks(E, &B, B.n, B.max_ql, 1, ctas_per_sm, nw, p, &bp))) return rc;
-		pl.ctas = (int)bp.ctas, pl.slot = bp.lay.total;
+	if (bp) {
+		pl.ctas = (int)bp->ctas, pl.slot = bp->lay.total;
 	} else if (classes) {
 		if ((rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl))) return rc;
 		pl.ctas = cl.ctas, pl.slot = cl.cp.cta_bytes;
@@ -1038,8 +1035,8 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 	                         (uint64_t)(uint32_t)p.flags | (uint64_t)(uint32_t)p.max_lag << 32,
 	                         (uint64_t)(uintptr_t)B.res.p,
 	                         (uint64_t)(uintptr_t)E.h_small.p, (uint64_t)(uintptr_t)E.retry_list.p,
-	                         blocks ? ~(1ULL | (uint64_t)defer << 1 | (uint64_t)bp.n_mw << 8 | (uint64_t)bp.mw << 40 |
-	                                    (uint64_t)bp.ctas_mw << 46)
+	                         bp ? ~(1ULL | (uint64_t)defer << 1 | (uint64_t)bp->n_mw << 8 | (uint64_t)bp->mw << 40 |
+	                                (uint64_t)bp->ctas_mw << 46)
 	                         : classes ? B.cls_key ^ B.cls_gen << 40
 	                                   : ~0ULL};
 	if (!B.gexec || memcmp(key, B.gkey, sizeof key) != 0) {
@@ -1047,7 +1044,7 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 		CK(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
 		int erc = enqueue_pack(E, B);
 		if (!erc && cudaMemsetAsync(B.d_count, 0, 4, E.stream) != cudaSuccess) erc = GWF_E_CUDA;
-		if (!erc) erc = blocks ? enqueue_blocks(E, p, bp, B.d_order, B.n, defer)
+		if (!erc) erc = bp ? enqueue_blocks(E, p, *bp, B.d_order, B.n, defer)
 		                : classes ? enqueue_classes(E, p, cl)
 		                        : enqueue_persistent(E, p, pl, B.d_order, B.n, B.max_ql, 0);
 		if (!erc && cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream) != cudaSuccess)
@@ -1071,7 +1068,7 @@ static int launch_level0_graph(Engine &E, Batch &B, const KParams &p, int ctas_p
 		memcpy(B.gkey, key, sizeof key);
 	}
 	CK(cudaGraphLaunch(B.gexec, E.stream));
-	*launches += 2 + (blocks && bp.n_mw > 0 && bp.n_mw < B.n); // packing and the batch's kernels
+	*launches += 2 + (bp && bp->n_mw > 0 && bp->n_mw < B.n); // packing and the batch's kernels
 	return 0;
 }
 
@@ -1124,24 +1121,31 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	// the block form: forced, or by rule (plan_blocks). Not the tuned counts: those are a bucket's, on
 	// a sample of its reads, and a count for a whole batch switches off its split by length (30,000
 	// mixed reads: 153 ms with the count tuned on 300 reads a bucket, 22 by rule)
-	const bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p) && (warps_per_read > 0 || !sorted_is_faster(E, B, p));
+	bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p) && (warps_per_read > 0 || !sorted_is_faster(E, B, p));
 	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp at lag 20 7.5 ms, 10.1 with two.
 	// From kFreeLag on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the dense graph
 	// at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 / 62; 1,000 x 3 kbp on the sparse one at
 	// lag 200 2.3 / 2.6, 600 4.6 / 4.1)
 	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 && p.max_lag < kFreeLag ? 1 : 0;
+	const int warps_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm * kWarpsPerCta, E.blocks_warps_per_sm) : E.blocks_warps_per_sm;
+	BlocksPlan bp;
+	if (blocks) {
+		rc = plan_blocks(E, &B, B.n, B.max_ql, 1, warps_per_sm, nw_blocks, p, &bp);
+		if (rc && rc != GWF_E_NOMEM) return rc;
+		if (rc) blocks = false; // short of memory: the sorted form's arenas may fit
+	}
+	const bool defer = blocks && defer_unlike(E, B.n, warps_per_sm, nw_blocks);
 	if (mode != GWF_MODE_PLAIN && !blocks) {
 		const int64_t slots = (int64_t)E.sm_count * E.persistent_ctas_per_sm * kWarpsPerCta;
 		if ((rc = plan_classes(E, B, nw_b, slots, G.dens_milli))) return rc;
 		classes = B.cls_n > 1 || B.cls_nw[0] > 1;
 	}
-	const int warps_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm * kWarpsPerCta, E.blocks_warps_per_sm) : E.blocks_warps_per_sm;
 	if (ctas_per_sm <= 0)
 		ctas_per_sm = classes ? E.classes_ctas_per_sm : E.persistent_ctas_per_sm;
 	bool count_copied = false;
 	if (ms) CK(cudaEventRecord(E.ev0, E.stream));
 	if (use_graph && mode != GWF_MODE_PLAIN) {
-		if ((rc = launch_level0_graph(E, B, p, blocks ? warps_per_sm : ctas_per_sm, classes, blocks, nw_blocks, &launches)))
+		if ((rc = launch_level0_graph(E, B, p, ctas_per_sm, classes, blocks ? &bp : nullptr, defer, &launches)))
 			return rc;
 		count_copied = true;
 	} else {
@@ -1150,10 +1154,8 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		if (mode == GWF_MODE_PLAIN) rc = launch_plain(E, p, B, &launches);
 		else if (blocks) {
-			BlocksPlan pl;
-			if (!(rc = plan_blocks(E, &B, B.n, B.max_ql, 1, warps_per_sm, nw_blocks, p, &pl)) &&
-			    !(rc = enqueue_blocks(E, p, pl, B.d_order, B.n, defer_unlike(E, B.n, warps_per_sm, nw_blocks))))
-				launches += 1 + (pl.n_mw > 0 && pl.n_mw < B.n);
+			if (!(rc = enqueue_blocks(E, p, bp, B.d_order, B.n, defer)))
+				launches += 1 + (bp.n_mw > 0 && bp.n_mw < B.n);
 		} else if (classes) {
 			ClassLaunch cl;
 			if (!(rc = plan_class_launch(E, B, ctas_per_sm, p.dens_milli, &cl)) && !(rc = enqueue_classes(E, p, cl)))
@@ -1162,9 +1164,9 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 			rc = launch_persistent(E, p, B.d_order, B.n, B.max_ql, 0, ctas_per_sm, &launches);
 		if (rc) return rc;
 	}
-	// re-run arena overflows at larger size classes (the block form's first in a larger arena of its
-	// own, then as the sorted form's)
-	for (int level = blocks ? 0 : 1; level <= kMaxLevel; ++level) {
+	// re-run arena overflows at larger size classes: the block form's first in a larger arena of its own
+	// (-1), then as the sorted form's, from 4x on, or from 1x where the block form's does not fit
+	for (int level = blocks ? -1 : 1; level <= kMaxLevel; ++level) {
 		int32_t nr = 0;
 		if (fetch) { // results and the overflow count in one copy, through the pinned input block
 			if ((rc = B.h_meta.ensure(8 * (size_t)B.n + 64))) return rc;
@@ -1189,15 +1191,18 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 		CK(cudaMemcpyAsync(E.order.p, ids.data(), 4 * (size_t)nr, cudaMemcpyHostToDevice, E.stream));
 		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
 		KParams q = p;
-		if (level == 0) {
+		if (level < 0) {
+			level = 0;
 			BlocksPlan pl; // as many warps per read as keep all reads running at once
 			int32_t nw = 16;
 			while (nw > 1 && (int64_t)nw * nr > (int64_t)E.sm_count * warps_per_sm) nw >>= 1;
-			if ((rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p, &pl)) ||
-			    (rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr, false)))
-				return rc;
-			++launches;
-			continue;
+			rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p, &pl);
+			if (!rc) {
+				if ((rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr, false))) return rc;
+				++launches;
+				continue;
+			}
+			if (rc != GWF_E_NOMEM) return rc;
 		}
 		if (level == kMaxLevel) q.retry_list = nullptr; // last class: keep GWF_E_CAPACITY
 		if ((rc = launch_persistent(E, q, (const int32_t *)E.order.p, nr, cap, level,
