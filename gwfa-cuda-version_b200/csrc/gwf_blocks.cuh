@@ -1052,8 +1052,8 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 		lag = (float)h0 < 1.7f * (float)(ql / g.bloom_k);
 		if (!lag && p.defer) { // such a read makes thousands of states per step: left to a group of warps
 			if (lead) {
-				p.dist[r] = -1, p.status[r] = ST_CAPACITY;
-				if (p.retry_list) p.retry_list[atomicAdd(p.retry_n, 1)] = r;
+				p.dist[r] = -1, p.status[r] = p.retry_list ? ST_CAPACITY : ST_UNLIKE;
+				if (p.retry_list) p.retry_list[atomicAdd(p.retry_n, 1)] = ~r;
 			}
 			return;
 		}

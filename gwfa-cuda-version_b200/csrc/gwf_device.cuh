@@ -32,6 +32,7 @@ constexpr uint64_t PAD_KEY = ~0ULL;
 constexpr int32_t ST_OK = 0;
 constexpr int32_t ST_BAD_INPUT = -2;
 constexpr int32_t ST_CAPACITY = -4;
+constexpr int32_t ST_UNLIKE = -104; // inside the serving loop: given up before a step, for an arena that holds the read
 
 constexpr uint32_t kVArcsBits = 28, kVArcsMask = (1u << kVArcsBits) - 1, kVArcsMany = 15;
 

@@ -1052,7 +1052,7 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constan
 		const int64_t qb = srv_qbytes(ql);
 		KParams lp;
 		memset(&lp, 0, sizeof lp);
-		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli, bw_open(p.g.bloom, ql, p.max_lag));
+		if (blocks) lp.bw = bw_layout(ql, level, p.dens_milli, p.g.bloom, p.max_lag);
 		const int64_t need = blocks ? lp.bw.total : ws_layout(caps_for(ql, level, p.dens_milli)).total;
 		if (qb + need <= abytes) { // the host sized it so; else report capacity
 			lp.g = p.g;
@@ -1073,7 +1073,7 @@ __global__ void __launch_bounds__(32 * NW, 24 / NW) k_serve(const __grid_constan
 			if (blocks) {
 				lp.defer = level == 0;
 				bw_init(lp.g, lp.bw, ab + qb);
-				const bool open = bw_open(p.g.bloom, ql, p.max_lag) && bw_u10(ql, p.dens_milli) >= 10;
+				const bool open = bw_open(p.g.bloom, ql, p.max_lag, p.dens_milli) && bw_u10(ql, p.dens_milli) >= 10;
 				if (NW > 1 && (level > 0 || ql >= kServeMwMinQl || open))
 					align_read_blocks<(NW > 1)>(lp, 0, ab + qb);
 				else if (threadIdx.x < 32)

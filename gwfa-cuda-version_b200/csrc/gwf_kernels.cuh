@@ -13,12 +13,14 @@ struct BwLay {
 };
 
 constexpr int32_t kPruneMinQl = 600; // shorter reads are not pruned: their few steps cost less than a bound
-constexpr int32_t kFreeLag = 300;    // the caller's lag pruning from here on keeps many states
+constexpr int32_t kFreeLag = 300, kFreeLagDens = 8000; // the caller's lag from which it keeps many states,
+                                                       // or lag x vertices per 1000 bases
 
 // Does a read run without a bound, and without a small lag of the caller's?
-__host__ __device__ inline bool bw_open(bool bloom, int32_t ql, int32_t max_lag)
+__host__ __device__ inline bool bw_open(bool bloom, int32_t ql, int32_t max_lag, int32_t dens_milli)
 {
-	return max_lag > 0 ? max_lag >= kFreeLag : !bloom || ql < kPruneMinQl;
+	if (max_lag > 0) return max_lag >= kFreeLag || (int64_t)max_lag * dens_milli >= kFreeLagDens;
+	return !bloom || ql < kPruneMinQl;
 }
 
 // A read's size in tenths of the unit u of bw_layout
@@ -35,17 +37,22 @@ constexpr int32_t kSparse = 20, kSparseU10 = 120;
 // Arena for reads of up to ql bases at retry class level on a graph of dens_milli vertices per 1000
 // bases. Blocks that reads make, in units of u = dens_milli ql^2 / 10^6 (64 reads each of 1, 3 and 10
 // kbp, graphs of 5 to 550 vertices per 1000 bases): with a bound 0.4 to 5.7 at 2 to 10% errors, the
-// upper end short reads, which the other terms hold; open 3 to 26, or lag 2000 up to 17, 600 up to 7;
-// reads unlike the graph 90 to 110. Class 0 (serving's first, where arenas share a budget) leaves out
-// the last, class 1 (the first of a batch) holds short ones of them, class 2 all (reads of 3 kbp on
-// the dense benchmark graph that met no such class ended in the sorted form).
-__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli, bool open)
+// upper end short reads, which the other terms hold; without a bound 3 to 26; with a lag 0.03 to 0.05
+// ql x lag per vertex and 1000 bases; reads unlike the graph 90 to 110. Class 0 (serving's first, where arenas share a budget) leaves out
+// the last, class 1 (the first of a batch) holds short ones of them, class 2 reads with a bound at twice
+// those errors, class 3 all (reads of 3 kbp unlike the dense benchmark graph that met no such class
+// ended in the sorted form; 1,000 x 10 kbp at 12 to 15% that met only class 3 after 1: 171 -> 223 ms).
+__host__ __device__ inline BwLay bw_layout(int32_t ql, int32_t level, int32_t dens_milli, bool bloom, int32_t max_lag)
 {
 	const int64_t q = ql < 64 ? 64 : ql, u10 = bw_u10((int32_t)q, dens_milli);
 	int64_t nb = 128 + (int64_t)dens_milli * q * 8 / 1000 + u10 / 4;
 	if (level > 0) nb += q / 2;
-	if (level > 1) nb = 8 * nb + 13 * u10;
-	else if (open) nb += 5 * u10 / 2;
+	if (level > 1) nb = 8 * nb + (level > 2 ? 13 * u10 : 0);
+	else if (max_lag > 0) {
+		const int64_t lag = (int64_t)dens_milli * q / 1000 * max_lag / 20;
+		nb += lag < 5 * u10 / 2 ? lag : 5 * u10 / 2;
+	} else if (!bloom || q < kPruneMinQl)
+		nb += 5 * u10 / 2;
 	if (nb > (1 << 22)) nb = 1 << 22;
 	BwLay o;
 	o.nb = (int32_t)nb, o.hs = pow2ceil_i(2 * o.nb);
@@ -91,7 +98,7 @@ struct KParams {
 	int32_t *path_arc;      // arc index into path_v[j] (-1 for j = 0)
 	int32_t max_nv;
 	BwLay bw;               // block form: layout of a CTA's arena
-	int32_t defer;          // block form, one warp: reads unlike the graph are given up (GWF_E_CAPACITY)
+	int32_t defer;          // block form, one warp: reads unlike the graph are given up
 };
 
 // ---- serving: one resident kernel, warps pull single reads from a device queue

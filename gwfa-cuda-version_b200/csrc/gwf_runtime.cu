@@ -702,7 +702,7 @@ static double mw_min_ql(const KParams &p, const Batch &B, bool one_length)
 {
 	const double unit = 1e6 / p.dens_milli;
 	const bool sparse = p.dens_milli < kSparse;
-	if (bw_open(p.g.bloom, B.max_ql, p.max_lag)) return sqrt(sparse ? 4 * unit : unit);
+	if (bw_open(p.g.bloom, B.max_ql, p.max_lag, p.dens_milli)) return sqrt(sparse ? 4 * unit : unit);
 	return sparse || B.n < 8 || !one_length ? 1500 : std::min(1500.0, sqrt(40 * unit));
 }
 
@@ -722,7 +722,7 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 		while (all > 1 && (int64_t)all * B->n > slots) all >>= 1;
 		// at least four where reads without a bound make that many states (dense graph, one warp / four:
 		// 5,000 x 3 kbp 89 / 65 ms, 6,000 x 10 kbp 1190 / 830, 79 and 1080 in the sorted form)
-		if (all < 4 && p.max_lag == 0 && bw_open(p.g.bloom, B->max_ql, 0) && bw_u10(B->max_ql, p.dens_milli) >= 3000) all = 4;
+		if (all < 4 && p.max_lag == 0 && bw_open(p.g.bloom, B->max_ql, 0, p.dens_milli) && bw_u10(B->max_ql, p.dens_milli) >= 3000) all = 4;
 		const bool one_length = mean > kMwUniform * top;
 		const double min_ql = mw_min_ql(p, *B, one_length);
 		double from = std::max(sqrt(kMwShare * per * per * mean), min_ql);
@@ -738,8 +738,8 @@ static int plan_blocks(Engine &E, const Batch *B, int32_t n_order, int32_t ql_ca
 		if (from == 0) pl->mw = all;
 		else if (pl->n_mw) pl->mw = 16LL * pl->n_mw <= slots ? 16 : 8;
 	}
-	pl->lay_mw = bw_layout(ql_cap, level, p.dens_milli, bw_open(p.g.bloom, ql_cap, p.max_lag));
-	pl->lay = bw_layout(cap, level, p.dens_milli, bw_open(p.g.bloom, cap, p.max_lag));
+	pl->lay_mw = bw_layout(ql_cap, level, p.dens_milli, p.g.bloom, p.max_lag);
+	pl->lay = bw_layout(cap, level, p.dens_milli, p.g.bloom, p.max_lag);
 	const int64_t budget = std::max<int64_t>(E.mem_budget, (int64_t)E.ws.cap);
 	const int32_t n_one = n_order - pl->n_mw;
 	if (pl->n_mw) pl->ctas_mw = std::min<int64_t>(pl->n_mw, std::max<int64_t>(1, slots / pl->mw));
@@ -1083,11 +1083,46 @@ static const int32_t kBulkShort = 160, kBulkQl = 320, kBulkU10 = 80;
 
 static bool sorted_is_faster(const Engine &E, const Batch &B, const KParams &p)
 {
-	if (!bw_open(p.g.bloom, B.max_ql, p.max_lag)) return false;
+	if (!bw_open(p.g.bloom, B.max_ql, p.max_lag, p.dens_milli)) return false;
 	const int64_t slots = (int64_t)E.sm_count * E.blocks_warps_per_sm, u10 = bw_u10(B.max_ql, p.dens_milli);
 	if (p.dens_milli < kSparse) return u10 >= 10 && u10 < kSparseU10 && 8LL * B.n <= slots;
 	const bool brief = B.max_ql <= kBulkShort || (B.max_ql <= kBulkQl && u10 <= kBulkU10);
 	return p.max_lag == 0 && !B.both && brief && B.n > slots;
+}
+
+// The reads that the launches so far gave up, as the retry list has them (~r for one found unlike
+// the graph before its first step); none: the results are complete. fetch: results and count in one copy,
+// through the pinned input block. have_count: the count is on its way to h_small already.
+static int overflowed(Engine &E, Batch &B, bool fetch, bool have_count, std::vector<int32_t> *ids)
+{
+	int rc;
+	if (fetch) {
+		if ((rc = B.h_meta.ensure(8 * (size_t)B.n + 64))) return rc;
+		CK(cudaMemcpyAsync(B.h_meta.p, B.res.p, 8 * (size_t)B.n + 4, cudaMemcpyDeviceToHost, E.stream));
+	} else if (!have_count)
+		CK(cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream));
+	CK(cudaStreamSynchronize(E.stream));
+	const int32_t nr = fetch ? ((const int32_t *)B.h_meta.p)[2 * (size_t)B.n] : *(int32_t *)E.h_small.p;
+	B.fetched = fetch && nr == 0;
+	ids->clear();
+	if (nr == 0) return 0;
+	CK(cudaMemcpyAsync(E.h_small.p, E.retry_list.p, 4 * (size_t)nr, cudaMemcpyDeviceToHost, E.stream));
+	CK(cudaStreamSynchronize(E.stream));
+	ids->assign((const int32_t *)E.h_small.p, (const int32_t *)E.h_small.p + nr);
+	return 0;
+}
+
+// Queue of a retry launch, longest read first, and an empty retry list
+static int upload_order(Engine &E, Batch &B, std::vector<int32_t> &ids, int32_t *cap)
+{
+	std::sort(ids.begin(), ids.end(), [&](int32_t x, int32_t y) { return B.h_ql[(size_t)x] > B.h_ql[(size_t)y]; });
+	*cap = B.h_ql[(size_t)ids[0]];
+	B.fetched = false;
+	int rc;
+	if ((rc = E.order.ensure(4 * ids.size()))) return rc;
+	CK(cudaMemcpyAsync(E.order.p, ids.data(), 4 * ids.size(), cudaMemcpyHostToDevice, E.stream));
+	CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
+	return 0;
 }
 
 int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t flags,
@@ -1123,10 +1158,11 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 	// mixed reads: 153 ms with the count tuned on 300 reads a bucket, 22 by rule)
 	bool blocks = mode != GWF_MODE_PLAIN && blocks_ok(p) && (warps_per_read > 0 || !sorted_is_faster(E, B, p));
 	// (with lag pruning one warp: few states live at a time; 2,000 x 10 kbp at lag 20 7.5 ms, 10.1 with two.
-	// From kFreeLag on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the dense graph
-	// at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 / 62; 1,000 x 3 kbp on the sparse one at
-	// lag 200 2.3 / 2.6, 600 4.6 / 4.1)
-	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : p.max_lag > 0 && p.max_lag < kFreeLag ? 1 : 0;
+	// From kFreeLag or kFreeLagDens on by rule, as without it, one warp / by rule: 1,000 x 10 kbp on the
+	// dense graph (49 vertices per 1000 bases) at lag 60 8.8 / 9.4 ms, 200 16 / 13, 600 48 / 23, 2000 182 /
+	// 62; 1,000 x 3 kbp on the sparse one (5) at lag 200 2.3 / 2.6, 600 4.6 / 4.1)
+	const bool narrow = p.max_lag > 0 && !bw_open(p.g.bloom, B.max_ql, p.max_lag, p.dens_milli);
+	const int32_t nw_blocks = warps_per_read > 0 ? warps_per_read : narrow ? 1 : 0;
 	const int warps_per_sm = ctas_per_sm > 0 ? std::min(ctas_per_sm * kWarpsPerCta, E.blocks_warps_per_sm) : E.blocks_warps_per_sm;
 	BlocksPlan bp;
 	if (blocks) {
@@ -1164,49 +1200,49 @@ int gwf_batch_exec(Engine &E, const GraphDev &G, Batch &B, int32_t mode, int32_t
 			rc = launch_persistent(E, p, B.d_order, B.n, B.max_ql, 0, ctas_per_sm, &launches);
 		if (rc) return rc;
 	}
-	// re-run arena overflows at larger size classes: the block form's first in a larger arena of its own
-	// (-1), then as the sorted form's, from 4x on, or from 1x where the block form's does not fit
-	for (int level = blocks ? -1 : 1; level <= kMaxLevel; ++level) {
-		int32_t nr = 0;
-		if (fetch) { // results and the overflow count in one copy, through the pinned input block
-			if ((rc = B.h_meta.ensure(8 * (size_t)B.n + 64))) return rc;
-			CK(cudaMemcpyAsync(B.h_meta.p, B.res.p, 8 * (size_t)B.n + 4, cudaMemcpyDeviceToHost, E.stream));
-		} else if (!count_copied)
-			CK(cudaMemcpyAsync(E.h_small.p, B.d_count, 4, cudaMemcpyDeviceToHost, E.stream));
-		count_copied = false;
-		CK(cudaStreamSynchronize(E.stream));
-		nr = fetch ? ((const int32_t *)B.h_meta.p)[2 * (size_t)B.n] : *(int32_t *)E.h_small.p;
-		if (nr == 0) {
-			B.fetched = fetch;
-			break;
-		}
-		std::vector<int32_t> ids((size_t)nr);
-		CK(cudaMemcpyAsync(E.h_small.p, E.retry_list.p, 4 * (size_t)nr, cudaMemcpyDeviceToHost, E.stream));
-		CK(cudaStreamSynchronize(E.stream));
-		memcpy(ids.data(), E.h_small.p, 4 * (size_t)nr);
-		int32_t cap = 0;
-		for (int32_t r : ids) cap = std::max(cap, B.h_ql[(size_t)r]);
-		std::sort(ids.begin(), ids.end(), [&](int32_t x, int32_t y) { return B.h_ql[(size_t)x] > B.h_ql[(size_t)y]; });
-		if ((rc = E.order.ensure(4 * (size_t)nr))) return rc;
-		CK(cudaMemcpyAsync(E.order.p, ids.data(), 4 * (size_t)nr, cudaMemcpyHostToDevice, E.stream));
-		CK(cudaMemsetAsync(B.d_count, 0, 4, E.stream));
-		KParams q = p;
-		if (level < 0) {
-			level = 0;
-			BlocksPlan pl; // as many warps per read as keep all reads running at once
-			int32_t nw = 16;
-			while (nw > 1 && (int64_t)nw * nr > (int64_t)E.sm_count * warps_per_sm) nw >>= 1;
-			rc = plan_blocks(E, nullptr, nr, cap, 2, warps_per_sm, nw, p, &pl);
-			if (!rc) {
-				if ((rc = enqueue_blocks(E, q, pl, (const int32_t *)E.order.p, nr, false))) return rc;
+	// re-run arena overflows at larger size classes: the block form's class 2, and class 3 for reads unlike
+	// the graph (or without a bound that would have told so), then as the sorted form's, from 4x on, or
+	// from 1x where the block form's do not fit
+	std::vector<int32_t> ids;
+	if ((rc = overflowed(E, B, fetch, count_copied, &ids))) return rc;
+	int level = 1;
+	if (blocks && !ids.empty()) {
+		const bool open = bw_open(p.g.bloom, B.max_ql, p.max_lag, p.dens_milli);
+		std::vector<int32_t> part[2], over;
+		int32_t top = 0;
+		for (int32_t r : ids) part[open || r < 0].push_back(r < 0 ? ~r : r), top = std::max(top, B.h_ql[(size_t)(r < 0 ? ~r : r)]);
+		// together where class 3 is small enough for all: one launch, one end (1,000 reverse complements of
+		// 1 kbp on the dense graph 48 ms one after the other, 33 together)
+		const int64_t at_once = std::min<int64_t>((int64_t)ids.size(), (int64_t)E.sm_count * warps_per_sm);
+		if ((double)at_once * (double)bw_layout(top, 3, p.dens_milli, p.g.bloom, p.max_lag).total <= kLiveArenaBytes)
+			part[1].insert(part[1].end(), part[0].begin(), part[0].end()), part[0].clear();
+		ids.clear();
+		for (int k = 0; k < 2; ++k) {
+			if (part[k].empty()) continue;
+			int32_t cap, nw = 16; // as many warps per read as keep all reads running at once
+			while (nw > 1 && (int64_t)nw * (int64_t)part[k].size() > (int64_t)E.sm_count * warps_per_sm) nw >>= 1;
+			const int32_t nr = (int32_t)part[k].size();
+			if ((rc = upload_order(E, B, part[k], &cap))) return rc;
+			rc = plan_blocks(E, nullptr, nr, cap, 2 + k, warps_per_sm, nw, p, &bp);
+			if (rc && rc != GWF_E_NOMEM) return rc;
+			if (rc) over = part[k], level = 0;
+			else {
+				if ((rc = enqueue_blocks(E, p, bp, (const int32_t *)E.order.p, nr, false))) return rc;
 				++launches;
-				continue;
+				if ((rc = overflowed(E, B, fetch, false, &over))) return rc;
 			}
-			if (rc != GWF_E_NOMEM) return rc;
+			std::vector<int32_t> &next = k == 0 ? part[1] : ids;
+			next.insert(next.end(), over.begin(), over.end());
 		}
+	}
+	for (; level <= kMaxLevel && !ids.empty(); ++level) {
+		int32_t cap;
+		KParams q = p;
+		if ((rc = upload_order(E, B, ids, &cap))) return rc;
 		if (level == kMaxLevel) q.retry_list = nullptr; // last class: keep GWF_E_CAPACITY
-		if ((rc = launch_persistent(E, q, (const int32_t *)E.order.p, nr, cap, level,
-		                            std::min(ctas_per_sm, E.persistent_ctas_per_sm), &launches)))
+		if ((rc = launch_persistent(E, q, (const int32_t *)E.order.p, (int32_t)ids.size(), cap, level,
+		                            std::min(ctas_per_sm, E.persistent_ctas_per_sm), &launches)) ||
+		    (rc = overflowed(E, B, fetch, false, &ids)))
 			return rc;
 	}
 	if (ms) {

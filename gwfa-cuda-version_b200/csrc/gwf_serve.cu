@@ -180,35 +180,37 @@ int32_t *busy_dev(gwf_srv_s *S) { return (int32_t *)((char *)S->ctl.p + 256); }
 int64_t arena_bytes(const gwf_srv_s *S, int32_t ql, bool blocks, int32_t level)
 {
 	const int32_t dens = S->G->dens_milli;
-	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens, gwfb::bw_open(S->G->bloom.p, ql, S->max_lag)).total
+	const int64_t ws = blocks ? gwfb::bw_layout(ql, level, dens, S->G->bloom.p, S->max_lag).total
 	                          : gwfb::ws_layout(gwfb::caps_for(ql, level, dens)).total;
 	const int64_t bytes = gwfb::srv_al256(gwfb::srv_qbytes(ql) + ws);
 	return bytes <= S->pool.cap() ? bytes : -1;
 }
 
 // Arena classes of a read, in turn. Reads without a target vertex, but for short ones without a bound
-// on sparse graphs, take the block form's 0 and 2 (1 where 2 does not fit the budget), as long as they
-// fit, then the sorted form's from 4x on (as the batch path), or from 1x where 4x does
-// not fit; the others take the sorted form's. A read whose first sorted arena does not fit is not
-// served. Both return false when no class is left.
+// on sparse graphs, take the block form's, as long as they fit the budget (from class 0 straight to 3
+// where the read is unlike the graph, or has no bound that would have told so), then the sorted form's
+// from 4x on (as the batch path), or from 1x where 4x does not fit; the others take the sorted form's.
+// A read whose first sorted arena does not fit is not served. Both return false when no class is left.
 bool first_class(const gwf_srv_s *S, Slot &sl)
 {
 	const int32_t ql = sl.r->ql[(size_t)sl.read];
 	const int32_t dens = S->G->dens_milli;
 	sl.level = 0;
 	sl.blocks = S->blocks && sl.r->v1 < 0 && arena_bytes(S, ql, true, 0) >= 0 &&
-	            !(dens < gwfb::kSparse && gwfb::bw_open(S->G->bloom.p, ql, S->max_lag) &&
+	            !(dens < gwfb::kSparse && gwfb::bw_open(S->G->bloom.p, ql, S->max_lag, S->G->dens_milli) &&
 	              gwfb::bw_u10(ql, dens) < gwfb::kSparseU10);
 	return arena_bytes(S, ql, false, 0) >= 0;
 }
-bool next_class(const gwf_srv_s *S, Slot &sl)
+bool next_class(const gwf_srv_s *S, Slot &sl, int32_t st)
 {
 	const int32_t ql = sl.r->ql[(size_t)sl.read];
 	if (sl.blocks) {
-		if (sl.level == 0) { // most often a read unlike the graph
-			sl.level = arena_bytes(S, ql, true, 2) >= 0 ? 2 : 1;
-			if (arena_bytes(S, ql, true, sl.level) >= 0) return true;
-		}
+		const bool most = st == gwfb::ST_UNLIKE || gwfb::bw_open(S->G->bloom.p, ql, S->max_lag, S->G->dens_milli);
+		if (sl.level == 0 && most)
+			for (sl.level = 3; sl.level > 1 && arena_bytes(S, ql, true, sl.level) < 0;) --sl.level;
+		else
+			++sl.level;
+		if (sl.level <= 3 && arena_bytes(S, ql, true, sl.level) >= 0) return true;
 		sl.blocks = false, sl.level = arena_bytes(S, ql, false, 1) >= 0 ? 1 : 0;
 		return true;
 	}
@@ -256,7 +258,8 @@ int drain(gwf_srv_s *S)
 		volatile SrvDone *d = S->cq + (S->cq_pos & (S->ccap - 1));
 		if (d->gen != (int32_t)((S->cq_pos >> S->cq_shift) + 1)) break;
 		std::atomic_thread_fence(std::memory_order_acquire);
-		const int32_t tag = d->tag, dist = d->dist, st = d->status;
+		const int32_t tag = d->tag, dist = d->dist;
+		int32_t st = d->status;
 		++S->cq_pos, ++n;
 		if (tag < 0 || (size_t)tag >= S->slots.size() || !S->slots[(size_t)tag].r) {
 			fail_all(S, GWF_E_CUDA);
@@ -266,12 +269,12 @@ int drain(gwf_srv_s *S)
 		Slot &sl = S->slots[(size_t)tag];
 		S->pool.release(sl.off, sl.bytes);
 		sl.off = -1;
-		if (st == GWF_E_CAPACITY && next_class(S, sl)) {
+		if ((st == GWF_E_CAPACITY || st == gwfb::ST_UNLIKE) && next_class(S, sl, st)) {
 			++S->retries;
 			S->retry.push_back(tag); // keeps its slot; re-admitted with a larger arena
 			continue;
 		}
-		finish_read(S, sl.r, sl.read, dist, st);
+		finish_read(S, sl.r, sl.read, dist, st == gwfb::ST_UNLIKE ? GWF_E_CAPACITY : st);
 		release_slot(S, tag);
 	}
 	return n;
