@@ -649,7 +649,8 @@ def main():
                             "frac": achieved / peak, "traffic": traffic,
                             "peak_source": src + " hbm_gbs (burst)",
                             "algorithmic_bytes_per_step": alg,
-                            "note": "B_read = ql + 4 + 32 W + 2 E per read, W/E from the oracle"
+                            "note": "B_read = ql + 4 + 32 W + 2 E per read, W/E of the unpruned run (the oracle's): "
+                                    "counts states that pruning no longer makes; traffic is what DRAM moved"
                                     + ("" if cpu["full"] else " sample, scaled")}
     if rank == 0:
         print(json.dumps(line), flush=True)

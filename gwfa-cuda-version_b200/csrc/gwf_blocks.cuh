@@ -23,9 +23,11 @@
 // instructions issued per cycle and scheduler at 32 warps per SM, 9.2 of a warp's 20.4 cycles per
 // instruction waiting for its next instruction, 4.6 for loads, 2.8 for fixed latencies; DRAM 0.76 GB
 // in 7.6 ms), and the latency of one read's chain of steps where a batch has few or unequal reads.
-// Resident reads, graph replay, kernel_ms against the sorted form: 100,000 x 1 kbp 26.1 -> 12.7 ms,
-// 50,000 mixed 137 -> 26 ms, 4,000 x 10 kbp on the dense graph 600 -> 30 ms, one 20 kbp read at 10%
-// 374 -> 69 ms (259 with one warp, 16 here).
+// Resident reads, graph replay, kernel_ms against the sorted form: 100,000 x 1 kbp 26.1 -> 12.6 ms,
+// 50,000 mixed 137 -> 27 ms, 4,000 x 10 kbp on the dense graph 600 -> 30 ms, one 20 kbp read at 10%
+// 374 -> 67 ms (243 with one warp, 16 here). With several warps per read barriers bound it: 100 reads
+// of 10 kbp at 5% with 16 warps each, 38 of a warp's 48 cycles per instruction, 2.3 for loads: most of
+// a read's steps have work for a warp or two.
 #pragma once
 #include "gwf_kernels.cuh"
 
@@ -1138,7 +1140,8 @@ __device__ __forceinline__ void align_read_blocks(const KParams &p, int32_t r, u
 				attained = true, T = sc;
 				// The exact run makes about beta / 4 slack^2 iterations of step 1 more than one per
 				// score (slack = T - h; beta 1.2 measured on the sparse benchmark graph, 4 to 14 on the
-				// dense one); windows from every base cost the time of ~0.2 per base and make the
+				// dense one, 5 and 49 vertices per 1000 bases, nothing between measured: the line
+				// decides time only); windows from every base cost the time of ~0.2 per base and make the
 				// slack 2.2 times smaller.
 				const float slack = (float)(T - h0);
 				if ((p.dens_milli >= 20 ? 8.0f : 1.2f) * slack * slack > (float)ql) bw_seeds<MW>(1);

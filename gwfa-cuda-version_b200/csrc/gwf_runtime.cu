@@ -685,11 +685,11 @@ struct BlocksPlan {
 // error rate is not known here): the longest reads set the batch's end on one warp each, and the more
 // so the fewer reads there are per warp slot. Reads with ql^2 above kMwShare (n / slots)^2 times the
 // mean get 8 warps (16 where that few are as long). Measured, ms with that rule / with one warp
-// each / with 8 each: 3,001 reads of 0.5-10 kbp on the sparse graph 11.3 / 17.7 / 11.3, 8,000 12.8 /
-// 19.3 / 12.0, 20,000 19.8 / 21.5 / -, 50,000 28.5 / 28.3 / 73; 4,000 of 0.5-20 kbp on the dense
-// graph 149 / 403 / 131. Reads of one length (mean above kMwUniform of the largest ql^2) get as many
-// as keep all of them running at once: 1,500 x 10 kbp 22.4 with two / 24.5 / 39.1, 3,000 with one 29.1
-// / 29.1 / 69.9. nw > 0: that many for every read.
+// each / with 8 each: 3,001 reads of 0.5-10 kbp on the sparse graph 11.0 / 15.7 / 11.0, 8,000 12.2 /
+// 17.3 / 11.4, 20,000 19.8 / 19.5 / -, 50,000 27.1 / 27.2 / 73; 4,000 of 0.5-20 kbp on the dense
+// graph 142 / 394 / 130. Reads of one length (mean above kMwUniform of the largest ql^2) get as many
+// as keep all of them running at once: 1,500 x 10 kbp 21.6 with two / 24.6 / 37.9, 3,000 with one 28.1
+// / 28.2 / 68.8. nw > 0: that many for every read.
 static const double kMwShare = 0.2, kMwUniform = 0.67;
 
 // Shortest read that gets several warps: shorter ones have no more than a few blocks at a time. With a

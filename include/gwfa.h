@@ -86,9 +86,10 @@ typedef struct {
 	                           0 = by rule: in a batch of mixed lengths the longest reads get 8 or
 	                           16 warps, the more of them the fewer reads there are per warp slot;
 	                           reads of one length get as many (up to 16) as keep all of them
-	                           running at once; the others, and runs with lag pruning, one. With a
+	                           running at once; the others, and runs with a small lag, one. With a
 	                           target vertex (v1 >= 0), or arcs into one vertex of different
-	                           overlaps, per read: the gwf_tune value of its length bucket for
+	                           overlaps, and in batches of short reads that take the sorted form,
+	                           per read: the gwf_tune value of its length bucket for
 	                           GWF_MODE_AUTO, else 2, 4 or 8 warps by its share of the batch's work
 	                           (cost ql^2) and its arena size.
 	                           The plain form uses one warp per read. */
@@ -243,10 +244,11 @@ void gwf_pinned_free(void *p);
 
 /* ---- serving: continuous batching on a resident graph ----
  * No reference counterpart. One resident kernel aligns reads pulled from a device queue, a group
- * of warps per read (reads below 1,500 bases on one warp of it). Reads of queued requests are admitted in FIFO order while a slot is free and
- * the arena budget holds the read's wavefront arena (sized for its own length); a read that
- * overflows its arena is queued again in a 4x larger one, up to three times, ahead of new
- * reads. Results equal those of gwf_ed_batch for the same reads, whatever else is in flight. */
+ * of warps per read (short reads that make few states on one warp of it). Reads of queued requests
+ * are admitted in FIFO order while a slot is free and the arena budget holds the read's arena (sized
+ * for its own length); a read that overflows its arena is queued again in a larger one, through the
+ * block form's classes as far as they fit the budget and the sorted form's 4x, 16x and 64x, ahead of
+ * new reads. Results equal those of gwf_ed_batch for the same reads, whatever else is in flight. */
 typedef struct gwf_srv_s gwf_srv_t;
 typedef struct {
 	int64_t arena_budget_bytes; /* device bytes for in-flight wavefront arenas; 0 = 1/4 of free */
