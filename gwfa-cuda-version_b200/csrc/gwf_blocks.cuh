@@ -66,7 +66,9 @@ struct BwBits {
 	static __device__ __forceinline__ int32_t taken(int32_t c) { return MW ? BW_NONE : 2 * BW_NONE | (c & 1); }
 };
 
-// Word of a string in the graph's filter, and its bits there: two in each half of the word.
+// Word of a string in the graph's filter, and its bits there: two in each half of the word. The
+// multipliers, here and in bw_tag, are those of published 32-bit mixers: 2^32 / golden ratio (xxHash's
+// first prime), MurmurHash3's finaliser, and a pair found by the hash-prospector search.
 __host__ __device__ inline uint32_t bloom_word(uint32_t x, uint32_t mask)
 {
 	x *= 0x9E3779B1u;
